@@ -66,6 +66,7 @@
 // this branch.
 #include <atomic>
 #include <chrono>
+#include <cstring>
 #include <thread>
 #define MVBT_DEV inline
 #define MVBT_COLD static inline
@@ -329,6 +330,14 @@ MVBT_DEV void st_lane(uint32_t* p, const node_regs<W>& n) {
     __atomic_store_n(p + 2 * j + 1, n.v[j], __ATOMIC_RELAXED);
   }
 }
+template <bool kStrong>
+MVBT_DEV void copy_16(uint32_t* dst, const uint32_t* src) {
+  for (int j = 0; j < 4; ++j) dst[j] = __atomic_load_n(src + j, __ATOMIC_RELAXED);
+}
+MVBT_DEV void copy_wait() {}
+MVBT_DEV void store_16(uint32_t* dst, const uint32_t (&w)[4]) {
+  for (int j = 0; j < 4; ++j) __atomic_store_n(dst + j, w[j], __ATOMIC_RELAXED);
+}
 #else
 // Ordinal of the calling tile among the tiles of the launch.
 template <class Tile>
@@ -401,6 +410,29 @@ MVBT_DEV void st_lane(uint32_t* p, const node_regs<W>& n) {
                  : "l"(p), "r"(n.k[0]), "r"(n.v[0])
                  : "memory");
   }
+}
+
+// Asynchronous copy of 16 bytes from global to shared memory (both 16-byte aligned), and the wait
+// for this thread's copies. kStrong: read at L2 (writers may run in the same kernel).
+template <bool kStrong>
+MVBT_DEV void copy_16(uint32_t* dst, const uint32_t* src) {
+  if constexpr (kStrong)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                 :
+                 : "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;"
+                 :
+                 : "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+MVBT_DEV void copy_wait() { asm volatile("cp.async.wait_all;" : : : "memory"); }
+MVBT_DEV void store_16(uint32_t* dst, const uint32_t (&w)[4]) {
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1,%2,%3,%4};"
+               :
+               : "l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+               : "memory");
 }
 
 #endif  // MVBT_HOST_EMULATION
@@ -1928,6 +1960,142 @@ struct device_tree {
     return t.shfl(s, 0);
   }
 };
+
+// ----------------------------------------------------------------------------------------------
+// Lookups of a whole warp in a tree no writer changes meanwhile (concurrent = false)
+// ----------------------------------------------------------------------------------------------
+// Each lane holds one key. A step of the warp copies the node every lane has reached into shared
+// memory -- eight lanes per node, each distinct neighbour once -- and each lane then searches its
+// own node there. A tile per key (find_quiescent) spends the instructions of a whole tile on
+// one key's node; here 32 keys share them, and keys that are near each other share the node
+// reads too.
+struct alignas(16) warp_stage {
+  uint32_t node[32][kNodeWords];  // 16-byte pieces of node s at piece ^ (s & 7): the lanes' reads
+                                  // of one word of different nodes spread over the banks
+  uint32_t idx[32];               // the nodes to copy
+  uint32_t path[kMaxLevels][4];   // last key's node per level {index, low, high}: the next keys' start
+  // Word w of staged node s, and its words 28..31.
+  MVBT_DEV uint32_t word(uint32_t s, uint32_t w) const { return node[s][(((w >> 2) ^ (s & 7u)) << 2) | (w & 3u)]; }
+  MVBT_DEV const uint32_t* last_words(uint32_t s) const { return &node[s][(7u ^ (s & 7u)) << 2]; }
+};
+#if defined(MVBT_HOST_EMULATION)
+MVBT_DEV void ld_shared_4(const uint32_t* p, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  a = p[0], b = p[1], c = p[2], d = p[3];
+}
+#else
+MVBT_DEV void ld_shared_4(const uint32_t* p, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  const uint4 v = *reinterpret_cast<const uint4*>(p);
+  a = v.x, b = v.y, c = v.z, d = v.w;
+}
+#endif
+
+template <class Warp>
+MVBT_DEV void clear_path(warp_stage& st, const Warp& warp) {
+  const uint32_t lane = warp.thread_rank();
+  if (lane < (uint32_t)kMaxLevels) {
+    st.path[lane][0] = kNone;
+    st.path[lane][1] = kEmptyKey;  // covers nothing
+    st.path[lane][2] = 0;
+  }
+  warp.sync();
+}
+
+// Lowest remembered node that covers all of [first, last], or the anchor. Every lane looks at a level.
+template <class Warp>
+MVBT_DEV uint32_t path_start(const warp_stage& st, uint32_t first, uint32_t last, const Warp& warp) {
+  const uint32_t l  = warp.thread_rank() & (kMaxLevels - 1u);
+  const uint32_t in = warp.ballot(st.path[l][1] <= first && last < st.path[l][2]);
+  return in ? st.path[__ffs(in) - 1][0] : kAnchor;
+}
+
+// Copies the nodes idx of the live lanes (m) into st, neighbouring lanes' equal ones once; returns
+// the lane's slot. The caller keeps every lane's reads of the last nodes before this (warp.sync).
+template <bool kStrong, class Warp>
+MVBT_DEV uint32_t stage_nodes(const device_tree& T, uint32_t idx, bool live, uint32_t m, warp_stage& st,
+                              const Warp& warp) {
+  const uint32_t lane  = warp.thread_rank();
+  const uint32_t prev  = warp.shfl(idx, lane ? (int)lane - 1 : 0);
+  const bool lead      = live && (lane == 0 || !((m >> (lane - 1)) & 1u) || prev != idx);
+  const uint32_t leads = warp.ballot(lead);
+  const uint32_t slot  = (uint32_t)__popc(leads & ((2u << lane) - 1u)) - 1u;
+  if (lead) st.idx[slot] = idx;
+  warp.sync();
+  const uint32_t nodes = (uint32_t)__popc(leads), piece = lane & 7u;
+  for (uint32_t s = lane >> 3; s < nodes; s += 4)
+    copy_16<kStrong>(&st.node[s][(piece ^ (s & 7u)) << 2], T.node_ptr(st.idx[s]) + piece * 4);
+  copy_wait();
+  warp.sync();
+  return slot;
+}
+
+// Pairs of staged node s whose key is <= key: they are sorted, and unused ones hold the highest key.
+MVBT_DEV uint32_t count_up_to(const warp_stage& st, uint32_t s, uint32_t key) {
+  uint32_t c = st.word(s, 2 * 7) <= key ? 8u : 0u;
+  if (st.word(s, 2 * (c + 3)) <= key) c += 4;
+  if (c + 1 < (uint32_t)kDataPairs && st.word(s, 2 * (c + 1)) <= key) c += 2;
+  if (c < (uint32_t)kDataPairs && st.word(s, 2 * c) <= key) c += 1;
+  return c;
+}
+
+// The value of each live lane's key at snapshot ts (kLatest: newest), kNotFound elsewhere; the
+// route and results of find_quiescent. start: a node on every live key's route (the anchor, or
+// path_start). keep_path: the nodes that the highest live lane passes are remembered for it.
+template <class Warp>
+MVBT_DEV uint32_t find_warp(const device_tree& T, uint32_t key, bool live, uint32_t ts, uint32_t start,
+                            bool keep_path, warp_stage& st, const Warp& warp) {
+  const bool snap     = T.versioned && ts != kLatest;
+  const uint32_t lane = warp.thread_rank();
+  uint32_t found      = kNotFound;
+  uint32_t idx        = start;
+  live                = live && key != kEmptyKey;
+  const uint32_t all  = warp.ballot(live);
+  const bool last     = keep_path && live && (all >> lane) == 1u;
+  for (uint32_t step = 0; step < kMaxSteps; ++step) {
+    if (live && idx >= T.capacity) {
+      T.set_error(kErrCorrupt, 1);
+      live = false;
+    }
+    const uint32_t m = warp.ballot(live);
+    if (m == 0) return found;
+    const uint32_t slot = stage_nodes<false>(T, idx, live, m, st, warp);
+    if (live) {
+      const uint32_t low = st.word(slot, 26);
+      uint32_t high, link, nts, ol;
+      ld_shared_4(st.last_words(slot), high, link, nts, ol);
+      link &= kIndexMask;
+      if (snap && nts > ts) {  // a newer version: move to the older one
+        idx = ol & kIndexMask;
+        if (idx == kNone) {
+          T.set_error(kErrCorrupt, 3);
+          live = false;
+        }
+      } else if (key < low) {
+        idx = kAnchor;
+      } else if (key >= high && link != kNone) {
+        idx = link;
+      } else {
+        const uint32_t level = ol >> 28;
+        if (last) {
+          st.path[level][0] = idx;
+          st.path[level][1] = low;
+          st.path[level][2] = high;
+        }
+        const uint32_t c  = count_up_to(st, slot, key);
+        const uint32_t pk = c ? st.word(slot, 2 * c - 2) : kEmptyKey;
+        const uint32_t pv = c ? st.word(slot, 2 * c - 1) : kAnchor;
+        if (level == 0) {
+          if (pk == key) found = pv;
+          live = false;
+        } else {
+          idx = pv;
+        }
+      }
+    }
+    warp.sync();
+  }
+  if (live) T.set_error(kErrStepLimit, 4);
+  return found;
+}
 
 // ----------------------------------------------------------------------------------------------
 // Mixed operation batches

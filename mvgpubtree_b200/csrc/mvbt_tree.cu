@@ -151,6 +151,57 @@ __global__ void __launch_bounds__(256) k_find(device_tree T, const uint32_t* __r
   }
 }
 
+// Lookups in a tree no writer changes meanwhile, 32 keys per warp at a time (mvbt::find_warp).
+// kSorted: the keys are a sorted call's, each warp takes one contiguous run of them and starts at
+// the deepest node of the last keys' path that covers the next ones, and the results go back to the
+// caller's positions (spos). A tile per key spends about 40 instructions of every lane on each of
+// its nodes (issue-bound); here they serve 32 keys. 36 KB of shared memory and 40 registers: six
+// blocks per SM.
+constexpr int kReadSortLowBit   = 8;  // reads: order by the top 24 bits (locality is all they need)
+constexpr uint32_t kUnsortedBits = (1u << kReadSortLowBit) - 1u;
+constexpr int kWarpsPerBlock    = 8;
+template <bool kSorted>
+__global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t* __restrict__ keys,
+                                                   const uint32_t* __restrict__ spos, uint32_t* __restrict__ out,
+                                                   uint32_t n, uint32_t ts) {
+  __shared__ mvbt::warp_stage stage[kWarpsPerBlock];
+  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
+  mvbt::warp_stage& st  = stage[threadIdx.x >> 5];
+  const uint32_t lane   = threadIdx.x & 31u;
+  const uint64_t warps  = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint64_t w      = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t groups = ((uint64_t)n + 31) / 32;
+  const uint64_t per    = (groups + warps - 1) / warps;
+  uint64_t g            = kSorted ? w * per : w;
+  const uint64_t end    = kSorted ? (g + per < groups ? g + per : groups) : groups;
+  const uint64_t stride = kSorted ? 1 : warps;
+  uint32_t key = 0, pos = 0;
+  auto fetch = [&](uint64_t group) {  // the lane's key of a group, and whether it has one
+    const uint64_t i = group * 32 + lane;
+    const bool has   = group < end && i < n;
+    if (has) {
+      key = keys[i];
+      pos = kSorted ? spos[i] : (uint32_t)i;
+    }
+    return has;
+  };
+  if (kSorted) mvbt::clear_path(st, warp);
+  bool live = fetch(g);
+  for (; g < end; g += stride) {
+    const uint32_t k = key, p = pos;
+    const bool here  = live;
+    live             = fetch(g + stride);  // on its way while this group is looked up
+    uint32_t start   = mvbt::kAnchor;
+    if (kSorted) {  // the keys are in order down to the bits that the sort left out
+      const uint32_t m = __ballot_sync(0xffffffffu, here);
+      start = mvbt::path_start(st, __shfl_sync(0xffffffffu, k, 0) & ~kUnsortedBits,
+                               __shfl_sync(0xffffffffu, k, 31 - __clz(m)) | kUnsortedBits, warp);
+    }
+    const uint32_t v = mvbt::find_warp(T, k, here, ts, start, kSorted, st, warp);
+    if (here) out[p] = v;
+  }
+}
+
 template <int W>
 __global__ void __launch_bounds__(256) k_insert(device_tree T, const uint32_t* __restrict__ keys,
                                                 const uint32_t* __restrict__ values, uint32_t n) {
@@ -260,7 +311,7 @@ __device__ __forceinline__ void tile_run(uint64_t n, uint64_t& begin, uint64_t& 
   end                = begin + per < n ? begin + per : n;
 }
 
-template <int W, bool kStrong>
+template <int W>
 __global__ void __launch_bounds__(256) k_find_sorted(device_tree T, const uint32_t* __restrict__ skeys,
                                                      const uint32_t* __restrict__ spos,
                                                      uint32_t* __restrict__ out, uint32_t n, uint32_t ts) {
@@ -271,8 +322,7 @@ __global__ void __launch_bounds__(256) k_find_sorted(device_tree T, const uint32
   for (; warp_any(i < end); ++i) {
     if (i >= end) continue;
     const uint32_t key = skeys[i];
-    const uint32_t v   = kStrong ? T.cooperative_find<W>(key, tile, ts, true, f.start_for(key, tile), &f)
-                                 : T.find_quiescent<W>(key, tile, ts, f.start_for(key, tile), &f);
+    const uint32_t v   = T.cooperative_find<W>(key, tile, ts, true, f.start_for(key, tile), &f);
     if (tile.thread_rank() == 0) out[spos[i]] = v;
   }
 }
@@ -371,6 +421,18 @@ unsigned grid_for(const mvbt_tree* t, K kernel, uint64_t ops) {
   return (unsigned)g;
 }
 
+// Grid of k_find_warp for n keys: its warps take 32 at a time.
+template <class K>
+unsigned grid_for_warps(const mvbt_tree* t, K kernel, uint64_t n) {
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, t->block_size, 0);
+  if (per_sm < 1) per_sm = 1;
+  if (t->blocks_per_sm && (int)t->blocks_per_sm < per_sm) per_sm = (int)t->blocks_per_sm;
+  uint64_t g = std::min<uint64_t>((n + t->block_size - 1) / t->block_size, (uint64_t)per_sm * t->num_sms);
+  if (t->max_blocks) g = std::min<uint64_t>(g, t->max_blocks);
+  return (unsigned)std::max<uint64_t>(g, 1);
+}
+
 int check_launch() {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MVBT_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
@@ -383,6 +445,10 @@ int status_from_bits(uint32_t bits) {
   if (bits & (mvbt::kErrCorrupt | mvbt::kErrStepLimit)) return MVBT_ERR_CORRUPT;
   return MVBT_OK;
 }
+
+// Fewer lookups than this leave most warps of k_find_warp empty; a tile per key has the shorter
+// chain then.
+constexpr uint32_t kWarpFindMin = 1u << 13;
 
 // Bulk insert of n keys. On a tree that is small against the batch, the tiles of a full grid
 // would queue on the few leaves there are, and every handoff of a queued lock costs an atomic per
@@ -417,6 +483,16 @@ bool use_sorted(const mvbt_tree* t, uint32_t n) {
   if (t->frontend == MVBT_FRONTEND_UNSORTED) return false;
   return n >= (1u << 16) && (uint64_t)n * 128 >= t->grown;
 }
+
+// Whether lookups in a tree no writer changes meanwhile are sorted first. A warp's lookups in the
+// caller's order cost about as much as sorting and then looking up at 2^20 keys (us, unsorted /
+// sorted: 93 / 91 in a tree of 2^20 keys, 125 / 120 in one of 40M, 73 / 80 in one of 2^16); at 2^22
+// they cost twice as much (354 / 195, 474 / 262, 271 / 169), at 2^18 half (29 / 62, 38 / 71, 23 / 58).
+bool sorted_lookups(const mvbt_tree* t, uint32_t n) {
+  if (t->frontend == MVBT_FRONTEND_AUTO) return n >= (1u << 20);
+  return t->frontend == MVBT_FRONTEND_SORTED && n > 1;
+}
+
 
 // A stream-ordered memory pool per device for the sort's scratch: no device-wide synchronisation,
 // and freed blocks stay cached in the pool for the next call (up to kPoolKeepBytes).
@@ -478,8 +554,6 @@ int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaSt
   }
   return MVBT_OK;
 }
-
-constexpr int kReadSortLowBit = 8;  // reads: order by the top 24 bits (locality is all they need)
 
 template <int W>
 int insert_sorted_launches(mvbt_tree* t, const sorted_ops& so, const uint32_t* values, uint32_t n, cudaStream_t s) {
@@ -1130,21 +1204,21 @@ int mvbt_find(mvbt_tree* t, const uint32_t* keys, uint32_t* values, uint32_t n, 
   if (t->kind == MVBT_KIND_BLINK) ts = mvbt::kLatest;
   cudaStream_t s = as_stream(stream);
   const int bs   = t->block_size;
-  if (use_sorted(t, n)) {
+  if (concurrent ? use_sorted(t, n) : sorted_lookups(t, n)) {
     sorted_ops so;
     int st = sort_ops(t, keys, n, kReadSortLowBit, s, &so);
     if (st) return st;
     const device_tree v = t->view();
-    if (t->tile_width == 8) {
-      if (concurrent) k_find_sorted<8, true><<<grid_for(t, k_find_sorted<8, true>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
-      else k_find_sorted<8, false><<<grid_for(t, k_find_sorted<8, false>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
-    } else {
-      if (concurrent) k_find_sorted<16, true><<<grid_for(t, k_find_sorted<16, true>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
-      else k_find_sorted<16, false><<<grid_for(t, k_find_sorted<16, false>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
-    }
+    if (!concurrent) k_find_warp<true><<<grid_for_warps(t, k_find_warp<true>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
+    else if (t->tile_width == 8) k_find_sorted<8><<<grid_for(t, k_find_sorted<8>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
+    else k_find_sorted<16><<<grid_for(t, k_find_sorted<16>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
     st = check_launch();
     const int rs = so.release(s);
     return st ? st : rs;
+  }
+  if (!concurrent && n >= kWarpFindMin) {
+    k_find_warp<false><<<grid_for_warps(t, k_find_warp<false>, n), bs, 0, s>>>(t->view(), keys, nullptr, values, n, ts);
+    return check_launch();
   }
   if (t->tile_width == 8) {
     if (concurrent) k_find<8, true><<<grid_for(t, k_find<8, true>, n), bs, 0, s>>>(t->view(), keys, values, n, ts);

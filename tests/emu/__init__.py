@@ -27,6 +27,7 @@ def lib():
             "emu_insert": (None, [vp, u32p, u32p, u64, i, i]),
             "emu_erase": (None, [vp, u32p, u64, i, i]),
             "emu_find": (None, [vp, u32p, u32p, u64, u32, i, i, i]),
+            "emu_find_warp": (None, [vp, u32p, u32p, u32p, u64, u32, i, u32, i, u32]),
             "emu_range": (None, [vp, u32p, u32p, vp, vp, u32, u64, u32, i, i, i]),
             "emu_insert_range": (None, [vp, u32p, u32p, u64, u32p, u32p, u64, vp, vp, u32, i, i]),
             "emu_find_erase": (None, [vp, u32p, u32p, u64, u32p, u64, i, i]),
@@ -97,6 +98,16 @@ class EmuTree:
         k = _u32(k)
         out = np.empty_like(k)
         self.L.emu_find(self.h, k, out, k.size, ts, self.tiles, self.W, int(quiescent))
+        return out
+
+    def find_warp(self, k, ts=0xFFFFFFFF, warps=2, lanes=32, sorted_run=False, bits=32):
+        """Warp lookups; sorted_run: the keys ordered by their top `bits` (a stable sort, as the sorted
+        front-end orders reads), results in input order."""
+        k = _u32(k)
+        order = np.argsort(k >> np.uint32(32 - bits), kind="stable").astype(np.uint32) if sorted_run else np.arange(k.size, dtype=np.uint32)
+        out = np.zeros_like(k)
+        self.L.emu_find_warp(self.h, np.ascontiguousarray(k[order]), order, out, k.size, ts, warps, lanes, int(sorted_run),
+                             (1 << (32 - bits)) - 1)
         return out
 
     def range(self, lo, hi, avg_len, ts=0xFFFFFFFF, quiescent=False):

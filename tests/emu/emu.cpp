@@ -223,6 +223,36 @@ void emu_find(void* h, const uint32_t* keys, uint32_t* out, uint64_t n, uint32_t
   }));
 }
 
+// Warp lookups (find_warp): `lanes` keys per warp at a time over `warps` warps; sorted != 0: each
+// warp takes a contiguous run of groups and keeps the last key's path, as the sorted kernel does
+// (low_bits: the key bits its order left out).
+void emu_find_warp(void* h, const uint32_t* keys, const uint32_t* pos, uint32_t* out, uint64_t n, uint32_t ts,
+                   int warps, uint32_t lanes, int sorted, uint32_t low_bits) {
+  auto* t = static_cast<emu_tree*>(h);
+  auto v  = t->view();
+  if (!v.versioned) ts = mvbt::kLatest;
+  const uint64_t groups = (n + lanes - 1) / lanes, per = (groups + warps - 1) / warps;
+  std::vector<mvbt::warp_stage> stage(warps);
+  run_warps(warps, 8, [&](const emu_tile& warp, const emu_tile&) {
+    const uint64_t w = mvbt::emu::sm;
+    uint64_t g       = sorted ? w * per : w;
+    const uint64_t end = sorted ? std::min(g + per, groups) : groups;
+    if (sorted) mvbt::clear_path(stage[w], warp);
+    for (; g < end; g += sorted ? 1 : warps) {
+      const uint64_t i = g * lanes + warp.thread_rank();
+      const bool live  = (uint32_t)warp.thread_rank() < lanes && i < n;
+      const uint32_t k = live ? keys[i] : 0u;
+      uint32_t start = mvbt::kAnchor;
+      if (sorted) {
+        const uint32_t m = warp.ballot(live);
+        start = mvbt::path_start(stage[w], warp.shfl(k, 0) & ~low_bits, warp.shfl(k, 31 - __clz(m)) | low_bits, warp);
+      }
+      const uint32_t r = mvbt::find_warp(v, k, live, ts, start, sorted != 0, stage[w], warp);
+      if (live) out[sorted ? pos[i] : i] = r;
+    }
+  });
+}
+
 // quiescent != 0: the range query of a tree no writer changes meanwhile (range_quiescent).
 void emu_range(void* h, const uint32_t* lo, const uint32_t* hi, uint32_t* pairs, uint32_t* counts,
                uint32_t avg_len, uint64_t n, uint32_t ts, int tiles, int W, int quiescent) {

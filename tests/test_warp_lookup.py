@@ -1,0 +1,68 @@
+"""Lookups by whole warps (mvbt::find_warp, k_find_warp): every lane holds a key, nodes are staged in
+shared memory. Checked against the oracle on trees whose snapshots, erased keys and split nodes give
+every kind of step, in a sorted run (with path memory) and in the caller's order, with full and
+partial groups of keys."""
+import numpy as np
+import pytest
+
+ABSENT = np.array([0, 1, 2**31, 0xFFFFFFFE, 0xFFFFFFFF], np.uint32)
+
+
+def _history(seed, n0):
+    """Initial keys, updates, erases and late inserts with their values, and lookups of all of them."""
+    import workload as wl
+    keys = wl.distinct_keys(seed, 0, n0)
+    late = wl.distinct_keys(seed, n0, n0 // 2)
+    upd, gone = wl.shuffle(seed + 1, keys)[: n0 // 3], wl.shuffle(seed + 2, keys)[: n0 // 4]
+    q = wl.shuffle(seed + 3, np.concatenate([keys, late, wl.distinct_keys(seed, wl.MISS_INDEX_BASE, n0 // 2), ABSENT]))
+    v = lambda k, s: wl.values_for(k, seed + s)
+    return [("insert", keys, v(keys, 0)), ("insert", upd, v(upd, 1)), ("erase", gone, None), ("insert", late, v(late, 2))], q
+
+
+@pytest.mark.parametrize("versioned", [False, True])
+@pytest.mark.parametrize("lanes,sorted_run,bits", [(32, False, 0), (8, False, 0), (5, False, 0), (32, True, 32), (32, True, 8)])
+def test_emulated_warp_lookups_match_oracle(versioned, lanes, sorted_run, bits):
+    from emu import EmuTree
+    import oracle
+    ops, q = _history(71, 900)
+    t, m = EmuTree(versioned, capacity=1 << 14, tiles=4, W=8), oracle.MVMap(versioned)
+    snaps = [0xFFFFFFFF]
+    for kind, k, v in ops:
+        for x in (t, m):
+            x.insert(k, v) if kind == "insert" else x.erase(k)
+        if versioned:
+            snaps.append(t.snapshot())
+            assert snaps[-1] == m.take_snapshot()
+    for ts in snaps:
+        for n in (1, 31, 33, q.size):
+            got = t.find_warp(q[:n], ts=ts, warps=3, lanes=lanes, sorted_run=sorted_run, bits=bits)
+            assert np.array_equal(got, m.find(q[:n], ts) if versioned else m.find(q[:n]))
+    assert t.errors == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("versioned,block", [(False, 256), (True, 256), (True, 32), (True, 96)])
+def test_gpu_lookup_sizes_around_the_rules_match_oracle(versioned, block):
+    """Call sizes on both sides of the tile / warp and the unsorted / sorted rules, odd ones among them."""
+    import torch
+    import mvgpubtree_b200 as mv
+    import oracle
+    ops, q = _history(72, 40_000)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.uint32).view(np.int32)).cuda()
+    cls = mv.gpu_versioned_btree if versioned else mv.gpu_blink_tree
+    t, m = cls(pool_bytes=1 << 28, block_size=block), oracle.MVMap(versioned)
+    snaps = [mv.LATEST]
+    for kind, k, v in ops:
+        t.insert(dev(k), dev(v)) if kind == "insert" else t.erase(dev(k))
+        m.insert(k, v) if kind == "insert" else m.erase(k)
+        if versioned:
+            snaps.append(t.take_snapshot())
+            assert snaps[-1] == m.take_snapshot()
+    many = np.resize(q, (1 << 20) + 33)
+    for ts in snaps[:1] + snaps[2:3]:
+        want = m.find(q, ts) if versioned else m.find(q)
+        for n in (1, 8191, 8192, 8193, (1 << 20) - 1, 1 << 20, (1 << 20) + 33):
+            out = torch.zeros(n, dtype=torch.int32, device="cuda")
+            t.find(dev(many[:n]), out, timestamp=ts)
+            assert np.array_equal(out.cpu().numpy().view(np.uint32), np.resize(want, n))
+    assert t.check_errors() == 0

@@ -1,0 +1,46 @@
+"""Inserts and erases by whole warps (mvbt::write_warp): one op per lane, the leaves of a warp locked, copied
+and written back together, full leaves split by the tile path. Checked against the oracle: dense runs
+that split a leaf several times, updates, erases of present and absent keys, several warps writing at
+once, snapshots in between, reclamation."""
+import numpy as np
+import pytest
+
+
+@pytest.mark.parametrize("w", [8, 16])
+@pytest.mark.parametrize("versioned,reclaim,chunk", [(False, False, 64), (True, False, 64), (True, True, 32), (True, False, 8)])
+@pytest.mark.parametrize("sorted_run", [False, True])
+def test_emulated_warp_writes_match_oracle(w, versioned, reclaim, chunk, sorted_run):
+    from emu import EmuTree
+    import oracle
+    import workload as wl
+    seed = 83
+    t = EmuTree(versioned, capacity=1 << 14, tiles=4, W=w, chunk=chunk, reclaim=reclaim)
+    m = oracle.MVMap(versioned)
+    keys = wl.distinct_keys(seed, 0, 600)
+    dense = np.arange(keys[0], keys[0] + 130, dtype=np.uint32)  # more than one group in one leaf
+    every = np.unique(np.concatenate([keys, dense, np.array([0, 1, 0xFFFFFFFE], np.uint32)]))
+    rng = np.random.default_rng(seed)
+    for r in range(4):
+        op = rng.permutation(every)[: every.size * (3 if r else 4) // 4]
+        kind = np.where(rng.random(op.size) < (0.35 if r else 0.0), 2, 1).astype(np.uint32)
+        vals = wl.values_for(op, seed + r)
+        if sorted_run:  # repeated keys: only the last op of each counts
+            op, kind, vals = np.concatenate([op[:40], op]), np.concatenate([np.full(40, 1, np.uint32), kind]), np.concatenate([vals[:40] ^ 1, vals])
+        t.write_warp(kind, op, vals, warps=3, sorted_run=sorted_run)
+        last = {int(k): i for i, k in enumerate(op)}
+        idx = np.array(sorted(last.values()))
+        ok, kk, vv = op[idx], kind[idx], vals[idx]
+        m.insert(ok[kk == 1], vv[kk == 1])
+        m.erase(ok[kk == 2])
+        assert t.errors == 0, t.stats()
+        assert np.array_equal(t.find(every), m.find(every))
+        if versioned:
+            s = t.snapshot()
+            assert s == m.take_snapshot()
+            if r:
+                assert np.array_equal(t.find(every, s - 1), m.find(every, s - 1))
+            if reclaim and r == 2:
+                t.reclaim(s)
+    rep = t.validate()
+    assert rep["violations"] == 0 and rep["locked_nodes"] == 0
+    assert t.stats()["splits"] > 20
