@@ -71,6 +71,7 @@
 #define MVBT_DEV inline
 #define MVBT_COLD static inline
 #define MVBT_OUTLINE inline
+#define MVBT_CALL inline
 struct uint2 {
   uint32_t x, y;
 };
@@ -128,6 +129,8 @@ inline thread_local uint32_t sm = 0;  // emulated SM id of the calling lane
 #ifndef MVBT_OUTLINE
 #define MVBT_OUTLINE __device__ __forceinline__
 #endif
+// A called function: the rare path of a warp's writes, kept out of its loop's code and registers.
+#define MVBT_CALL __device__ __noinline__
 #endif
 
 namespace mvbt {
@@ -2095,6 +2098,350 @@ MVBT_DEV uint32_t find_warp(const device_tree& T, uint32_t key, bool live, uint3
   }
   if (live) T.set_error(kErrStepLimit, 4);
   return found;
+}
+
+// ----------------------------------------------------------------------------------------------
+// Writes of a whole warp
+// ----------------------------------------------------------------------------------------------
+struct write_stage : warp_stage {
+  uint32_t op[32][2];  // each lane's {key, value}
+  uint32_t done[32];   // 1: the lane's op was applied, 0: its leaf is full
+  uint32_t dst[32];    // where each staged node is stored (kNone: nowhere)
+};
+
+// The leaf that each live lane's key belongs to, unread: the child its level-1 node names (kNone:
+// failed). Routing at the newest state while writers run, as descend_for_write.
+template <class Warp>
+MVBT_DEV uint32_t leaf_warp(const device_tree& T, uint32_t key, bool live, uint32_t start, bool keep_path,
+                            warp_stage& st, const Warp& warp) {
+  const uint32_t lane = warp.thread_rank();
+  uint32_t leaf       = kNone;
+  uint32_t idx        = start;
+  const uint32_t all  = warp.ballot(live);
+  const bool last     = keep_path && live && (all >> lane) == 1u;
+  for (uint32_t step = 0; step < kMaxSteps; ++step) {
+    if (live && idx >= T.capacity) {
+      T.set_error(kErrCorrupt, 1);
+      live = false;
+    }
+    const uint32_t m = warp.ballot(live);
+    if (m == 0) return leaf;
+    const uint32_t slot = stage_nodes<true>(T, idx, live, m, st, warp);
+    if (live) {
+      const uint32_t low = st.word(slot, 26);
+      uint32_t high, link, nts, ol;
+      ld_shared_4(st.last_words(slot), high, link, nts, ol);
+      link &= kIndexMask;
+      const uint32_t level = ol >> 28;
+      if (key < low) {
+        idx = kAnchor;
+      } else if (key >= high && link != kNone) {
+        idx = link;
+      } else if (level == 0) {  // reached through a sibling link or a misrouted read
+        leaf = idx;
+        live = false;
+      } else {
+        if (last) {
+          st.path[level][0] = idx;
+          st.path[level][1] = low;
+          st.path[level][2] = high;
+        }
+        const uint32_t c = count_up_to(st, slot, key);
+        idx              = c ? st.word(slot, 2 * c - 1) : kAnchor;
+        if (c && level == 1) {
+          leaf = idx;
+          live = false;
+        }
+      }
+    }
+    warp.sync();
+  }
+  if (live) T.set_error(kErrStepLimit, 8);
+  return leaf;
+}
+
+// A fresh node for each lane with `need` set (kNone: the pool is full or the wait limit ran out): one
+// atomic of the warp on the SM's chunk cursor instead of one per node.
+template <class Warp>
+MVBT_DEV uint32_t alloc_warp(const device_tree& T, bool need, const Warp& warp) {
+  const uint32_t m = warp.ballot(need);
+  if (m == 0) return kNone;
+  control_block* c    = T.ctl;
+  const uint32_t lane = warp.thread_rank();
+  const uint32_t C    = c->chunk;
+  const uint32_t k    = (uint32_t)__popc(m);
+  const int lead      = __ffs(m) - 1;
+  uint32_t idx        = kNone;
+  if (C < 32) {  // a request could span chunks
+    if (need) idx = T.alloc_one();
+  } else {
+    uint32_t base = 0, used = 0, next = kNone;  // nodes base + used .. below chunk C, then next, next + 1, ..
+    bool got = false;
+    if ((int)lane == lead) {
+      unsigned long long* slot    = &c->sm_pool[sm_id() % kMaxSmSlots];
+      const uint32_t limit        = c->spin_limit;
+      const unsigned long long t0 = global_ns();
+      for (uint32_t tries = 0; tries < limit; ++tries) {
+        if (tries && (ld_relaxed_u32(&c->error) & kErrPoolExhausted)) break;
+        const unsigned long long old = atomicAdd(slot, (unsigned long long)k);
+        base = (uint32_t)(old >> 32), used = (uint32_t)old;
+        if (used + k <= C) {
+          got = true;
+          break;
+        }
+        if (used <= C) {  // this request holds position C: it refills the chunk, as alloc_one does
+          got = true;
+          if (!(T.reclaim && take_free_chunk(c, C, next))) {
+            next = atomicAdd(&c->bump, C);
+            if ((unsigned long long)next + C > c->capacity) {
+              next = kNone;
+              atomicOr(&c->error, kErrPoolExhausted);
+              atomicAdd(&c->err_site[15], 1u);
+            }
+          }
+          if (next != kNone) atomicExch(slot, ((unsigned long long)next << 32) | (used + k - C));
+          break;
+        }
+        for (uint32_t w = 0; w < limit; ++w) {  // another request refills it
+          __nanosleep(64);
+          const unsigned long long cur = ld_relaxed_u64(slot);
+          if ((uint32_t)(cur >> 32) != base || (uint32_t)cur < C) break;
+          if (ld_relaxed_u32(&c->error) & kErrPoolExhausted) break;
+          if (global_ns() - t0 > c->wait_ns) break;
+        }
+        if (global_ns() - t0 > c->wait_ns) break;
+      }
+      if (!got && !(ld_relaxed_u32(&c->error) & kErrPoolExhausted)) {
+        atomicOr(&c->error, kErrSpinLimit);
+        atomicAdd(&c->err_site[0], 1u);
+      }
+    }
+    base             = warp.shfl(base, lead);
+    used             = warp.shfl(used, lead);
+    next             = warp.shfl(next, lead);
+    const bool given = warp.shfl(got ? 1u : 0u, lead) != 0;
+    if (need && given) {
+      const uint32_t at = used + (uint32_t)__popc(m & ((1u << lane) - 1u));
+      if (at < C) idx = base + at;
+      else if (next != kNone) idx = next + (at - C);
+    }
+  }
+  if (idx != kNone && (idx & kRingChunk)) idx = chunk_node(c, idx, 0);  // a position in the free ring
+  return idx;
+}
+
+// Records the lanes' version copies (`has` set), as device_tree::retire, with one reservation.
+template <class Warp>
+MVBT_DEV void retire_warp(const device_tree& T, bool has, uint32_t copy, const Warp& warp) {
+  const uint32_t m = warp.ballot(has);
+  if (m == 0) return;
+  control_block* c    = T.ctl;
+  const uint32_t lane = warp.thread_rank();
+  const int lead      = __ffs(m) - 1;
+  unsigned long long pos = 0;
+  if ((int)lane == lead) {
+    if (T.reclaim) pos = atomicAdd(&c->retire_tail, (unsigned long long)__popc(m));
+    else atomicAdd(&c->sm_stats[sm_id() % kMaxSmSlots][0], (unsigned long long)__popc(m));
+  }
+  if (!T.reclaim) return;  // the same in every lane
+  pos = warp.shfl(pos, lead) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+  if (has) {
+    if (pos - ld_relaxed_u64(&c->retire_head) < c->reclaim_cap)
+      reinterpret_cast<uint32_t*>(c->retire_log)[pos & (c->reclaim_cap - 1u)] = copy;
+    else
+      atomicAdd(&c->stat_log_dropped, 1ull);
+  }
+}
+
+// Applies one op to staged leaf s of n pairs; false: an insert found it full. Called by one lane.
+MVBT_DEV bool apply_staged(warp_stage& st, uint32_t s, uint32_t& n, uint32_t key, uint32_t value, bool erase) {
+  auto at           = [&](uint32_t w) -> uint32_t& { return st.node[s][(((w >> 2) ^ (s & 7u)) << 2) | (w & 3u)]; };
+  const uint32_t c  = count_up_to(st, s, key);
+  const bool hit    = c && at(2 * c - 2) == key;
+  if (erase) {
+    if (!hit) return true;
+    for (uint32_t p = c; p < n; ++p) at(2 * p - 2) = at(2 * p), at(2 * p - 1) = at(2 * p + 1);
+    at(2 * n - 2) = kEmptyKey, at(2 * n - 1) = kEmptyKey;
+    --n;
+    return true;
+  }
+  if (hit) {
+    at(2 * c - 1) = value;
+    return true;
+  }
+  if (n == (uint32_t)kDataPairs) return false;
+  for (uint32_t p = n; p > c; --p) at(2 * p) = at(2 * p - 2), at(2 * p + 1) = at(2 * p - 1);
+  at(2 * c) = key, at(2 * c + 1) = value;
+  ++n;
+  return true;
+}
+
+// One write by a tile, from the leaf where its warp found it.
+template <int W, class Tile>
+MVBT_CALL void write_tile(device_tree T, uint32_t key, uint32_t value, bool erase, uint32_t E, uint32_t leaf, Tile tile) {
+  if (erase) T.erase_at<W>(key, tile, E, leaf);
+  else T.insert_at<W>(key, value, tile, E, leaf, kNone, kNone, 0u);
+}
+
+// Runs the live lanes' inserts (key -> value) and erases in write epoch E. The warp locks the leaves
+// of all its keys with one atomic per leaf, stages them, copies the versions that need it, applies
+// every key of a leaf to its staged copy and writes the leaves back, so two fences serve up to 32
+// leaves where a tile per key (insert_at, erase_at) spends them on one. The steps on a leaf and their
+// order are those of the tile path: lock, read, version copy complete before a header names it,
+// leaf stored, release. No lane waits for a lock while the warp holds one: leaves found locked are
+// tried again after the others are released. A leaf without room for a new key is split by the tile
+// path (one key per leaf at a time), and the leaf's other keys go on from there.
+// start / keep_path: as in find_warp. Two live lanes may hold one key only if either order will do.
+template <int W, class Warp, class Tile>
+MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, bool erase, bool live, uint32_t E,
+                         uint32_t start, bool keep_path, write_stage& st, const Warp& warp, const Tile& tile) {
+  constexpr uint32_t kTiles = 32 / W;
+  const uint32_t lane       = warp.thread_rank();
+  const uint32_t piece      = lane & 7u;
+  live                      = live && key != kEmptyKey;
+  uint32_t leaf             = leaf_warp(T, key, live, start, keep_path, st, warp);
+  bool pend                 = live && leaf != kNone;
+  const uint32_t erases     = warp.ballot(erase);
+  st.op[lane][0]            = key;
+  st.op[lane][1]            = value;
+  uint32_t tries = 0, backoff = 32;
+  unsigned long long t0     = 0;
+  for (uint32_t step = 0; step < kMaxSteps; ++step) {
+    if (pend && leaf >= T.capacity) {
+      T.set_error(kErrCorrupt, 1);
+      pend = false;
+    }
+    const uint32_t pm = warp.ballot(pend);
+    if (pm == 0) return;
+    // one leader per run of neighbouring lanes with the same leaf
+    const uint32_t prev = warp.shfl(leaf, lane ? (int)lane - 1 : 0);
+    const bool lead     = pend && (lane == 0 || !((pm >> (lane - 1)) & 1u) || prev != leaf);
+    const uint32_t lm   = warp.ballot(lead);
+    uint32_t* const mod = T.node_ptr(pend ? leaf : 0u) + kModWord;
+    bool locked         = false;
+    if (lead) locked = !(atomicOr(mod, kLockBit) & kLockBit);
+    const uint32_t okm = warp.ballot(locked);
+    if (okm == 0) {
+      if (tries == 0) t0 = global_ns();
+      if (++tries >= T.ctl->spin_limit || wait_expired(t0, T.ctl->wait_ns, warp)) {
+        if (lead) T.set_error(kErrSpinLimit, 2);
+        return;
+      }
+      __nanosleep(backoff);
+      backoff = backoff < 1024 ? backoff * 2 : 1024;
+      continue;
+    }
+    tries   = 0;
+    backoff = 32;
+    __threadfence();
+    warp.sync();
+    const uint32_t upto = lm & ((2u << lane) - 1u);
+    const uint32_t boss = upto ? 31u - (uint32_t)__clz(upto) : 0u;  // the lane's leader
+    const bool have     = pend && ((okm >> boss) & 1u);
+    const uint32_t slot = (uint32_t)__popc(okm & ((1u << boss) - 1u));
+    const uint32_t nodes = (uint32_t)__popc(okm);
+    if (locked) st.idx[slot] = leaf;
+    warp.sync();
+    for (uint32_t s = lane >> 3; s < nodes; s += 4)
+      copy_16<true>(&st.node[s][(piece ^ (s & 7u)) << 2], T.node_ptr(st.idx[s]) + piece * 4);
+    copy_wait();
+    warp.sync();
+    // what each lane finds: its leaf, a leaf further right, or a stale route
+    bool cover = false, act = false, stale = false;
+    uint32_t high = 0, link = 0, nts = 0, ol = 0;
+    if (have) {
+      ld_shared_4(st.last_words(slot), high, link, nts, ol);
+      const uint32_t sib = link & kIndexMask;
+      if ((ol >> 28) != 0 || key < st.word(slot, 26)) {
+        stale = true;
+      } else if (key >= high && sib != kNone) {
+        leaf = sib;  // next round
+      } else {
+        cover            = true;
+        const uint32_t c = count_up_to(st, slot, key);
+        act              = (c && st.word(slot, 2 * c - 2) == key) ||
+              (!erase && st.word(slot, 2 * (kDataPairs - 1)) == kEmptyKey);
+      }
+    }
+    const uint32_t coverm = warp.ballot(cover), actm = warp.ballot(act);
+    const uint32_t after  = lm & ~((2u << lane) - 1u);  // leaders above this lane
+    const uint32_t mine   = (after ? (1u << (__ffs(after) - 1)) - 1u : 0xFFFFFFFFu) & ~((1u << lane) - 1u) & pm;
+    bool change           = locked && (actm & mine) != 0;  // (leaders) some op changes the leaf
+    const bool need       = change && T.versioned && nts != E;
+    const uint32_t copies = warp.ballot(need);
+    uint32_t copy         = kNone;
+    bool dropped          = false;  // no node for the version copy: the leaf's ops are given up
+    if (copies) {
+      copy = alloc_warp(T, need, warp);
+      if (need && copy == kNone) {
+        dropped = true;
+        change  = false;
+      }
+      if (locked) st.dst[slot] = copy;
+      warp.sync();
+      for (uint32_t s = lane >> 3; s < nodes; s += 4) {
+        const uint32_t dst = st.dst[s];
+        if (dst == kNone) continue;
+        uint32_t w[4];
+        ld_shared_4(&st.node[s][(piece ^ (s & 7u)) << 2], w[0], w[1], w[2], w[3]);
+        if (piece == kModWord / 4) w[kModWord % 4] = kRetiredBit | (E & kCountMask);  // read only at snapshots < E
+        store_16(T.node_ptr(dst) + piece * 4, w);
+      }
+      __threadfence();  // the copies are complete before a header names them
+      warp.sync();
+      retire_warp(T, copy != kNone, copy, warp);
+    }
+    const uint32_t changem = warp.ballot(change), dropm = warp.ballot(dropped);
+    if (change) {
+      if (copy != kNone) {
+        auto at = [&](uint32_t w) -> uint32_t& { return st.node[slot][(((w >> 2) ^ (slot & 7u)) << 2) | (w & 3u)]; };
+        at(30)  = E;
+        at(31)  = (ol & ~kIndexMask) | copy;
+      }
+      uint32_t n = count_up_to(st, slot, kEmptyKey - 1u);
+      for (uint32_t todo = coverm & mine; todo; todo &= todo - 1u) {
+        const uint32_t j = (uint32_t)__ffs(todo) - 1u;
+        st.done[j]       = apply_staged(st, slot, n, st.op[j][0], st.op[j][1], (erases >> j) & 1u) ? 1u : 0u;
+      }
+    }
+    if (locked) st.dst[slot] = change ? st.idx[slot] : kNone;
+    warp.sync();
+    for (uint32_t s = lane >> 3; s < nodes; s += 4) {
+      const uint32_t dst = st.dst[s];
+      if (dst == kNone) continue;
+      uint32_t w[4];
+      ld_shared_4(&st.node[s][(piece ^ (s & 7u)) << 2], w[0], w[1], w[2], w[3]);
+      store_16(T.node_ptr(dst) + piece * 4, w);
+    }
+    __threadfence();
+    warp.sync();
+    if (locked) {
+      if (change) atomicExch(mod, ((st.word(slot, kModWord) & kCountMask) + 1u) & kCountMask);
+      else atomicAnd(mod, ~kLockBit);
+    }
+    bool full = false;
+    if (cover) {
+      if ((changem >> boss) & 1u) full = st.done[lane] == 0;
+      else full = !((dropm >> boss) & 1u) && !erase;  // an erase that found nothing is done
+      pend = full;
+    }
+    // The tile path: stale routes, and one key of each full leaf, which splits it.
+    const uint32_t fullm = warp.ballot(full);
+    const bool first     = full && (fullm & ((1u << lane) - 1u) & ~((1u << boss) - 1u)) == 0;
+    for (uint32_t left = warp.ballot(stale || first); left;) {
+      uint32_t m = left;
+      for (uint32_t q = 0; q < lane / W; ++q) m &= m - 1u;
+      const bool run     = m != 0;  // the same in every lane of a tile
+      const int src      = run ? __ffs(m) - 1 : 0;
+      const uint32_t k   = warp.shfl(key, src), v = warp.shfl(value, src), to = warp.shfl(leaf, src);
+      if (run) write_tile<W>(T, k, v, (erases >> src) & 1u, E, to, tile);
+      for (uint32_t q = 0; q < kTiles; ++q) left &= left - 1u;
+      warp.sync();
+    }
+    if (stale || first) pend = false;
+    warp.sync();
+  }
+  if (pend) T.set_error(kErrStepLimit, 11);
 }
 
 // ----------------------------------------------------------------------------------------------

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(256) k_find(device_tree T, const uint32_t* __r
 constexpr int kReadSortLowBit   = 8;  // reads: order by the top 24 bits (locality is all they need)
 constexpr uint32_t kUnsortedBits = (1u << kReadSortLowBit) - 1u;
 constexpr int kWarpsPerBlock    = 8;
+constexpr int kSlowTile         = 8;  // tile of a warp's rare writes one by one (write_tile)
 template <bool kSorted>
 __global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t* __restrict__ keys,
                                                    const uint32_t* __restrict__ spos, uint32_t* __restrict__ out,
@@ -354,22 +355,38 @@ __device__ __forceinline__ bool superseded(const uint32_t* skeys, uint64_t i, ui
   return i + 1 < n && skeys[i + 1] == skeys[i];
 }
 
-template <int W>
-__global__ void __launch_bounds__(256, 6) k_insert_sorted(device_tree T, const uint32_t* __restrict__ skeys,
+// Inserts (kErase: erases), 32 per warp at a time (mvbt::write_warp). kSorted: the keys are a sorted
+// call's with values at their input positions, and each warp takes one contiguous run of them.
+template <bool kSorted, bool kErase>
+__global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint32_t* __restrict__ keys,
                                                        const uint32_t* __restrict__ spos,
                                                        const uint32_t* __restrict__ values, uint32_t n) {
-  auto tile        = cg::tiled_partition<W>(cg::this_thread_block());
-  const uint32_t E = T.versioned ? T.current_epoch() : 0u;
-  uint64_t i, end;
-  tile_run<W>(n, i, end);
-  mvbt::finger<W> f;
-  while (warp_any(i < end)) {
-    if (i >= end) continue;
-    if (superseded(skeys, i, n)) {
-      ++i;
-      continue;
+  __shared__ mvbt::write_stage stage[kWarpsPerBlock];
+  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
+  auto tile             = cg::tiled_partition<kSlowTile>(cg::this_thread_block());
+  mvbt::write_stage& st = stage[threadIdx.x >> 5];
+  const uint32_t lane   = threadIdx.x & 31u;
+  const uint32_t E      = T.versioned ? T.current_epoch() : 0u;
+  const uint64_t warps  = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint64_t w      = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t groups = ((uint64_t)n + 31) / 32;
+  const uint64_t per    = (groups + warps - 1) / warps;
+  uint64_t g            = kSorted ? w * per : w;
+  const uint64_t end    = kSorted ? (g + per < groups ? g + per : groups) : groups;
+  if (kSorted) mvbt::clear_path(st, warp);
+  for (; g < end; g += kSorted ? 1 : warps) {
+    const uint64_t i = g * 32 + lane;
+    const bool has   = i < n;
+    const uint32_t k = has ? keys[i] : 0u;
+    const bool live  = has && !(kSorted && superseded(keys, i, n));
+    uint32_t v       = 0;
+    if (!kErase && live) v = values[kSorted ? spos[i] : i];
+    uint32_t start = mvbt::kAnchor;
+    if (kSorted) {
+      const uint32_t m = __ballot_sync(0xffffffffu, has);
+      start = mvbt::path_start(st, __shfl_sync(0xffffffffu, k, 0), __shfl_sync(0xffffffffu, k, 31 - __clz(m)), warp);
     }
-    T.insert_run_group<W>(skeys, spos, values, i, end, n, tile, E, f);
+    mvbt::write_warp<kSlowTile>(T, k, v, kErase, live, E, start, kSorted, st, warp, tile);
   }
 }
 
@@ -390,18 +407,6 @@ __global__ void __launch_bounds__(256) k_insert_spread(device_tree T, const uint
     if (superseded(skeys, i, n)) continue;
     T.cooperative_insert<W>(skeys[i], values[spos[i]], tile, E);
   }
-}
-
-template <int W>
-__global__ void __launch_bounds__(256) k_erase_sorted(device_tree T, const uint32_t* __restrict__ skeys,
-                                                      uint32_t n) {
-  auto tile        = cg::tiled_partition<W>(cg::this_thread_block());
-  const uint32_t E = T.versioned ? T.current_epoch() : 0u;
-  uint64_t i, end;
-  tile_run<W>(n, i, end);
-  mvbt::finger<W> f;
-  for (; warp_any(i < end); ++i)
-    if (i < end) T.erase_in_run<W>(skeys[i], tile, E, f);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -448,7 +453,8 @@ int status_from_bits(uint32_t bits) {
 
 // Fewer lookups than this leave most warps of k_find_warp empty; a tile per key has the shorter
 // chain then.
-constexpr uint32_t kWarpFindMin = 1u << 13;
+constexpr uint32_t kWarpFindMin  = 1u << 13;
+constexpr uint32_t kWarpWriteMin = 1u << 13;  // writes likewise
 
 // Bulk insert of n keys. On a tree that is small against the batch, the tiles of a full grid
 // would queue on the few leaves there are, and every handoff of a queued lock costs an atomic per
@@ -465,8 +471,14 @@ int insert_launches(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, 
     uint64_t blocks = std::max<uint64_t>(1, (t->grown / 10) / tiles);
     uint64_t chunk  = n - done;
     if (blocks < full) chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(t->grown, blocks * tiles * 16));
-    blocks = std::min(blocks, full);
-    k_insert<W><<<(unsigned)blocks, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);
+    if (blocks >= full && chunk >= kWarpWriteMin) {  // the rest in one launch, 32 keys a warp
+      const uint64_t in_flight = std::max<uint64_t>(1, (t->grown / 10) / t->block_size);  // about a key per leaf
+      const unsigned grid      = (unsigned)std::min<uint64_t>(grid_for_warps(t, k_write_warp<false, false>, chunk), in_flight);
+      k_write_warp<false, false><<<grid, t->block_size, 0, s>>>(t->view(), keys + done, nullptr, values + done, (uint32_t)chunk);
+    } else {
+      blocks = std::min(blocks, full);
+      k_insert<W><<<(unsigned)blocks, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);
+    }
     int st = check_launch();
     if (st) return st;
     done += chunk;
@@ -557,7 +569,7 @@ int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaSt
 
 template <int W>
 int insert_sorted_launches(mvbt_tree* t, const sorted_ops& so, const uint32_t* values, uint32_t n, cudaStream_t s) {
-  const uint64_t full  = grid_for(t, k_insert_sorted<W>, n);
+  const uint64_t full  = grid_for(t, k_insert_spread<W>, n);
   const uint64_t tiles = (uint64_t)t->block_size / W;
   uint64_t spread      = 0;
   while (t->grown / 10 < full * tiles && spread < n) {  // fewer leaves than tiles: spread first
@@ -571,7 +583,7 @@ int insert_sorted_launches(mvbt_tree* t, const sorted_ops& so, const uint32_t* v
     spread = m;
   }
   if (spread < n) {
-    k_insert_sorted<W><<<(unsigned)full, t->block_size, 0, s>>>(t->view(), so.keys, so.pos, values, n);
+    k_write_warp<true, false><<<grid_for_warps(t, k_write_warp<true, false>, n), t->block_size, 0, s>>>(t->view(), so.keys, so.pos, values, n);
     int st = check_launch();
     if (st) return st;
     t->grown += n - spread;
@@ -1240,15 +1252,14 @@ int mvbt_erase(mvbt_tree* t, const uint32_t* keys, uint32_t n, void* stream, int
     sorted_ops so;
     int st = sort_ops(t, keys, n, 0, s, &so);
     if (st) return st;
-    if (t->tile_width == 8)
-      k_erase_sorted<8><<<grid_for(t, k_erase_sorted<8>, n), t->block_size, 0, s>>>(t->view(), so.keys, n);
-    else
-      k_erase_sorted<16><<<grid_for(t, k_erase_sorted<16>, n), t->block_size, 0, s>>>(t->view(), so.keys, n);
+    k_write_warp<true, true><<<grid_for_warps(t, k_write_warp<true, true>, n), t->block_size, 0, s>>>(t->view(), so.keys, nullptr, nullptr, n);
     st = check_launch();
     const int rs = so.release(s);
     return st ? st : rs;
   }
-  if (t->tile_width == 8) {
+  if (n >= kWarpWriteMin) {
+    k_write_warp<false, true><<<grid_for_warps(t, k_write_warp<false, true>, n), t->block_size, 0, s>>>(t->view(), keys, nullptr, nullptr, n);
+  } else if (t->tile_width == 8) {
     k_erase<8><<<grid_for(t, k_erase<8>, n), t->block_size, 0, s>>>(t->view(), keys, n);
   } else {
     k_erase<16><<<grid_for(t, k_erase<16>, n), t->block_size, 0, s>>>(t->view(), keys, n);

@@ -28,6 +28,7 @@ def lib():
             "emu_erase": (None, [vp, u32p, u64, i, i]),
             "emu_find": (None, [vp, u32p, u32p, u64, u32, i, i, i]),
             "emu_find_warp": (None, [vp, u32p, u32p, u32p, u64, u32, i, u32, i, u32]),
+            "emu_write_warp": (None, [vp, u32p, u32p, u32p, u64, i, i, i]),
             "emu_range": (None, [vp, u32p, u32p, vp, vp, u32, u64, u32, i, i, i]),
             "emu_insert_range": (None, [vp, u32p, u32p, u64, u32p, u32p, u64, vp, vp, u32, i, i]),
             "emu_find_erase": (None, [vp, u32p, u32p, u64, u32p, u64, i, i]),
@@ -109,6 +110,15 @@ class EmuTree:
         self.L.emu_find_warp(self.h, np.ascontiguousarray(k[order]), order, out, k.size, ts, warps, lanes, int(sorted_run),
                              (1 << (32 - bits)) - 1)
         return out
+
+    def write_warp(self, kind, keys, vals, warps=2, sorted_run=False):
+        """Warp writes: kind 1 insert, 2 erase per op; sorted_run: in key order (stable) with path memory, the
+        last op of a repeated key alone."""
+        kind, k, v = _u32(kind), _u32(keys), _u32(vals)
+        if sorted_run:
+            order = np.argsort(k, kind="stable")
+            kind, k, v = (np.ascontiguousarray(x[order]) for x in (kind, k, v))
+        self.L.emu_write_warp(self.h, kind, k, v, k.size, warps, self.W, int(sorted_run))
 
     def range(self, lo, hi, avg_len, ts=0xFFFFFFFF, quiescent=False):
         lo, hi = _u32(lo), _u32(hi)

@@ -253,6 +253,37 @@ void emu_find_warp(void* h, const uint32_t* keys, const uint32_t* pos, uint32_t*
   });
 }
 
+// Warp writes (write_warp), 32 ops per warp at a time over `warps` warps: kind 1 insert, 2 erase.
+// sorted != 0: the ops are in key order, each warp takes a contiguous run with its path memory, and of
+// a repeated key the last op alone is run.
+void emu_write_warp(void* h, const uint32_t* kind, const uint32_t* keys, const uint32_t* vals, uint64_t n, int warps,
+                    int W, int sorted) {
+  auto* t = static_cast<emu_tree*>(h);
+  auto v  = t->view();
+  const uint32_t E      = v.versioned ? v.current_epoch() : 0u;
+  const uint64_t groups = (n + 31) / 32, per = (groups + warps - 1) / warps;
+  std::vector<mvbt::write_stage> stage(warps);
+  EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {
+    const uint64_t w = mvbt::emu::sm;
+    auto& st         = stage[w];
+    uint64_t g       = sorted ? w * per : w;
+    const uint64_t end = sorted ? std::min(g + per, groups) : groups;
+    if (sorted) mvbt::clear_path(st, warp);
+    for (; g < end; g += sorted ? 1 : warps) {
+      const uint64_t i = g * 32 + warp.thread_rank();
+      const bool has   = i < n;
+      const uint32_t k = has ? keys[i] : 0u;
+      const bool live  = has && !(sorted && i + 1 < n && keys[i + 1] == k);
+      uint32_t start   = mvbt::kAnchor;
+      if (sorted) {
+        const uint32_t m = warp.ballot(has);
+        start = mvbt::path_start(st, warp.shfl(k, 0), warp.shfl(k, 31 - __clz(m)), warp);
+      }
+      mvbt::write_warp<kW>(v, k, has ? vals[i] : 0u, has && kind[i] == 2, live, E, start, sorted != 0, st, warp, tile);
+    }
+  }));
+}
+
 // quiescent != 0: the range query of a tree no writer changes meanwhile (range_quiescent).
 void emu_range(void* h, const uint32_t* lo, const uint32_t* hi, uint32_t* pairs, uint32_t* counts,
                uint32_t avg_len, uint64_t n, uint32_t ts, int tiles, int W, int quiescent) {

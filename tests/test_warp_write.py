@@ -6,9 +6,9 @@ import numpy as np
 import pytest
 
 
-@pytest.mark.parametrize("w", [8, 16])
-@pytest.mark.parametrize("versioned,reclaim,chunk", [(False, False, 64), (True, False, 64), (True, True, 32), (True, False, 8)])
-@pytest.mark.parametrize("sorted_run", [False, True])
+@pytest.mark.parametrize("w,versioned,reclaim,chunk,sorted_run", [
+    (8, False, False, 64, False), (16, False, False, 64, True), (8, True, True, 64, False), (16, True, True, 32, True),
+    (8, True, False, 8, True)])
 def test_emulated_warp_writes_match_oracle(w, versioned, reclaim, chunk, sorted_run):
     from emu import EmuTree
     import oracle
