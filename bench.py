@@ -70,7 +70,7 @@ def parse_args():
     ap.add_argument("--seed", type=int, default=20240611)
     ap.add_argument("--tile-width", type=int, default=8)
     ap.add_argument("--blocks-per-sm", type=int, default=0,
-                    help="0 = full occupancy of the default kernel; 6 / 8 = register-capped variants")
+                    help="0 = full occupancy (4 blocks); a smaller number caps it")
     ap.add_argument("--e2e-steps", type=int, default=12,
                     help="timed steps of the end-to-end pipeline (two in flight; more steps amortise its fill and drain)")
     ap.add_argument("--pool-gb", type=float, default=30.0,

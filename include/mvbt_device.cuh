@@ -160,6 +160,7 @@ constexpr uint32_t kCountMask  = 0x1FFFFFFFu;  // count (live node) or epoch (re
 constexpr int kModWord         = 27;
 constexpr uint32_t kRingChunk  = 0x80000000u;  // per-SM chunk base: positions in the free ring
 constexpr uint32_t kRingEmpty  = 0xFFFFFFFFu;  // a free-ring slot not written yet (or read already)
+constexpr uint32_t kReclaimClaim = 64;        // log positions a warp reclaims at once inside a launch
 constexpr uint32_t kReclaimAll = 0xFFFFFFFFu;  // reclaim watermark: the current epoch
 constexpr uint32_t kAnchor    = 0;  // fixed entry node: one entry {0 -> top}, level = top + 1
 constexpr uint32_t kFirstLeaf = 1;  // the initial leaf (holds the tombstone {0, 0})
@@ -315,6 +316,7 @@ MVBT_DEV unsigned long long global_ns() {
       .count();
 }
 MVBT_DEV uint32_t ld_relaxed_u32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
+MVBT_DEV uint32_t ld_block_u32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
 MVBT_DEV void st_relaxed_u32(uint32_t* p, uint32_t v) { __atomic_store_n(p, v, __ATOMIC_RELAXED); }
 MVBT_DEV unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   return __atomic_load_n(p, __ATOMIC_RELAXED);
@@ -369,6 +371,8 @@ MVBT_DEV unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(r) : "l"(p) : "memory");
   return r;
 }
+// A word of shared memory that other warps of the block change.
+MVBT_DEV uint32_t ld_block_u32(const uint32_t* p) { return *reinterpret_cast<const volatile uint32_t*>(p); }
 MVBT_DEV void st_relaxed_u32(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" : : "l"(p), "r"(v) : "memory");
 }
@@ -783,8 +787,10 @@ MVBT_DEV bool take_free_chunk(control_block* c, uint32_t C, uint32_t& base) {
 // ring's previous lap has not yet read), then one fence and the count published in free_avail.
 // ring_cap >= capacity + kMaxSmSlots * chunk: the entries written and not yet read (free nodes,
 // and the rest of per-SM chunks taken from the ring) never fill the ring, so a pusher meets a
-// slot of the previous lap only while its reader is about to clear it.
-template <class Warp>
+// slot of the previous lap only while its reader is about to clear it -- or while it is the unread
+// rest of the chunk of an SM that has stopped allocating, which flush_chunk returns in time.
+// kCount: the nodes were freed just now (stat_reclaimed).
+template <bool kCount = true, class Warp>
 MVBT_DEV void ring_push(control_block* c, bool freed, uint32_t node, const Warp& warp) {
   const uint32_t m = warp.ballot(freed);
   if (!m) return;
@@ -804,8 +810,51 @@ MVBT_DEV void ring_push(control_block* c, bool freed, uint32_t node, const Warp&
   warp.sync();
   if ((int)lane == lead) {
     atomicAdd(&c->free_avail, (unsigned long long)__popc(m));
-    atomicAdd(&c->stat_reclaimed, (unsigned long long)__popc(m));
+    if (kCount) atomicAdd(&c->stat_reclaimed, (unsigned long long)__popc(m));
   }
+}
+// Returns the unread rest of SM slot `sm`'s chunk to the free ring if the chunk is a run of ring
+// positions that lies `behind` or more positions behind the ring's tail (warp-collective). Without it
+// an SM that took a chunk and then stopped allocating would keep its positions unread until the ring's
+// tail comes round, and the pushers that meet them would wait out their limit.
+template <class Warp>
+MVBT_DEV void flush_chunk(control_block* c, uint32_t sm, uint32_t behind, const Warp& warp) {
+  unsigned long long* slot = &c->sm_pool[sm];
+  const uint32_t C         = c->chunk;
+  unsigned long long cur   = 0;
+  uint32_t take            = 0;
+  if (warp.thread_rank() == 0) {
+    cur                 = ld_relaxed_u64(slot);
+    const uint32_t base = (uint32_t)(cur >> 32), used = (uint32_t)cur;
+    const uint32_t lag  = ((uint32_t)ld_relaxed_u64(&c->free_tail) - (base & ~kRingChunk)) & (c->ring_cap - 1u);
+    // used up without taking the refill on: the next request refills it
+    if ((base & kRingChunk) && used < C && lag >= behind &&
+        atomicCAS(slot, cur, (cur & 0xFFFFFFFF00000000ull) | C) == cur)
+      take = C - used;
+  }
+  take = warp.shfl(take, 0);
+  if (take == 0) return;
+  cur = warp.shfl(cur, 0);
+  const uint32_t base = (uint32_t)(cur >> 32), used = (uint32_t)cur;
+  for (uint32_t j = 0; j < take; j += 32) {  // read (and clear) before pushing: no pusher waits for this warp
+    const uint32_t at = j + warp.thread_rank();
+    uint32_t node     = kNone;
+    if (at < take) {
+      node = chunk_node(c, base, used + at);
+      atomicAdd(&c->sm_stats[sm_id() % kMaxSmSlots][2], (unsigned long long)-1ll);  // not handed out after all
+    }
+    ring_push<false>(c, node != kNone, node, warp);
+  }
+}
+// flush_chunk of all SM slots: warp w looks at slots [32 w, 32 w + 32), a lane at each.
+template <class Warp>
+MVBT_DEV void flush_chunks(control_block* c, uint32_t w, uint32_t behind, const Warp& warp) {
+  if (w >= (uint32_t)kMaxSmSlots / 32) return;
+  const unsigned long long cur = ld_relaxed_u64(&c->sm_pool[32 * w + warp.thread_rank()]);
+  const uint32_t base = (uint32_t)(cur >> 32);
+  const uint32_t lag  = ((uint32_t)ld_relaxed_u64(&c->free_tail) - (base & ~kRingChunk)) & (c->ring_cap - 1u);
+  for (uint32_t m = warp.ballot((base & kRingChunk) && (uint32_t)cur < c->chunk && lag >= behind); m; m &= m - 1u)
+    flush_chunk(c, 32 * w + (uint32_t)__ffs(m) - 1u, behind, warp);
 }
 // Records a version copy in the retire log. A copy the full log cannot take is never freed
 // (counted in stat_log_dropped).
@@ -1080,8 +1129,8 @@ struct device_tree {
     c->retire_head      = head + (keep == 0xFFFFFFFFu ? n : keep);
     c->rc_first_kept    = 0xFFFFFFFFu;
   }
-  // Reclamation while kernels run (warp-collective): claims up to 32 retire-log positions below
-  // `limit` -- positions the caller knows hold only copies that no live snapshot reads -- frees
+  // Reclamation while kernels run (warp-collective): claims up to kReclaimClaim retire-log positions
+  // below `limit` -- positions the caller knows hold only copies that no live snapshot reads -- frees
   // their copies and appends them to the free ring. Returns the number of positions claimed.
   template <class Warp>
   MVBT_DEV uint32_t reclaim_online(unsigned long long limit, const Warp& warp) const {
@@ -1093,7 +1142,7 @@ struct device_tree {
       const unsigned long long tail = ld_relaxed_u64(&c->retire_tail);
       if (limit > tail) limit = tail;  // never past the entries reserved so far
       if (h < limit) {
-        n = (uint32_t)(limit - h < 32 ? limit - h : 32);
+        n = (uint32_t)(limit - h < kReclaimClaim ? limit - h : kReclaimClaim);
         if (atomicCAS(&c->retire_head, h, h + n) != h) n = 0;  // another warp took them
       }
     }
@@ -1101,10 +1150,12 @@ struct device_tree {
     n = warp.shfl(n, 0);
     if (n == 0) return 0;
     __threadfence();  // the copies' last readers finished before `limit` was published
-    const uint32_t lane = warp.thread_rank();
-    uint32_t idx        = kNone;
-    const bool freed    = lane < n && reclaim_entry(h + lane, 0, idx, false) == 1;
-    ring_push(c, freed, idx, warp);
+    for (uint32_t j = 0; j < n; j += 32) {
+      const uint32_t at = j + warp.thread_rank();
+      uint32_t idx      = kNone;
+      const bool freed  = at < n && reclaim_entry(h + at, 0, idx, false) == 1;
+      ring_push(c, freed, idx, warp);
+    }
     return n;
   }
 
@@ -1976,7 +2027,6 @@ struct alignas(16) warp_stage {
   uint32_t node[32][kNodeWords];  // 16-byte pieces of node s at piece ^ (s & 7): the lanes' reads
                                   // of one word of different nodes spread over the banks
   uint32_t idx[32];               // the nodes to copy
-  uint32_t path[kMaxLevels][4];   // last key's node per level {index, low, high}: the next keys' start
   // Word w of staged node s, and its words 28..31.
   MVBT_DEV uint32_t word(uint32_t s, uint32_t w) const { return node[s][(((w >> 2) ^ (s & 7u)) << 2) | (w & 3u)]; }
   MVBT_DEV const uint32_t* last_words(uint32_t s) const { return &node[s][(7u ^ (s & 7u)) << 2]; }
@@ -1992,24 +2042,29 @@ MVBT_DEV void ld_shared_4(const uint32_t* p, uint32_t& a, uint32_t& b, uint32_t&
 }
 #endif
 
-template <class Warp>
-MVBT_DEV void clear_path(warp_stage& st, const Warp& warp) {
-  const uint32_t lane = warp.thread_rank();
-  if (lane < (uint32_t)kMaxLevels) {
-    st.path[lane][0] = kNone;
-    st.path[lane][1] = kEmptyKey;  // covers nothing
-    st.path[lane][2] = 0;
+// Path memory of a warp that runs keys in ascending order: the last key's node per level
+// {index, low, high}, from which the next keys start.
+struct warp_path {
+  uint32_t at[kMaxLevels][3];
+  template <class Warp>
+  MVBT_DEV void clear(const Warp& warp) {
+    const uint32_t lane = warp.thread_rank();
+    if (lane < (uint32_t)kMaxLevels) record(lane, kNone, kEmptyKey, 0);  // covers nothing
+    warp.sync();
   }
-  warp.sync();
-}
-
-// Lowest remembered node that covers all of [first, last], or the anchor. Every lane looks at a level.
-template <class Warp>
-MVBT_DEV uint32_t path_start(const warp_stage& st, uint32_t first, uint32_t last, const Warp& warp) {
-  const uint32_t l  = warp.thread_rank() & (kMaxLevels - 1u);
-  const uint32_t in = warp.ballot(st.path[l][1] <= first && last < st.path[l][2]);
-  return in ? st.path[__ffs(in) - 1][0] : kAnchor;
-}
+  MVBT_DEV void record(uint32_t level, uint32_t idx, uint32_t low, uint32_t high) {
+    at[level][0] = idx;
+    at[level][1] = low;
+    at[level][2] = high;
+  }
+  // Lowest remembered node that covers all of [first, last], or the anchor. Every lane looks at a level.
+  template <class Warp>
+  MVBT_DEV uint32_t start(uint32_t first, uint32_t last, const Warp& warp) const {
+    const uint32_t l  = warp.thread_rank() & (kMaxLevels - 1u);
+    const uint32_t in = warp.ballot(at[l][1] <= first && last < at[l][2]);
+    return in ? at[__ffs(in) - 1][0] : kAnchor;
+  }
+};
 
 // Copies the nodes idx of the live lanes (m) into st, neighbouring lanes' equal ones once; returns
 // the lane's slot. The caller keeps every lane's reads of the last nodes before this (warp.sync).
@@ -2041,18 +2096,18 @@ MVBT_DEV uint32_t count_up_to(const warp_stage& st, uint32_t s, uint32_t key) {
 }
 
 // The value of each live lane's key at snapshot ts (kLatest: newest), kNotFound elsewhere; the
-// route and results of find_quiescent. start: a node on every live key's route (the anchor, or
-// path_start). keep_path: the nodes that the highest live lane passes are remembered for it.
+// route and results of find_quiescent. start: a node on the key's route (the anchor, or path->start).
+// path (nullable): the nodes that the highest live lane passes are recorded in it.
 template <class Warp>
 MVBT_DEV uint32_t find_warp(const device_tree& T, uint32_t key, bool live, uint32_t ts, uint32_t start,
-                            bool keep_path, warp_stage& st, const Warp& warp) {
+                            warp_path* path, warp_stage& st, const Warp& warp) {
   const bool snap     = T.versioned && ts != kLatest;
   const uint32_t lane = warp.thread_rank();
   uint32_t found      = kNotFound;
   uint32_t idx        = start;
   live                = live && key != kEmptyKey;
   const uint32_t all  = warp.ballot(live);
-  const bool last     = keep_path && live && (all >> lane) == 1u;
+  const bool last     = path && live && (all >> lane) == 1u;
   for (uint32_t step = 0; step < kMaxSteps; ++step) {
     if (live && idx >= T.capacity) {
       T.set_error(kErrCorrupt, 1);
@@ -2078,11 +2133,7 @@ MVBT_DEV uint32_t find_warp(const device_tree& T, uint32_t key, bool live, uint3
         idx = link;
       } else {
         const uint32_t level = ol >> 28;
-        if (last) {
-          st.path[level][0] = idx;
-          st.path[level][1] = low;
-          st.path[level][2] = high;
-        }
+        if (last) path->record(level, idx, low, high);
         const uint32_t c  = count_up_to(st, slot, key);
         const uint32_t pk = c ? st.word(slot, 2 * c - 2) : kEmptyKey;
         const uint32_t pv = c ? st.word(slot, 2 * c - 1) : kAnchor;
@@ -2100,25 +2151,99 @@ MVBT_DEV uint32_t find_warp(const device_tree& T, uint32_t key, bool live, uint3
   return found;
 }
 
+// find_warp at snapshot ts (of each lane) while writers run in the same kernel: cooperative_find's
+// route and checks. start: a node on the key's route, as read at the newest state.
+template <class Warp>
+MVBT_DEV uint32_t find_warp_live(const device_tree& T, uint32_t key, bool live, uint32_t ts, uint32_t start,
+                                 warp_stage& st, const Warp& warp) {
+  uint32_t found = kNotFound;
+  uint32_t idx   = start;
+  bool copy      = false;  // idx is an older version, which is never written again
+  live           = live && key != kEmptyKey;
+  for (uint32_t step = 0; step < kMaxSteps; ++step) {
+    if (live && idx >= T.capacity) {
+      T.set_error(kErrCorrupt, 1);
+      live = false;
+    }
+    const uint32_t m = warp.ballot(live);
+    if (m == 0) return found;
+    const uint32_t slot = stage_nodes<true>(T, idx, live, m, st, warp);
+    bool check          = false;  // the leaf of the snapshot, unless a writer is changing it
+    uint32_t value      = kNotFound;
+    if (live) {
+      const uint32_t low = st.word(slot, 26);
+      uint32_t high, link, nts, ol;
+      ld_shared_4(st.last_words(slot), high, link, nts, ol);
+      link &= kIndexMask;
+      if (nts > ts) {
+        idx  = ol & kIndexMask;
+        copy = true;
+        if (idx == kNone) {
+          T.set_error(kErrCorrupt, 3);
+          live = false;
+        }
+      } else if (key < low) {
+        idx  = kAnchor;
+        copy = false;
+      } else if (key >= high && link != kNone) {
+        idx  = link;
+        copy = false;
+      } else {
+        const uint32_t c  = count_up_to(st, slot, key);
+        const uint32_t pk = c ? st.word(slot, 2 * c - 2) : kEmptyKey;
+        const uint32_t pv = c ? st.word(slot, 2 * c - 1) : kAnchor;
+        if ((ol >> 28) == 0) {
+          if (pk == key) value = pv;
+          check = !copy;
+          live  = check;
+          found = value;
+        } else {
+          idx  = pv;
+          copy = false;
+        }
+      }
+    }
+    if (warp.ballot(check)) {  // as recheck_version
+      __threadfence();
+      warp.sync();
+      if (check) {
+        const uint32_t* node = T.node_ptr(idx);
+        const uint32_t mod0 = st.word(slot, kModWord), mod1 = ld_relaxed_u32(node + kModWord);
+        const unsigned long long v = ld_relaxed_u64(reinterpret_cast<const unsigned long long*>(node + 30));
+        if ((uint32_t)v > ts) {  // changed meanwhile: its immutable copy instead
+          idx  = (uint32_t)(v >> 32) & kIndexMask;
+          copy = true;
+        } else if (!(mod0 & kLockBit) && mod1 == mod0) {
+          live = false;
+        } else {
+          __nanosleep(64);  // a writer is changing it: read it again
+        }
+      }
+    }
+    warp.sync();
+  }
+  if (live) T.set_error(kErrStepLimit, 4);
+  return found;
+}
+
 // ----------------------------------------------------------------------------------------------
 // Writes of a whole warp
 // ----------------------------------------------------------------------------------------------
 struct write_stage : warp_stage {
-  uint32_t op[32][2];  // each lane's {key, value}
-  uint32_t done[32];   // 1: the lane's op was applied, 0: its leaf is full
+  uint32_t op[32][2];  // each lane's {key, value}; once tried, whether its leaf was full in place of the key
   uint32_t dst[32];    // where each staged node is stored (kNone: nowhere)
 };
 
 // The leaf that each live lane's key belongs to, unread: the child its level-1 node names (kNone:
 // failed). Routing at the newest state while writers run, as descend_for_write.
 template <class Warp>
-MVBT_DEV uint32_t leaf_warp(const device_tree& T, uint32_t key, bool live, uint32_t start, bool keep_path,
+MVBT_DEV uint32_t leaf_warp(const device_tree& T, uint32_t key, bool live, uint32_t start, warp_path* path,
                             warp_stage& st, const Warp& warp) {
   const uint32_t lane = warp.thread_rank();
   uint32_t leaf       = kNone;
   uint32_t idx        = start;
   const uint32_t all  = warp.ballot(live);
-  const bool last     = keep_path && live && (all >> lane) == 1u;
+  const bool last     = path && live && (all >> lane) == 1u;
   for (uint32_t step = 0; step < kMaxSteps; ++step) {
     if (live && idx >= T.capacity) {
       T.set_error(kErrCorrupt, 1);
@@ -2141,11 +2266,7 @@ MVBT_DEV uint32_t leaf_warp(const device_tree& T, uint32_t key, bool live, uint3
         leaf = idx;
         live = false;
       } else {
-        if (last) {
-          st.path[level][0] = idx;
-          st.path[level][1] = low;
-          st.path[level][2] = high;
-        }
+        if (last) path->record(level, idx, low, high);
         const uint32_t c = count_up_to(st, slot, key);
         idx              = c ? st.word(slot, 2 * c - 1) : kAnchor;
         if (c && level == 1) {
@@ -2160,8 +2281,8 @@ MVBT_DEV uint32_t leaf_warp(const device_tree& T, uint32_t key, bool live, uint3
   return leaf;
 }
 
-// A fresh node for each lane with `need` set (kNone: the pool is full or the wait limit ran out): one
-// atomic of the warp on the SM's chunk cursor instead of one per node.
+// A fresh node for each lane with `need` set (kNone: the pool is full or the wait limit ran out): the
+// warp's nodes with one atomic on the SM's chunk cursor instead of one per node.
 template <class Warp>
 MVBT_DEV uint32_t alloc_warp(const device_tree& T, bool need, const Warp& warp) {
   const uint32_t m = warp.ballot(need);
@@ -2291,19 +2412,16 @@ MVBT_CALL void write_tile(device_tree T, uint32_t key, uint32_t value, bool eras
 // leaf stored, release. No lane waits for a lock while the warp holds one: leaves found locked are
 // tried again after the others are released. A leaf without room for a new key is split by the tile
 // path (one key per leaf at a time), and the leaf's other keys go on from there.
-// start / keep_path: as in find_warp. Two live lanes may hold one key only if either order will do.
+// leaf: each live lane's leaf as leaf_warp found it, possibly stale (kNone: the op is given up). Two
+// live lanes may hold one key only if either order will do.
 template <int W, class Warp, class Tile>
 MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, bool erase, bool live, uint32_t E,
-                         uint32_t start, bool keep_path, write_stage& st, const Warp& warp, const Tile& tile) {
+                         uint32_t leaf, write_stage& st, const Warp& warp, const Tile& tile) {
   constexpr uint32_t kTiles = 32 / W;
   const uint32_t lane       = warp.thread_rank();
   const uint32_t piece      = lane & 7u;
-  live                      = live && key != kEmptyKey;
-  uint32_t leaf             = leaf_warp(T, key, live, start, keep_path, st, warp);
-  bool pend                 = live && leaf != kNone;
+  bool pend                 = live && key != kEmptyKey && leaf != kNone;
   const uint32_t erases     = warp.ballot(erase);
-  st.op[lane][0]            = key;
-  st.op[lane][1]            = value;
   uint32_t tries = 0, backoff = 32;
   unsigned long long t0     = 0;
   for (uint32_t step = 0; step < kMaxSteps; ++step) {
@@ -2341,6 +2459,8 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
     const uint32_t slot = (uint32_t)__popc(okm & ((1u << boss) - 1u));
     const uint32_t nodes = (uint32_t)__popc(okm);
     if (locked) st.idx[slot] = leaf;
+    st.op[lane][0] = key;
+    st.op[lane][1] = value;
     warp.sync();
     for (uint32_t s = lane >> 3; s < nodes; s += 4)
       copy_16<true>(&st.node[s][(piece ^ (s & 7u)) << 2], T.node_ptr(st.idx[s]) + piece * 4);
@@ -2401,7 +2521,7 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
       uint32_t n = count_up_to(st, slot, kEmptyKey - 1u);
       for (uint32_t todo = coverm & mine; todo; todo &= todo - 1u) {
         const uint32_t j = (uint32_t)__ffs(todo) - 1u;
-        st.done[j]       = apply_staged(st, slot, n, st.op[j][0], st.op[j][1], (erases >> j) & 1u) ? 1u : 0u;
+        st.op[j][0]      = apply_staged(st, slot, n, st.op[j][0], st.op[j][1], (erases >> j) & 1u) ? 0u : 1u;
       }
     }
     if (locked) st.dst[slot] = change ? st.idx[slot] : kNone;
@@ -2421,7 +2541,7 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
     }
     bool full = false;
     if (cover) {
-      if ((changem >> boss) & 1u) full = st.done[lane] == 0;
+      if ((changem >> boss) & 1u) full = st.op[lane][0] != 0;
       else full = !((dropm >> boss) & 1u) && !erase;  // an erase that found nothing is done
       pend = full;
     }
@@ -2492,43 +2612,6 @@ MVBT_DEV bool run_batch_op(const device_tree& T, const batch_view& B, uint64_t i
   return write;
 }
 
-// An op whose batch is not ready yet does its descent first (routing at the newest state; nothing
-// it returns depends on the batches still running), then waits, then finishes from the leaf it
-// found: run_batch_op_at. Readers start their snapshot read at that leaf -- its low fence is fixed
-// for life, a node made after the snapshot leads to the version the snapshot reads through its
-// older pointer, and the fence checks move right or restart as needed -- and writers lock the
-// covering leaf from it. Returns the leaf (kNone: fall back to the whole op).
-template <int W, class Tile>
-MVBT_DEV uint32_t batch_op_descend(const device_tree& T, const batch_view& B, uint64_t i, uint32_t& path0,
-                                   uint32_t& path1, uint32_t& top, const Tile& t) {
-  const uint32_t k = B.key[i];
-  if (k == kEmptyKey) return kNone;
-  return T.descend_for_write<W>(k, path0, path1, top, t);
-}
-
-template <int W, class Tile>
-MVBT_DEV bool run_batch_op_at(const device_tree& T, const batch_view& B, uint64_t i, uint32_t S, uint32_t E,
-                              const Tile& t, uint32_t leaf, uint32_t path0, uint32_t path1, uint32_t top) {
-  if (leaf == kNone) return run_batch_op<W>(T, B, i, S, E, t);
-  const uint32_t ty = B.type[i], k = B.key[i];
-  uint32_t r        = 0;
-  bool write        = false;
-  if (ty == kOpFind) {
-    r = T.cooperative_find<W>(k, t, S, true, leaf);
-  } else if (ty == kOpRange) {
-    uint2* out = B.range_out ? B.range_out + B.out_off[i] : nullptr;
-    r          = T.cooperative_range_query<W>(k, B.arg[i], t, S, out, B.cap[i], true, leaf);
-  } else if (ty == kOpInsert) {
-    T.insert_at<W>(k, B.arg[i], t, E, leaf, path0, path1, top);
-    write = true;
-  } else if (ty == kOpErase) {
-    T.erase_at<W>(k, t, E, leaf);
-    write = true;
-  }
-  if (t.thread_rank() == 0) B.result[i] = r;
-  return write;
-}
-
 // Schedule of the persistent batched launch. Within each batch the claim order puts writes first
 // (perm maps a claim position to an op index). Writes of batch b may start once every write of
 // the batches before b has finished, reads of batch b likewise (they read the state after those
@@ -2561,10 +2644,10 @@ struct batch_sched {
                                               // free_avail, stat_reclaimed (memory over time)
 };
 
-constexpr uint32_t kWriteClaim   = 1;   // writes per tile per claim
-constexpr uint32_t kAdvancers    = 16;  // one waiting tile in 16 advances the batch chain each poll
-constexpr uint32_t kAdvanceEvery = 8;   // the others on every 8th poll
-constexpr uint32_t kReadClaim    = 4;   // reads per tile per claim
+constexpr uint32_t kWriteClaims  = 128; // claims a batch's writes are cut into at least, while lanes last
+constexpr uint32_t kReadClaims   = 4;   // claims of reads per warp of the launch likewise
+constexpr uint32_t kPollNs       = 400; // how often a block looks at done_batches while its warps wait
+constexpr uint32_t kAdvanceEvery = 64;  // a look in 64 also advances the batch chain
 
 // Largest b in [lo, nb) with pre[b] <= x (pre is non-decreasing), starting from the hint lo.
 MVBT_DEV uint32_t batch_of_ordinal(const uint64_t* pre, uint32_t nb, uint64_t x, uint32_t lo) {
@@ -2630,35 +2713,48 @@ MVBT_DEV void advance_full(const batch_sched& sc, uint32_t nb) {
   }
 }
 
+// What the warps of a block last saw of done_batches, and when one of them looked (ns, low 32 bits).
+struct batch_gate {
+  uint32_t done;
+  uint32_t looked;
+};
+
 // Waits (bounded) until the writes of every batch before b have finished; returns false on timeout.
-template <class Tile>
+// Thousands of warps can wait at once for one word on one L2 slice. So one warp of a block at a time
+// looks at it, every kPollNs, and the others read what it saw in shared memory: 592 blocks then
+// read the word about once a nanosecond, where a read per warp and half microsecond queued for longer
+// than the write phase that was waited for.
+template <class Warp>
 MVBT_DEV bool wait_batch_ready(const device_tree& T, const batch_sched& sc, uint32_t nb, uint32_t b,
-                               const Tile& t) {
+                               batch_gate& gate, const Warp& warp) {
   const unsigned long long t0 = global_ns();
-  // Thousands of tiles can wait here at once, and every poll reads the same few words (the batch
-  // counter and the finished batch's write count) on one L2 slice. One tile in kAdvancers tries
-  // to advance the chain on every poll, the others on every kAdvanceEvery-th and otherwise only
-  // read the counter, backing off longer, so the slice keeps up with the writers' own counting.
-  const bool advancer = tile_ordinal(t) % kAdvancers == 0;
   for (uint32_t w = 0;; ++w) {
     uint32_t d = 0;
-    if (t.thread_rank() == 0) {
-      if (advancer || w % kAdvanceEvery == kAdvanceEvery - 1) advance_done(sc, nb, T.ctl);
-      d = ld_relaxed_u32(sc.done_batches);
+    if (warp.thread_rank() == 0) {
+      d = ld_block_u32(&gate.done);
+      if (d < b) {
+        const uint32_t now = (uint32_t)global_ns(), last = ld_block_u32(&gate.looked);
+        if (now - last >= kPollNs && atomicCAS(&gate.looked, last, now) == last) {
+          if (w % kAdvanceEvery == kAdvanceEvery - 1) advance_done(sc, nb, T.ctl);
+          d = ld_relaxed_u32(sc.done_batches);
+          atomicMax(&gate.done, d);
+        }
+      }
     }
-    d = t.shfl(d, 0);
+    d = warp.shfl(d, 0);
     if (d >= b) {
       __threadfence();
-      t.sync();
+      warp.sync();
       return true;
     }
-    if (wait_expired(t0, T.ctl->wait_ns, t)) return false;
-    __nanosleep(advancer ? 128 : (w < 4 ? 256 : 2048));
+    if (wait_expired(t0, T.ctl->wait_ns, warp)) return false;
+    __nanosleep(kPollNs / 4);
   }
 }
 
-// One step of reclamation inside the launch (warp-collective): advances full_done, then frees up
-// to 32 copies below rc_limit. Returns true if it claimed any log position.
+// One step of reclamation inside the launch (warp-collective): advances full_done, then frees up to
+// kReclaimClaim copies below rc_limit; now and then (or with none to free) it returns this SM's chunk if the ring's tail
+// is about to come round to it. Returns true if it claimed any log position.
 template <class Warp>
 MVBT_DEV bool reclaim_step(const device_tree& T, const batch_sched& sc, uint32_t nb, const Warp& warp) {
   unsigned long long lim = 0;
@@ -2667,9 +2763,11 @@ MVBT_DEV bool reclaim_step(const device_tree& T, const batch_sched& sc, uint32_t
     lim = ld_relaxed_u64(sc.rc_limit);
   }
   lim = warp.shfl(lim, 0);
-  return T.reclaim_online(lim, warp) > 0;
+  const uint32_t n = T.reclaim_online(lim, warp);
+  if (n == 0 || (lim & 7u) == 0) flush_chunk(T.ctl, sm_id() % kMaxSmSlots, T.ctl->ring_cap - T.ctl->ring_cap / 8, warp);
+  return n > 0;
 }
-// At the end of a warp's work: one more reclamation step (at most 32 copies), then leave. The
+// At the end of a warp's work: one more reclamation step, then leave. The
 // copies the last batches made become reclaimable only when their last reads finish, at the very
 // end of the launch, when few warps are left; draining them there would stretch the launch, so
 // they wait for the next launch, whose warps free them from its start while work runs.
@@ -2679,25 +2777,70 @@ MVBT_DEV void reclaim_drain(const device_tree& T, const batch_sched& sc, uint32_
   reclaim_step(T, sc, nb, warp);
 }
 
-// Worker loop of one warp in the persistent batched launch. The warp claims consecutive claim
-// positions and hands them to its tiles interleaved (tile j takes every (32/W)-th position), and
-// the claim order inside a batch is writes | finds | ranges, so the tiles of a warp run the same
-// kind of op side by side and their instructions issue together.
+// Runs the ops of the lanes with `live` set (op index i, key, and its leaf as leaf_warp found it), all
+// of one batch or at least of one snapshot S: writes and finds by the warp, range queries by its
+// tiles. Results go to B.result.
 template <int W, class Warp, class Tile>
-MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const batch_sched& sc,
-                             const Warp& warp, const Tile& t) {
+MVBT_DEV void run_ops_warp(const device_tree& T, const batch_view& B, uint64_t i, uint32_t type, uint32_t key,
+                           bool live, uint32_t S, uint32_t leaf, write_stage& st, const Warp& warp, const Tile& tile) {
   constexpr uint32_t kTiles = 32 / W;
-  const uint32_t tid = warp.thread_rank() / W;
-  const uint32_t nb  = ld_relaxed_u32(sc.params + 0);
-  const uint32_t S0  = ld_relaxed_u32(sc.params + 1);
+  const uint32_t at  = leaf == kNone ? kAnchor : leaf;
+  const bool write   = live && is_write_op(type);
+  if (warp.ballot(write)) {
+    const uint32_t value = write && type == kOpInsert ? B.arg[i] : 0u;
+    write_warp<W>(T, key, value, type == kOpErase, write, S + 1, leaf, st, warp, tile);
+  }
+  const bool find = live && type == kOpFind;
+  uint32_t r      = 0;
+  if (warp.ballot(find)) {
+    const uint32_t v = find_warp_live(T, key, find, S, at, st, warp);
+    if (find) r = v;
+  }
+  const bool range = live && type == kOpRange;
+  if (live && !range) B.result[i] = r;
+  for (uint32_t left = warp.ballot(range); left;) {
+    uint32_t m = left;
+    for (uint32_t q = 0; q < warp.thread_rank() / W; ++q) m &= m - 1u;
+    const bool run     = m != 0;  // the same in every lane of a tile
+    const int src      = run ? __ffs(m) - 1 : 0;
+    const uint64_t op  = warp.shfl(i, src);
+    const uint32_t lo  = warp.shfl(key, src), from = warp.shfl(at, src);
+    if (run) {
+      uint2* out       = B.range_out ? B.range_out + B.out_off[op] : nullptr;
+      const uint32_t c = T.cooperative_range_query<W>(lo, B.arg[op], tile, S, out, B.cap[op], true, from);
+      if (tile.thread_rank() == 0) B.result[op] = c;
+    }
+    for (uint32_t q = 0; q < kTiles; ++q) left &= left - 1u;
+    warp.sync();
+  }
+}
+
+// Ops a warp claims at once: a full warp's worth, less when there would be fewer than `share` claims.
+MVBT_DEV uint32_t claim_size(uint64_t ops, uint64_t share, uint32_t least) {
+  const uint64_t c = ops / share;
+  return c >= 32 ? 32u : (c < least ? least : (uint32_t)c);
+}
+
+// Worker loop of one warp in the persistent batched launch. The warp claims consecutive claim
+// positions, one per lane; all its lanes descend together (leaf_warp), then the lanes of each batch,
+// in order, wait for it and run (run_ops_warp). warps: how many the launch has; gate: the block's.
+template <int W, class Warp, class Tile>
+MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const batch_sched& sc, uint32_t warps,
+                             batch_gate& gate, write_stage& st, const Warp& warp, const Tile& tile) {
+  constexpr uint32_t kTiles = 32 / W;
+  const uint32_t lane = warp.thread_rank();
+  const uint32_t nb   = ld_relaxed_u32(sc.params + 0);
+  const uint32_t S0   = ld_relaxed_u32(sc.params + 1);
   const uint64_t TW = sc.wpre[nb], TR = sc.rpre[nb];
+  const uint32_t wclaim = claim_size(TW, (uint64_t)nb * kWriteClaims, kTiles);
+  const uint32_t rclaim = claim_size(TR, (uint64_t)warps * kReadClaims, kTiles);
   uint32_t wb = 0, rb = 0;  // batch hints for the two queues
   unsigned long long idle_since = 0;
   for (uint32_t spin = 0;;) {
     warp.sync();
     uint32_t d = 0;
     unsigned long long g = 0, r = 0;
-    if (warp.thread_rank() == 0) {
+    if (lane == 0) {
       d = ld_relaxed_u32(sc.done_batches);
       g = ld_relaxed_u64(sc.wcursor);
       r = ld_relaxed_u64(sc.rcursor);
@@ -2712,78 +2855,65 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
     }
     __threadfence();  // the batches counted in d are finished: see their writes
     warp.sync();
-    bool did = false;
     // writes first: they gate every later batch. Work is taken up to one batch past the finished
-    // ones; an op of a batch that is not ready does its descent, then waits (run_batch_op_at).
+    // ones; the ops of a batch that is not ready do their descent, then wait.
+    bool writes = false, reads = false;
     if (g < TW) {
-      wb = batch_of_ordinal(sc.wpre, nb, g, wb);
-      if (wb <= d + 1) {
-        unsigned long long g0 = 0;
-        if (warp.thread_rank() == 0) g0 = atomicAdd(sc.wcursor, (unsigned long long)(kTiles * kWriteClaim));
-        g0 = warp.shfl(g0, 0);
-        did = g0 < TW;
-        uint32_t b = wb, dd = d;
-        for (uint32_t k = 0; k < kWriteClaim; ++k) {
-          const unsigned long long x = g0 + k * kTiles + tid;
-          if (x >= TW) break;
-          b = batch_of_ordinal(sc.wpre, nb, x, b);
-          const uint32_t i = sc.perm[sc.batch_off[b] + (x - sc.wpre[b])];
-          if (b > dd) {
-            uint32_t p0 = kNone, p1 = kNone, top = 0;
-            const uint32_t leaf = batch_op_descend<W>(T, B, i, p0, p1, top, t);
-            if (!wait_batch_ready(T, sc, nb, b, t) && t.thread_rank() == 0) T.set_error(kErrSpinLimit, 14);
-            dd = b;
-            run_batch_op_at<W>(T, B, i, S0 + b, S0 + b + 1, t, leaf, p0, p1, top);
-          } else {
-            run_batch_op<W>(T, B, i, S0 + b, S0 + b + 1, t);
-          }
-          // Counted without reading the sum back (a reduction the tile does not wait for): the
-          // tiles that wait for a batch (wait_batch_ready) and the warps with nothing runnable
-          // advance done_batches. No fence here: every write path ends with the fence of its
-          // last release or unlock, which orders its stores before this count.
-          t.sync();
-          if (t.thread_rank() == 0) atomicAdd(&sc.writes_done[b], 1u);
-        }
-        // the writes just made copies: free as many older ones as there are reclaimable, so
-        // that reclamation keeps pace with copying even when no warp is ever idle
-        if (did && sc.rc_limit) reclaim_step(T, sc, nb, warp);
-      }
+      wb     = batch_of_ordinal(sc.wpre, nb, g, wb);
+      writes = wb <= d + 1;
     }
-    if (!did && r < TR) {
-      rb = batch_of_ordinal(sc.rpre, nb, r, rb);
-      if (rb <= d + 1) {
-        unsigned long long r0 = 0;
-        if (warp.thread_rank() == 0) r0 = atomicAdd(sc.rcursor, (unsigned long long)(kTiles * kReadClaim));
-        r0 = warp.shfl(r0, 0);
-        did = r0 < TR;
-        uint32_t b = rb, dd = d;
-        uint32_t done_b[kReadClaim];  // batch of each read this tile ran (counted after a fence)
-#pragma unroll
-        for (uint32_t k = 0; k < kReadClaim; ++k) done_b[k] = 0xFFFFFFFFu;  // all set: the loop may stop early
-        for (uint32_t k = 0; k < kReadClaim; ++k) {
-          const unsigned long long x = r0 + k * kTiles + tid;
-          if (x >= TR) break;
-          b = batch_of_ordinal(sc.rpre, nb, x, b);
-          const uint32_t i = sc.perm[sc.batch_off[b] + sc.n_writes[b] + (x - sc.rpre[b])];
-          if (b > dd) {
-            uint32_t p0 = kNone, p1 = kNone, top = 0;
-            const uint32_t leaf = batch_op_descend<W>(T, B, i, p0, p1, top, t);
-            if (!wait_batch_ready(T, sc, nb, b, t) && t.thread_rank() == 0) T.set_error(kErrSpinLimit, 14);
-            dd = b;
-            run_batch_op_at<W>(T, B, i, S0 + b, S0 + b + 1, t, leaf, p0, p1, top);
-          } else {
-            run_batch_op<W>(T, B, i, S0 + b, S0 + b + 1, t);
-          }
-          done_b[k] = b;
-        }
-        if (sc.reads_done) {  // the reads' loads are complete before they are counted
-          __threadfence();
-          t.sync();
-          if (t.thread_rank() == 0)
-            for (uint32_t k = 0; k < kReadClaim; ++k)
-              if (done_b[k] < nb) atomicAdd(&sc.reads_done[done_b[k]], 1u);
-        }
+    if (!writes && r < TR) {
+      rb    = batch_of_ordinal(sc.rpre, nb, r, rb);
+      reads = rb <= d + 1;
+    }
+    bool did = false;
+    if (writes || reads) {
+      const uint32_t claim     = writes ? wclaim : rclaim;
+      const uint64_t total     = writes ? TW : TR;
+      const uint64_t* pre      = writes ? sc.wpre : sc.rpre;
+      unsigned long long first = 0;
+      if (lane == 0) first = atomicAdd(writes ? sc.wcursor : sc.rcursor, (unsigned long long)claim);
+      first = warp.shfl(first, 0);
+      did   = first < total;
+      const unsigned long long x = first + lane;
+      const bool has             = lane < claim && x < total;
+      uint32_t b = nb, type = kOpFind, key = kEmptyKey;
+      uint64_t i = 0;
+      if (has) {
+        b    = batch_of_ordinal(pre, nb, x, writes ? wb : rb);
+        i    = sc.perm[sc.batch_off[b] + (writes ? 0u : sc.n_writes[b]) + (x - pre[b])];
+        type = B.type[i];
+        key  = B.key[i];
       }
+      const uint32_t leaf = leaf_warp(T, key, has && key != kEmptyKey, kAnchor, nullptr, st, warp);
+      uint32_t ready      = d;
+      for (uint32_t left = warp.ballot(has); left;) {
+        const uint32_t now = warp.shfl(b, __ffs(left) - 1);  // the first batch left
+        const uint32_t cur = warp.ballot(has && b == now);
+        if (now > ready) {
+          if (!wait_batch_ready(T, sc, nb, now, gate, warp) && lane == 0) T.set_error(kErrSpinLimit, 14);
+          ready = now;
+        }
+        run_ops_warp<W>(T, B, i, type, key, has && b == now, S0 + now, leaf, st, warp, tile);
+        // The warp whose writes complete a batch advances done_batches. No fence before the count: every
+        // write path ends with the fence of its last release or unlock, which orders its stores before
+        // it. Reads: their loads are complete before they are counted.
+        if (!writes && sc.reads_done) __threadfence();
+        warp.sync();
+        if (lane == 0) {
+          const uint32_t n = (uint32_t)__popc(cur);
+          if (!writes) {
+            if (sc.reads_done) atomicAdd(&sc.reads_done[now], n);
+          } else if (atomicAdd(&sc.writes_done[now], n) + n >= sc.n_writes[now]) {
+            advance_done(sc, nb, T.ctl);
+          }
+        }
+        left &= ~cur;
+      }
+      // Reclamation keeps pace with copying even when no warp is ever idle: a step after each claim of
+      // reads, which nothing waits for, and after each claim of writes only where those outnumber the
+      // reads (the next batch waits for them).
+      if (did && sc.rc_limit && (reads || TW > TR)) reclaim_step(T, sc, nb, warp);
     }
     if (did) {
       spin       = 0;
@@ -2791,7 +2921,7 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
       continue;
     }
     // nothing runnable yet: help advance done_batches, reclaim, then back off (bounded)
-    if (warp.thread_rank() == 0) advance_done(sc, nb, T.ctl);
+    if (lane == 0) advance_done(sc, nb, T.ctl);
     if (sc.rc_limit && reclaim_step(T, sc, nb, warp)) {
       spin       = 0;
       idle_since = 0;
@@ -2799,7 +2929,7 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
     }
     if (idle_since == 0) idle_since = global_ns();
     if (wait_expired(idle_since, T.ctl->wait_ns, warp)) {
-      if (warp.thread_rank() == 0) T.set_error(kErrSpinLimit, 14);
+      if (lane == 0) T.set_error(kErrSpinLimit, 14);
       break;
     }
     __nanosleep(spin < 8 ? 256 : 2048);

@@ -6,15 +6,15 @@ was and every candidate starts from the same state. On the clone, the first samp
 untimed (it also loads the kernel variant), the remaining steps are timed with CUDA events around
 the persistent kernel; the candidate with the least kernel time wins and is set on the plan.
 
-Knobs: tile width 8 or 16 (the node is 16 pairs, so an 8-lane tile reads it with 16-byte lane
-loads and a 16-lane tile with 8-byte loads) and blocks per SM (0 = full occupancy of the
-unconstrained kernel, 4 / 6 / 8 = register-capped variants with more resident warps).
+Knobs: tile width 8 or 16 (of the writes that a warp hands to its tiles; the node is 16 pairs, so an
+8-lane tile reads it with 16-byte lane loads and a 16-lane tile with 8-byte loads) and blocks per SM
+(0 = full occupancy, 4 blocks; fewer leave fewer warps waiting for the batch chain).
 """
 from __future__ import annotations
 
 import numpy as np
 
-DEFAULT_CANDIDATES = ((8, 0), (8, 4), (8, 6), (16, 0), (16, 4), (16, 6))
+DEFAULT_CANDIDATES = ((8, 0), (8, 3), (8, 2), (16, 0), (16, 3), (16, 2))
 
 
 def _dev(torch, a):

@@ -201,8 +201,12 @@ __global__ void k_batch_begin(mvbt::control_block* ctl, uint32_t* params) {
 // Reclamation on: the copies made before this launch (epochs <= its first snapshot S0) are read
 // by no snapshot of the launch, so they are reclaimable from the start unless the caller still
 // reads a snapshot below S0 (watermark params[2] < S0).
-__global__ void k_batch_begin_reclaim(mvbt::control_block* ctl, const uint32_t* params,
-                                      unsigned long long* rc_limit) {
+__global__ void __launch_bounds__(256) k_batch_begin_reclaim(mvbt::control_block* ctl, const uint32_t* params,
+                                                             unsigned long long* rc_limit) {
+  // unread chunks half a lap behind go back to the ring; those that fall behind while the launch runs
+  // follow in its reclamation steps
+  auto warp = cg::tiled_partition<32>(cg::this_thread_block());
+  mvbt::flush_chunks(ctl, threadIdx.x >> 5, ctl->ring_cap / 2, warp);
   if (threadIdx.x == 0) {
     __threadfence();
     const uint32_t S0 = params[1], ext = params[2];
@@ -235,32 +239,45 @@ unsigned occupancy_grid(const launch_ctx& c, K kernel) {
   return (unsigned)g;
 }
 
-// MinBlocks > 0 caps registers so that many 256-thread blocks fit on an SM (more traversals in
-// flight, some spills); selected with mvbt_config::blocks_per_sm.
-template <int W, int MinBlocks>
-__global__ void __launch_bounds__(256, MinBlocks) k_batched(device_tree T, batch_view B, batch_sched sc) {
+#ifndef kBatchBlocks
+#define kBatchBlocks 4
+#endif
+constexpr int kWarpsPerBlock = 8;  // of 256 threads, the largest block
+
+template <int W>
+__global__ void __launch_bounds__(256, kBatchBlocks) k_batched(device_tree T, batch_view B, batch_sched sc) {
+  __shared__ mvbt::write_stage stage[kWarpsPerBlock];
   auto warp = cg::tiled_partition<32>(cg::this_thread_block());
   auto tile = cg::tiled_partition<W>(warp);
-  mvbt::batched_worker<W>(T, B, sc, warp, tile);
+  __shared__ mvbt::batch_gate gate;
+  if (threadIdx.x == 0) gate.done = 0, gate.looked = 0;
+  __syncthreads();
+  mvbt::batched_worker<W>(T, B, sc, gridDim.x * (blockDim.x >> 5), gate, stage[threadIdx.x >> 5], warp, tile);
 }
 
 template <int W>
 void launch_batched(const launch_ctx& c, const batch_view& B, const batch_sched& sc, cudaStream_t s) {
-  if (c.bps >= 8) k_batched<W, 8><<<occupancy_grid(c, k_batched<W, 8>), c.block, 0, s>>>(c.view, B, sc);
-  else if (c.bps >= 6) k_batched<W, 6><<<occupancy_grid(c, k_batched<W, 6>), c.block, 0, s>>>(c.view, B, sc);
-  else if (c.bps >= 4) k_batched<W, 4><<<occupancy_grid(c, k_batched<W, 4>), c.block, 0, s>>>(c.view, B, sc);
-  else k_batched<W, 3><<<occupancy_grid(c, k_batched<W, 3>), c.block, 0, s>>>(c.view, B, sc);
+  k_batched<W><<<occupancy_grid(c, k_batched<W>), c.block, 0, s>>>(c.view, B, sc);
 }
 
 // One batch [begin, end) in one launch: reads at the snapshot in snap_word, writes one epoch later.
 template <int W>
-__global__ void __launch_bounds__(256) k_mixed(device_tree T, batch_view B, uint64_t begin,
-                                               uint64_t end, const uint32_t* snap_word) {
-  auto tile        = cg::tiled_partition<W>(cg::this_thread_block());
-  const uint32_t S = mvbt::ld_relaxed_u32(snap_word);
-  const uint64_t tiles = ((uint64_t)gridDim.x * blockDim.x) / W;
-  for (uint64_t i = begin + ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / W; i < end; i += tiles)
-    mvbt::run_batch_op<W>(T, B, i, S, S + 1, tile);
+__global__ void __launch_bounds__(256, kBatchBlocks) k_mixed(device_tree T, batch_view B, uint64_t begin, uint64_t end,
+                                                             uint32_t lanes, const uint32_t* snap_word) {
+  __shared__ mvbt::write_stage stage[kWarpsPerBlock];
+  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
+  auto tile             = cg::tiled_partition<W>(warp);
+  mvbt::write_stage& st = stage[threadIdx.x >> 5];
+  const uint32_t S      = mvbt::ld_relaxed_u32(snap_word);
+  const uint32_t lane   = threadIdx.x & 31u;
+  const uint64_t stride = (((uint64_t)gridDim.x * blockDim.x) >> 5) * lanes;
+  for (uint64_t g = begin + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes; g < end; g += stride) {
+    const uint64_t i    = g + lane;
+    const bool has      = lane < lanes && i < end;
+    const uint32_t type = has ? B.type[i] : (uint32_t)mvbt::kOpFind, key = has ? B.key[i] : mvbt::kEmptyKey;
+    const uint32_t leaf = mvbt::leaf_warp(T, key, has && key != mvbt::kEmptyKey, mvbt::kAnchor, nullptr, st, warp);
+    mvbt::run_ops_warp<W>(T, B, i, type, key, has, S, leaf, st, warp, tile);
+  }
 }
 
 __global__ void k_snapshot_word(mvbt::control_block* ctl, uint32_t* out) {
@@ -300,7 +317,7 @@ int enqueue_persistent(mvbt_batch_plan* p, const launch_ctx& c, const batch_view
                                                      mb, p->d_perm);
   k_prefix<<<1, 1024, 0, s>>>(p->d_batch_off, p->d_params, nw, wpre, rpre);
   k_batch_begin<<<1, 32, 0, s>>>(c.ctl, p->d_params);
-  if (p->reclaim_on) k_batch_begin_reclaim<<<1, 32, 0, s>>>(c.ctl, p->d_params, rc_tail + mb);
+  if (p->reclaim_on) k_batch_begin_reclaim<<<1, 256, 0, s>>>(c.ctl, p->d_params, rc_tail + mb);
   batch_sched sc;
   sc.batch_off    = p->d_batch_off;
   sc.perm         = p->d_perm;
@@ -496,13 +513,14 @@ int mvbt_batch_run(mvbt_batch_plan* p, uint32_t num_batches, const uint64_t* bat
       const uint64_t lo = batch_off[b], hi = batch_off[b + 1];
       k_snapshot_word<<<1, 32, 0, s>>>(c.ctl, p->d_params + 1);
       if (hi == lo) continue;
-      uint64_t tiles = (hi - lo);
-      uint64_t need  = (tiles * c.W + c.block - 1) / c.block;
-      unsigned grid;
-      if (c.W == 8) grid = (unsigned)std::min<uint64_t>(need, occupancy_grid(c, k_mixed<8>));
-      else grid = (unsigned)std::min<uint64_t>(need, occupancy_grid(c, k_mixed<16>));
-      if (c.W == 8) k_mixed<8><<<grid, c.block, 0, s>>>(c.view, B, lo, hi, p->d_params + 1);
-      else k_mixed<16><<<grid, c.block, 0, s>>>(c.view, B, lo, hi, p->d_params + 1);
+      // ops per warp: fewer than 32 when that would leave SMs idle
+      const uint32_t lanes = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(4, (hi - lo) / (16ull * c.sms)));
+      const uint64_t warps = (uint64_t)c.block / 32;
+      const uint64_t need  = ((hi - lo) + lanes * warps - 1) / (lanes * warps);
+      if (c.W == 8)
+        k_mixed<8><<<(unsigned)std::min<uint64_t>(need, occupancy_grid(c, k_mixed<8>)), c.block, 0, s>>>(c.view, B, lo, hi, lanes, p->d_params + 1);
+      else
+        k_mixed<16><<<(unsigned)std::min<uint64_t>(need, occupancy_grid(c, k_mixed<16>)), c.block, 0, s>>>(c.view, B, lo, hi, lanes, p->d_params + 1);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(MVBT_ERR_CUDA, std::string("per-batch launch: ") + cudaGetErrorString(e));

@@ -88,6 +88,23 @@ __global__ void k_init(uint32_t* pool, control_block* c, uint32_t capacity, uint
                        (unsigned long long)free_ring, log_cap, ring_cap);
 }
 
+template <int W>
+__device__ __forceinline__ uint64_t first_tile() {
+  return ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / W;
+}
+template <int W>
+__device__ __forceinline__ uint64_t num_tiles() {
+  return ((uint64_t)gridDim.x * blockDim.x) / W;
+}
+
+// Before a reclaim pass (one block): the unread rests of the SMs' ring chunks that its pushes, with those
+// of the chunks themselves, could come round to go back to the ring.
+__global__ void __launch_bounds__(256) k_reclaim_flush(control_block* c) {
+  auto warp = cg::tiled_partition<32>(cg::this_thread_block());
+  const unsigned long long pushes = c->retire_tail - c->retire_head + (unsigned long long)mvbt::kMaxSmSlots * c->chunk;
+  mvbt::flush_chunks(c, threadIdx.x >> 5, pushes < c->ring_cap ? c->ring_cap - (uint32_t)pushes : 0u, warp);
+}
+
 // Reclaim pass over the retire log (mvbt_reclaim): frees every version copy made in an epoch <= M
 // (kReclaimAll: the current epoch) and appends it to the free ring (one reservation per warp).
 __global__ void __launch_bounds__(256) k_reclaim(device_tree T, uint32_t M) {
@@ -120,15 +137,6 @@ __global__ void k_snapshot(control_block* c, uint32_t* out) {
     uint32_t s = atomicAdd(&c->epoch, 1u);
     *out       = s;
   }
-}
-
-template <int W>
-__device__ __forceinline__ uint64_t first_tile() {
-  return ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / W;
-}
-template <int W>
-__device__ __forceinline__ uint64_t num_tiles() {
-  return ((uint64_t)gridDim.x * blockDim.x) / W;
 }
 
 // Loop condition of every tile loop below: true while any tile of the calling warp has work, so
@@ -166,8 +174,10 @@ __global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t
                                                    const uint32_t* __restrict__ spos, uint32_t* __restrict__ out,
                                                    uint32_t n, uint32_t ts) {
   __shared__ mvbt::warp_stage stage[kWarpsPerBlock];
+  __shared__ mvbt::warp_path paths[kSorted ? kWarpsPerBlock : 1];
   auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
   mvbt::warp_stage& st  = stage[threadIdx.x >> 5];
+  mvbt::warp_path* path = kSorted ? &paths[threadIdx.x >> 5] : nullptr;
   const uint32_t lane   = threadIdx.x & 31u;
   const uint64_t warps  = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint64_t w      = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -186,7 +196,7 @@ __global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t
     }
     return has;
   };
-  if (kSorted) mvbt::clear_path(st, warp);
+  if (kSorted) path->clear(warp);
   bool live = fetch(g);
   for (; g < end; g += stride) {
     const uint32_t k = key, p = pos;
@@ -195,10 +205,10 @@ __global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t
     uint32_t start   = mvbt::kAnchor;
     if (kSorted) {  // the keys are in order down to the bits that the sort left out
       const uint32_t m = __ballot_sync(0xffffffffu, here);
-      start = mvbt::path_start(st, __shfl_sync(0xffffffffu, k, 0) & ~kUnsortedBits,
+      start = path->start(__shfl_sync(0xffffffffu, k, 0) & ~kUnsortedBits,
                                __shfl_sync(0xffffffffu, k, 31 - __clz(m)) | kUnsortedBits, warp);
     }
-    const uint32_t v = mvbt::find_warp(T, k, here, ts, start, kSorted, st, warp);
+    const uint32_t v = mvbt::find_warp(T, k, here, ts, start, path, st, warp);
     if (here) out[p] = v;
   }
 }
@@ -362,9 +372,11 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
                                                        const uint32_t* __restrict__ spos,
                                                        const uint32_t* __restrict__ values, uint32_t n) {
   __shared__ mvbt::write_stage stage[kWarpsPerBlock];
+  __shared__ mvbt::warp_path paths[kSorted ? kWarpsPerBlock : 1];
   auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
   auto tile             = cg::tiled_partition<kSlowTile>(cg::this_thread_block());
   mvbt::write_stage& st = stage[threadIdx.x >> 5];
+  mvbt::warp_path* path = kSorted ? &paths[threadIdx.x >> 5] : nullptr;
   const uint32_t lane   = threadIdx.x & 31u;
   const uint32_t E      = T.versioned ? T.current_epoch() : 0u;
   const uint64_t warps  = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -373,7 +385,7 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
   const uint64_t per    = (groups + warps - 1) / warps;
   uint64_t g            = kSorted ? w * per : w;
   const uint64_t end    = kSorted ? (g + per < groups ? g + per : groups) : groups;
-  if (kSorted) mvbt::clear_path(st, warp);
+  if (kSorted) path->clear(warp);
   for (; g < end; g += kSorted ? 1 : warps) {
     const uint64_t i = g * 32 + lane;
     const bool has   = i < n;
@@ -384,9 +396,10 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
     uint32_t start = mvbt::kAnchor;
     if (kSorted) {
       const uint32_t m = __ballot_sync(0xffffffffu, has);
-      start = mvbt::path_start(st, __shfl_sync(0xffffffffu, k, 0), __shfl_sync(0xffffffffu, k, 31 - __clz(m)), warp);
+      start = path->start(__shfl_sync(0xffffffffu, k, 0), __shfl_sync(0xffffffffu, k, 31 - __clz(m)), warp);
     }
-    mvbt::write_warp<kSlowTile>(T, k, v, kErase, live, E, start, kSorted, st, warp, tile);
+    const uint32_t leaf = mvbt::leaf_warp(T, k, live && k != mvbt::kEmptyKey, start, path, st, warp);
+    mvbt::write_warp<kSlowTile>(T, k, v, kErase, live, E, leaf, st, warp, tile);
   }
 }
 
@@ -1385,6 +1398,7 @@ int mvbt_reclaim(mvbt_tree* t, uint32_t min_live_snapshot, void* stream) {
     return fail(MVBT_ERR_NOT_SUPPORTED, "reclamation is off: create the tree with mvbt_config.reclaim = 1");
   MVBT_CUDA_TRY(cudaSetDevice(t->device));
   cudaStream_t s = as_stream(stream);
+  k_reclaim_flush<<<1, 256, 0, s>>>(t->ctl);
   k_reclaim<<<(unsigned)t->num_sms * 4u, 256, 0, s>>>(t->view(), min_live_snapshot);
   int st = check_launch();
   if (st) return st;

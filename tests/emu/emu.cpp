@@ -4,7 +4,11 @@
 // as W host threads: shfl / ballot / sync go through a per-tile exchange buffer and a barrier,
 // atomics are GCC atomics on the shared pool. Several tiles run at once, so the lock, split and
 // versioning protocols are exercised concurrently on the CPU before any GPU run.
+#undef _FORTIFY_SOURCE  // its longjmp takes a jump to another stack for an error
 #define MVBT_HOST_EMULATION 1
+#include <setjmp.h>
+#include <ucontext.h>
+
 #include <barrier>
 #include <cstdint>
 #include <cstring>
@@ -18,10 +22,72 @@
 
 namespace {
 
+// The lanes of an emulated warp (run_warps) are contexts of one host thread that switch where they
+// wait, which costs a fraction of 32 host threads meeting in a barrier.
+struct fibers {
+  ucontext_t ctx[32];      // how a lane starts; it goes on by longjmp, which needs no system call
+  jmp_buf home, at[32];
+  bool started[32], done[32];
+  std::vector<char> stack[32];
+  std::function<void(int)> body;
+  int lane = 0;
+  void yield() {
+    if (_setjmp(at[lane]) == 0) _longjmp(home, 1);
+  }
+  void enter(int l) {
+    lane = l;
+    if (_setjmp(home) != 0) return;
+    if (started[l]) _longjmp(at[l], 1);
+    started[l] = true;
+    setcontext(&ctx[l]);
+  }
+  static void entry(unsigned lo, unsigned hi) {
+    auto* f = reinterpret_cast<fibers*>((uintptr_t)lo | ((uintptr_t)hi << 32));
+    f->body(f->lane);
+    f->done[f->lane] = true;
+    f->yield();
+  }
+  void run(std::function<void(int)> fn) {
+    body = std::move(fn);
+    const uintptr_t self = reinterpret_cast<uintptr_t>(this);
+    for (int l = 0; l < 32; ++l) {
+      started[l] = done[l] = false;
+      stack[l].resize(256 << 10);
+      getcontext(&ctx[l]);
+      ctx[l].uc_stack.ss_sp   = stack[l].data();
+      ctx[l].uc_stack.ss_size = stack[l].size();
+      ctx[l].uc_link          = nullptr;  // a finished lane yields for good
+      makecontext(&ctx[l], reinterpret_cast<void (*)()>(&entry), 2, (unsigned)self, (unsigned)(self >> 32));
+    }
+    for (volatile int left = 32; left > 0;)
+      for (volatile int l = 0; l < 32; ++l)
+        if (!done[l]) {
+          enter(l);
+          if (done[l]) left = left - 1;
+        }
+  }
+};
+
 struct tile_shared {
   std::barrier<> bar;
   uint64_t slot[32];
-  explicit tile_shared(int w) : bar(w) {}
+  fibers* fib = nullptr;  // the lanes are contexts of one thread
+  int width, arrived = 0;
+  unsigned generation = 0;
+  explicit tile_shared(int w) : bar(w), width(w) {}
+  void sync() {
+    if (!fib) {
+      bar.arrive_and_wait();
+      return;
+    }
+    const unsigned mine = generation;
+    if (++arrived == width) {
+      arrived = 0;
+      ++generation;
+      return;
+    }
+    while (generation == mine) fib->yield();
+  }
 };
 
 // Emulated cooperative-groups tile of W lanes.
@@ -30,7 +96,7 @@ struct emu_tile {
   int W;
   tile_shared* sh;
   int thread_rank() const { return rank; }
-  void sync() const { sh->bar.arrive_and_wait(); }
+  void sync() const { sh->sync(); }
   template <class T>
   T shfl(T v, int src) const {
     sh->slot[rank] = (uint64_t)v;
@@ -97,14 +163,17 @@ void run_warps(int warps, int W, const std::function<void(const emu_tile&, const
   }
   std::vector<std::thread> th;
   for (int w = 0; w < warps; ++w) {
-    for (int l = 0; l < 32; ++l) {
-      th.emplace_back([&, w, l] {
-        mvbt::emu::sm = (uint32_t)w;
+    th.emplace_back([&, w] {
+      mvbt::emu::sm = (uint32_t)w;
+      auto f        = std::make_unique<fibers>();
+      wsh[w]->fib   = f.get();
+      for (int j = 0; j < tpw; ++j) tsh[w * tpw + j]->fib = f.get();
+      f->run([&](int l) {
         emu_tile warp{l, 32, wsh[w].get()};
         emu_tile tile{l % W, W, tsh[w * tpw + l / W].get()};
         fn(warp, tile);
       });
-    }
+    });
   }
   for (auto& x : th) x.join();
 }
@@ -233,11 +302,12 @@ void emu_find_warp(void* h, const uint32_t* keys, const uint32_t* pos, uint32_t*
   if (!v.versioned) ts = mvbt::kLatest;
   const uint64_t groups = (n + lanes - 1) / lanes, per = (groups + warps - 1) / warps;
   std::vector<mvbt::warp_stage> stage(warps);
+  std::vector<mvbt::warp_path> path(warps);
   run_warps(warps, 8, [&](const emu_tile& warp, const emu_tile&) {
     const uint64_t w = mvbt::emu::sm;
     uint64_t g       = sorted ? w * per : w;
     const uint64_t end = sorted ? std::min(g + per, groups) : groups;
-    if (sorted) mvbt::clear_path(stage[w], warp);
+    if (sorted) path[w].clear(warp);
     for (; g < end; g += sorted ? 1 : warps) {
       const uint64_t i = g * lanes + warp.thread_rank();
       const bool live  = (uint32_t)warp.thread_rank() < lanes && i < n;
@@ -245,9 +315,9 @@ void emu_find_warp(void* h, const uint32_t* keys, const uint32_t* pos, uint32_t*
       uint32_t start = mvbt::kAnchor;
       if (sorted) {
         const uint32_t m = warp.ballot(live);
-        start = mvbt::path_start(stage[w], warp.shfl(k, 0) & ~low_bits, warp.shfl(k, 31 - __clz(m)) | low_bits, warp);
+        start = path[w].start(warp.shfl(k, 0) & ~low_bits, warp.shfl(k, 31 - __clz(m)) | low_bits, warp);
       }
-      const uint32_t r = mvbt::find_warp(v, k, live, ts, start, sorted != 0, stage[w], warp);
+      const uint32_t r = mvbt::find_warp(v, k, live, ts, start, sorted ? &path[w] : nullptr, stage[w], warp);
       if (live) out[sorted ? pos[i] : i] = r;
     }
   });
@@ -263,12 +333,13 @@ void emu_write_warp(void* h, const uint32_t* kind, const uint32_t* keys, const u
   const uint32_t E      = v.versioned ? v.current_epoch() : 0u;
   const uint64_t groups = (n + 31) / 32, per = (groups + warps - 1) / warps;
   std::vector<mvbt::write_stage> stage(warps);
+  std::vector<mvbt::warp_path> path(warps);
   EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {
     const uint64_t w = mvbt::emu::sm;
     auto& st         = stage[w];
     uint64_t g       = sorted ? w * per : w;
     const uint64_t end = sorted ? std::min(g + per, groups) : groups;
-    if (sorted) mvbt::clear_path(st, warp);
+    if (sorted) path[w].clear(warp);
     for (; g < end; g += sorted ? 1 : warps) {
       const uint64_t i = g * 32 + warp.thread_rank();
       const bool has   = i < n;
@@ -277,9 +348,10 @@ void emu_write_warp(void* h, const uint32_t* kind, const uint32_t* keys, const u
       uint32_t start   = mvbt::kAnchor;
       if (sorted) {
         const uint32_t m = warp.ballot(has);
-        start = mvbt::path_start(st, warp.shfl(k, 0), warp.shfl(k, 31 - __clz(m)), warp);
+        start = path[w].start(warp.shfl(k, 0), warp.shfl(k, 31 - __clz(m)), warp);
       }
-      mvbt::write_warp<kW>(v, k, has ? vals[i] : 0u, has && kind[i] == 2, live, E, start, sorted != 0, st, warp, tile);
+      const uint32_t leaf = mvbt::leaf_warp(v, k, live && k != mvbt::kEmptyKey, start, sorted ? &path[w] : nullptr, st, warp);
+      mvbt::write_warp<kW>(v, k, has ? vals[i] : 0u, has && kind[i] == 2, live, E, leaf, st, warp, tile);
     }
   }));
 }
@@ -452,8 +524,11 @@ void emu_batch_run(void* h, uint32_t nb, const uint64_t* off, const uint32_t* ty
     sc.rc_limit   = &rc_limit;
     sc.series     = ser.data();
   }
-  EMU_DISPATCH(W, run_warps(std::max(1, tiles * kW / 32), kW, [&](const emu_tile& warp, const emu_tile& tile) {
-    mvbt::batched_worker<kW>(v, B, sc, warp, tile);
+  const int warps = std::max(1, tiles * W / 32);
+  std::vector<mvbt::write_stage> stage(warps);
+  mvbt::batch_gate gate{0, 0};  // the warps as one block
+  EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {
+    mvbt::batched_worker<kW>(v, B, sc, (uint32_t)warps, gate, stage[mvbt::emu::sm], warp, tile);
   }));
   t->ctl.epoch = params[1] + nb;
   if (series && sc.series) std::memcpy(series, ser.data(), ser.size() * sizeof(uint64_t));
