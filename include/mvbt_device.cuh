@@ -2226,6 +2226,125 @@ MVBT_DEV uint32_t find_warp_live(const device_tree& T, uint32_t key, bool live, 
   return found;
 }
 
+// Range queries [lo, hi) of the live lanes at snapshot ts: cooperative_range_query's route, pairs and
+// full count (kLive: while writers run, at snapshots; otherwise range_quiescent's). Each lane writes
+// at most cap pairs at out (nullable). The lanes walk their leaves in step: the warp stages one leaf
+// per lane, each lane finds its pairs there, and eight lanes per query write them. start, path: as in
+// find_warp.
+template <bool kLive, class Warp>
+MVBT_DEV uint32_t range_warp(const device_tree& T, uint32_t lo, uint32_t hi, bool live, uint32_t ts, uint2* out,
+                             uint32_t cap, uint32_t start, warp_path* path, warp_stage& st, const Warp& warp) {
+  const bool snap     = T.versioned && ts != kLatest;
+  const uint32_t lane = warp.thread_rank();
+  live                = live && hi > lo;
+  uint32_t idx = start, count = 0, hops = 0, leaves = 0;
+  bool copy = false, scan = false;  // idx is an older version; idx is the next leaf to the right
+  const uint32_t all = warp.ballot(live);
+  const bool last    = path && live && (all >> lane) == 1u;
+  for (;;) {
+    if (live && idx >= T.capacity) {
+      T.set_error(kErrCorrupt, 1);
+      live = false;
+    }
+    if (live && ++hops > kMaxSteps) {
+      T.set_error(kErrStepLimit, scan ? 7 : 5);
+      live = false;
+    }
+    const uint32_t m = warp.ballot(live);
+    if (m == 0) return count;
+    const uint32_t slot = stage_nodes<kLive>(T, idx, live, m, st, warp);
+    bool use            = false;  // the staged node is the lane's next leaf at ts
+    uint32_t high = 0, link = kNone;
+    if (live) {
+      const uint32_t low = st.word(slot, 26);
+      uint32_t nts, ol;
+      ld_shared_4(st.last_words(slot), high, link, nts, ol);
+      link &= kIndexMask;
+      if (snap && nts > ts) {
+        idx  = ol & kIndexMask;
+        copy = true;
+        if (idx == kNone) {
+          T.set_error(kErrCorrupt, 3);
+          live = false;
+        }
+      } else if (scan) {
+        use = true;
+      } else if (lo < low) {
+        idx  = kAnchor;
+        copy = false;
+      } else if (lo >= high && link != kNone) {
+        idx  = link;
+        copy = false;
+      } else {
+        const uint32_t level = ol >> 28;
+        if (last) path->record(level, idx, low, high);
+        use = level == 0;
+        if (!use) {
+          const uint32_t c = count_up_to(st, slot, lo);
+          idx              = c ? st.word(slot, 2 * c - 1) : kAnchor;
+          copy             = false;
+        }
+      }
+    }
+    if (kLive) {
+      const bool check = use && !copy;
+      if (warp.ballot(check)) {  // as recheck_version
+        __threadfence();
+        warp.sync();
+        if (check) {
+          const uint32_t* node = T.node_ptr(idx);
+          const uint32_t mod0 = st.word(slot, kModWord), mod1 = ld_relaxed_u32(node + kModWord);
+          const unsigned long long v = ld_relaxed_u64(reinterpret_cast<const unsigned long long*>(node + 30));
+          if ((uint32_t)v > ts) {  // changed meanwhile: its immutable copy instead
+            idx  = (uint32_t)(v >> 32) & kIndexMask;
+            copy = true;
+            use  = false;
+          } else if ((mod0 & kLockBit) || mod1 != mod0) {
+            use = false;  // a writer is changing it: read it again
+            __nanosleep(64);
+          }
+        }
+      }
+    }
+    const uint32_t uses = warp.ballot(use);
+    uint32_t first = 0, pairs = 0, room = 0;
+    if (use) {
+      first = lo ? count_up_to(st, slot, lo - 1u) : 0u;
+      pairs = count_up_to(st, slot, hi - 1u) - first;
+      room  = out == nullptr || count >= cap ? 0u : (pairs < cap - count ? pairs : cap - count);
+    }
+    const uint32_t info = use ? slot | (first << 8) | (room << 16) : 0u;
+    const unsigned long long to = (unsigned long long)(out + count);
+    for (uint32_t q = 0; q < 32; q += 4) {  // four queries at a time
+      if (((uses >> q) & 15u) == 0) continue;
+      const int src             = (int)(q + (lane >> 3));
+      const uint32_t what       = warp.shfl(info, src);
+      const unsigned long long at = warp.shfl(to, src);
+      const uint32_t s = what & 255u, a = (what >> 8) & 255u;
+      for (uint32_t j = lane & 7u; j < what >> 16; j += 8) {
+        const uint32_t* w = &st.node[s][((((a + j) >> 1) ^ (s & 7u)) << 2) | (((a + j) & 1u) << 1)];
+        reinterpret_cast<uint2*>(at)[j] = make_uint2(w[0], w[1]);
+      }
+    }
+    if (use) {
+      count += pairs;
+      hops = 0;
+      if (hi > high && link != kNone) {
+        idx  = link;
+        scan = true;
+        copy = false;
+        if (++leaves > T.capacity) {  // a sibling chain is never longer than the pool
+          T.set_error(kErrStepLimit, 6);
+          live = false;
+        }
+      } else {
+        live = false;
+      }
+    }
+    warp.sync();
+  }
+}
+
 // ----------------------------------------------------------------------------------------------
 // Writes of a whole warp
 // ----------------------------------------------------------------------------------------------
@@ -2395,6 +2514,19 @@ MVBT_DEV bool apply_staged(warp_stage& st, uint32_t s, uint32_t& n, uint32_t key
   at(2 * c) = key, at(2 * c + 1) = value;
   ++n;
   return true;
+}
+
+// Calls f(src) by each tile for the lanes of m, a tile's share at a time: src is the lane (the same in
+// every lane of the tile) and run says whether the tile has one. f runs with the tile converged.
+template <int W, class Warp, class F>
+MVBT_DEV void for_lanes(uint32_t m, const Warp& warp, const F& f) {
+  for (uint32_t left = m; left;) {
+    uint32_t own = left;
+    for (uint32_t q = 0; q < warp.thread_rank() / (uint32_t)W; ++q) own &= own - 1u;
+    f(own != 0, own ? __ffs(own) - 1 : 0);
+    for (uint32_t q = 0; q < 32u / W; ++q) left &= left - 1u;
+    warp.sync();
+  }
 }
 
 // One write by a tile, from the leaf where its warp found it.
@@ -2855,7 +2987,9 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
     }
     __threadfence();  // the batches counted in d are finished: see their writes
     warp.sync();
-    // writes first: they gate every later batch. Work is taken up to one batch past the finished
+    // A claim may run past the batch after the finished ones and then waits for writes that other warps
+    // claim; a launch of one or two warps therefore reads only once every write is claimed.
+    // Writes first: they gate every later batch. Work is taken up to one batch past the finished
     // ones; the ops of a batch that is not ready do their descent, then wait.
     bool writes = false, reads = false;
     if (g < TW) {
@@ -2864,7 +2998,7 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
     }
     if (!writes && r < TR) {
       rb    = batch_of_ordinal(sc.rpre, nb, r, rb);
-      reads = rb <= d + 1;
+      reads = rb <= d + 1 && (warps > 2 || g >= TW);
     }
     bool did = false;
     if (writes || reads) {

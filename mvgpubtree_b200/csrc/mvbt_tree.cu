@@ -159,6 +159,10 @@ __global__ void __launch_bounds__(256) k_find(device_tree T, const uint32_t* __r
   }
 }
 
+constexpr int kWarpsPerBlock = 8;  // of 256 threads, the largest block
+constexpr int kSlowTile      = 8;  // tile of a warp's rare writes one by one (mvbt::write_tile)
+__device__ __forceinline__ auto slow_tile() { return cg::tiled_partition<kSlowTile>(cg::this_thread_block()); }
+
 // Lookups in a tree no writer changes meanwhile, 32 keys per warp at a time (mvbt::find_warp).
 // kSorted: the keys are a sorted call's, each warp takes one contiguous run of them and starts at
 // the deepest node of the last keys' path that covers the next ones, and the results go back to the
@@ -167,8 +171,6 @@ __global__ void __launch_bounds__(256) k_find(device_tree T, const uint32_t* __r
 // blocks per SM.
 constexpr int kReadSortLowBit   = 8;  // reads: order by the top 24 bits (locality is all they need)
 constexpr uint32_t kUnsortedBits = (1u << kReadSortLowBit) - 1u;
-constexpr int kWarpsPerBlock    = 8;
-constexpr int kSlowTile         = 8;  // tile of a warp's rare writes one by one (write_tile)
 template <bool kSorted>
 __global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t* __restrict__ keys,
                                                    const uint32_t* __restrict__ spos, uint32_t* __restrict__ out,
@@ -213,6 +215,43 @@ __global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t
   }
 }
 
+// Range queries in a tree no writer changes meanwhile, 32 per warp at a time (mvbt::range_warp);
+// kSorted as in k_find_warp, by lower bound.
+template <bool kSorted>
+__global__ void __launch_bounds__(256) k_range_warp(device_tree T, const uint32_t* __restrict__ lower,
+                                                    const uint32_t* __restrict__ spos,
+                                                    const uint32_t* __restrict__ upper, uint2* result,
+                                                    uint32_t* counts, uint32_t avg_len, uint32_t n, uint32_t ts) {
+  __shared__ mvbt::warp_stage stage[kWarpsPerBlock];
+  __shared__ mvbt::warp_path paths[kSorted ? kWarpsPerBlock : 1];
+  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
+  mvbt::warp_stage& st  = stage[threadIdx.x >> 5];
+  mvbt::warp_path* path = kSorted ? &paths[threadIdx.x >> 5] : nullptr;
+  const uint32_t lane   = threadIdx.x & 31u;
+  const uint64_t warps  = num_tiles<32>(), w = first_tile<32>();
+  const uint64_t groups = ((uint64_t)n + 31) / 32;
+  const uint64_t per    = (groups + warps - 1) / warps;
+  uint64_t g            = kSorted ? w * per : w;
+  const uint64_t end    = kSorted ? (g + per < groups ? g + per : groups) : groups;
+  if (kSorted) path->clear(warp);
+  for (; g < end; g += kSorted ? 1 : warps) {
+    const uint64_t i  = g * 32 + lane;
+    const bool has    = i < n;
+    const uint32_t lo = has ? lower[i] : 0u;
+    const uint64_t p  = !has ? 0u : (kSorted ? spos[i] : i);
+    const uint32_t hi = has ? upper[p] : 0u;
+    uint32_t start    = mvbt::kAnchor;
+    if (kSorted) {  // the keys are in order down to the bits that the sort left out
+      const uint32_t m = __ballot_sync(0xffffffffu, has);
+      start = path->start(__shfl_sync(0xffffffffu, lo, 0) & ~kUnsortedBits,
+                          __shfl_sync(0xffffffffu, lo, 31 - __clz(m)) | kUnsortedBits, warp);
+    }
+    uint2* out       = result ? result + p * (uint64_t)avg_len : nullptr;
+    const uint32_t c = mvbt::range_warp<false>(T, lo, hi, has, ts, out, avg_len, start, path, st, warp);
+    if (counts && has) counts[p] = c;
+  }
+}
+
 template <int W>
 __global__ void __launch_bounds__(256) k_insert(device_tree T, const uint32_t* __restrict__ keys,
                                                 const uint32_t* __restrict__ values, uint32_t n) {
@@ -253,58 +292,100 @@ __global__ void __launch_bounds__(256) k_range(device_tree T, const uint32_t* __
   }
 }
 
-// Op i of the mixed kernels: inserts are spread evenly over the op index space
-// (Bresenham split), so inserts and queries run side by side in every wave.
-__device__ __forceinline__ bool split_op(uint64_t i, uint64_t n_a, uint64_t total, uint64_t& a_idx,
-                                         uint64_t& b_idx) {
-  uint64_t a = (i * n_a) / total, b = ((i + 1) * n_a) / total;
-  a_idx      = a;
-  b_idx      = i - a;
+// The mixed kernels hand out units of up to 32 ops, one unit per warp at a time: unit u of the
+// `writes + reads` units is a write unit or a read unit (Bresenham split), so both kinds run side
+// by side in every wave. Returns whether it is a write unit, and its number among its kind.
+__device__ __forceinline__ bool split_unit(uint64_t u, uint64_t writes, uint64_t reads, uint64_t& number) {
+  const uint64_t total = writes + reads;
+  const uint64_t a = (u * writes) / total, b = ((u + 1) * writes) / total;
+  number           = b > a ? a : u - a;
   return b > a;
 }
 
+// Writes run by the warp (mvbt::write_warp); range queries at the launch snapshot by the warp
+// (mvbt::range_warp), those of a plain tree's newest state a tile per query from their leaves.
 template <int W>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
     k_insert_range(device_tree T, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ values,
                    uint32_t n_ins, const uint32_t* __restrict__ lower, const uint32_t* __restrict__ upper,
-                   uint32_t n_rq, uint2* result, uint32_t avg_len, uint32_t* counts,
+                   uint32_t n_rq, uint2* result, uint32_t avg_len, uint32_t* counts, uint32_t lanes,
                    const uint32_t* snap_word) {
-  auto tile            = cg::tiled_partition<W>(cg::this_thread_block());
-  const bool ver       = T.versioned != 0;
-  const uint32_t S     = ver ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
-  const uint32_t E     = ver ? S + 1 : 0u;
-  const uint64_t total = (uint64_t)n_ins + n_rq;
-  for (uint64_t i = first_tile<W>(); warp_any(i < total); i += num_tiles<W>()) {
-    if (i >= total) continue;
-    uint64_t a, r;
-    if (split_op(i, n_ins, total, a, r)) {
-      T.cooperative_insert<W>(keys[a], values[a], tile, E);
+  __shared__ mvbt::write_stage stage[kWarpsPerBlock];
+  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
+  auto tile             = cg::tiled_partition<W>(warp);
+  mvbt::write_stage& st = stage[threadIdx.x >> 5];
+  const uint32_t lane   = threadIdx.x & 31u;
+  const bool ver        = T.versioned != 0;
+  const uint32_t S      = ver ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
+  const uint32_t E      = ver ? S + 1 : 0u;
+  const uint64_t writes = ((uint64_t)n_ins + lanes - 1) / lanes, reads = ((uint64_t)n_rq + lanes - 1) / lanes;
+  for (uint64_t u = first_tile<32>(); u < writes + reads; u += num_tiles<32>()) {
+    uint64_t number;
+    const bool write   = split_unit(u, writes, reads, number);
+    const uint64_t i   = number * lanes + lane;
+    const bool has     = lane < lanes && i < (write ? n_ins : n_rq);
+    const uint32_t key = has ? (write ? keys[i] : lower[i]) : mvbt::kEmptyKey;
+    const uint32_t leaf = mvbt::leaf_warp(T, key, has && key != mvbt::kEmptyKey, mvbt::kAnchor, nullptr, st, warp);
+    if (write) {
+      mvbt::write_warp<kSlowTile>(T, key, has ? values[i] : 0u, false, has, E, leaf, st, warp, slow_tile());
     } else {
-      uint2* out = result ? result + r * (uint64_t)avg_len : nullptr;
-      uint32_t c = T.cooperative_range_query<W>(lower[r], upper[r], tile, S, out, avg_len, true);
-      if (counts && tile.thread_rank() == 0) counts[r] = c;
+      const uint32_t at = leaf == mvbt::kNone ? mvbt::kAnchor : leaf;
+      if (ver) {
+        uint2* out       = result ? result + i * (uint64_t)avg_len : nullptr;
+        const uint32_t c = mvbt::range_warp<true>(T, key, has ? upper[i] : 0u, has, S, out, avg_len, at, nullptr, st, warp);
+        if (counts && has) counts[i] = c;
+        continue;
+      }
+      mvbt::for_lanes<W>(warp.ballot(has), warp, [&](bool run, int src) {
+        const uint32_t lo = warp.shfl(key, src), from = warp.shfl(at, src);
+        if (run) {
+          const uint64_t r = number * lanes + src;
+          uint2* out       = result ? result + r * (uint64_t)avg_len : nullptr;
+          const uint32_t c = T.cooperative_range_query<W>(lo, upper[r], tile, S, out, avg_len, true, from);
+          if (counts && tile.thread_rank() == 0) counts[r] = c;
+        }
+      });
     }
   }
 }
 
+// Erases run by the warp; finds at the launch snapshot by the warp (mvbt::find_warp_live), finds of a
+// plain tree's newest state a tile per key from their leaves.
 template <int W>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
     k_find_erase(device_tree T, const uint32_t* __restrict__ fkeys, uint32_t* __restrict__ fres,
-                 uint32_t n_find, const uint32_t* __restrict__ ekeys, uint32_t n_erase,
+                 uint32_t n_find, const uint32_t* __restrict__ ekeys, uint32_t n_erase, uint32_t lanes,
                  const uint32_t* snap_word) {
-  auto tile            = cg::tiled_partition<W>(cg::this_thread_block());
-  const bool ver       = T.versioned != 0;
-  const uint32_t S     = ver ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
-  const uint32_t E     = ver ? S + 1 : 0u;
-  const uint64_t total = (uint64_t)n_find + n_erase;
-  for (uint64_t i = first_tile<W>(); warp_any(i < total); i += num_tiles<W>()) {
-    if (i >= total) continue;
-    uint64_t e, f;
-    if (split_op(i, n_erase, total, e, f)) {
-      T.cooperative_erase<W>(ekeys[e], tile, E);
+  __shared__ mvbt::write_stage stage[kWarpsPerBlock];
+  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
+  auto tile             = cg::tiled_partition<W>(warp);
+  mvbt::write_stage& st = stage[threadIdx.x >> 5];
+  const uint32_t lane   = threadIdx.x & 31u;
+  const bool ver        = T.versioned != 0;
+  const uint32_t S      = ver ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
+  const uint32_t E      = ver ? S + 1 : 0u;
+  const uint64_t writes = ((uint64_t)n_erase + lanes - 1) / lanes, reads = ((uint64_t)n_find + lanes - 1) / lanes;
+  for (uint64_t u = first_tile<32>(); u < writes + reads; u += num_tiles<32>()) {
+    uint64_t number;
+    const bool write   = split_unit(u, writes, reads, number);
+    const uint64_t i   = number * lanes + lane;
+    const bool has     = lane < lanes && i < (write ? n_erase : n_find);
+    const uint32_t key = has ? (write ? ekeys[i] : fkeys[i]) : mvbt::kEmptyKey;
+    const uint32_t leaf = mvbt::leaf_warp(T, key, has && key != mvbt::kEmptyKey, mvbt::kAnchor, nullptr, st, warp);
+    const uint32_t at   = leaf == mvbt::kNone ? mvbt::kAnchor : leaf;
+    if (write) {
+      mvbt::write_warp<kSlowTile>(T, key, 0u, true, has, E, leaf, st, warp, slow_tile());
+    } else if (ver) {
+      const uint32_t v = mvbt::find_warp_live(T, key, has, S, at, st, warp);
+      if (has) fres[i] = v;
     } else {
-      uint32_t v = T.cooperative_find<W>(fkeys[f], tile, S, true);
-      if (tile.thread_rank() == 0) fres[f] = v;
+      mvbt::for_lanes<W>(warp.ballot(has), warp, [&](bool run, int src) {
+        const uint32_t k = warp.shfl(key, src), from = warp.shfl(at, src);
+        if (run) {
+          const uint32_t v = T.cooperative_find<W>(k, tile, S, true, from);
+          if (tile.thread_rank() == 0) fres[number * lanes + src] = v;
+        }
+      });
     }
   }
 }
@@ -338,7 +419,7 @@ __global__ void __launch_bounds__(256) k_find_sorted(device_tree T, const uint32
   }
 }
 
-template <int W, bool kStrong>
+template <int W>
 __global__ void __launch_bounds__(256) k_range_sorted(device_tree T, const uint32_t* __restrict__ slower,
                                                       const uint32_t* __restrict__ spos,
                                                       const uint32_t* __restrict__ upper, uint2* result,
@@ -352,9 +433,7 @@ __global__ void __launch_bounds__(256) k_range_sorted(device_tree T, const uint3
     if (i >= end) continue;
     const uint32_t lo = slower[i], p = spos[i];
     uint2* out        = result ? result + p * (uint64_t)avg_len : nullptr;
-    const uint32_t c  = kStrong ? T.cooperative_range_query<W>(lo, upper[p], tile, ts, out, avg_len, true,
-                                                               f.start_for(lo, tile), &f)
-                                : T.range_quiescent<W>(lo, upper[p], tile, ts, out, avg_len, f.start_for(lo, tile), &f);
+    const uint32_t c  = T.cooperative_range_query<W>(lo, upper[p], tile, ts, out, avg_len, true, f.start_for(lo, tile), &f);
     if (counts && tile.thread_rank() == 0) counts[p] = c;
   }
 }
@@ -374,7 +453,6 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
   __shared__ mvbt::write_stage stage[kWarpsPerBlock];
   __shared__ mvbt::warp_path paths[kSorted ? kWarpsPerBlock : 1];
   auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
-  auto tile             = cg::tiled_partition<kSlowTile>(cg::this_thread_block());
   mvbt::write_stage& st = stage[threadIdx.x >> 5];
   mvbt::warp_path* path = kSorted ? &paths[threadIdx.x >> 5] : nullptr;
   const uint32_t lane   = threadIdx.x & 31u;
@@ -399,7 +477,7 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
       start = path->start(__shfl_sync(0xffffffffu, k, 0), __shfl_sync(0xffffffffu, k, 31 - __clz(m)), warp);
     }
     const uint32_t leaf = mvbt::leaf_warp(T, k, live && k != mvbt::kEmptyKey, start, path, st, warp);
-    mvbt::write_warp<kSlowTile>(T, k, v, kErase, live, E, leaf, st, warp, tile);
+    mvbt::write_warp<kSlowTile>(T, k, v, kErase, live, E, leaf, st, warp, slow_tile());
   }
 }
 
@@ -451,6 +529,11 @@ unsigned grid_for_warps(const mvbt_tree* t, K kernel, uint64_t n) {
   return (unsigned)std::max<uint64_t>(g, 1);
 }
 
+// Ops per unit of the mixed kernels: 32, and fewer for a call that would leave warps idle.
+uint32_t unit_lanes(const mvbt_tree* t, uint64_t ops) {
+  return (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(4, ops / (16ull * t->num_sms)));
+}
+
 int check_launch() {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MVBT_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
@@ -462,6 +545,12 @@ int status_from_bits(uint32_t bits) {
   if (bits & mvbt::kErrSpinLimit) return MVBT_ERR_SPIN_LIMIT;
   if (bits & (mvbt::kErrCorrupt | mvbt::kErrStepLimit)) return MVBT_ERR_CORRUPT;
   return MVBT_OK;
+}
+
+// Whether range queries likewise are sorted by lower bound first.
+bool sorted_ranges(const mvbt_tree* t, uint32_t n) {
+  if (t->frontend == MVBT_FRONTEND_AUTO) return n >= (1u << 20);
+  return t->frontend == MVBT_FRONTEND_SORTED && n > 1;
 }
 
 // Fewer lookups than this leave most warps of k_find_warp empty; a tile per key has the shorter
@@ -1289,21 +1378,21 @@ int mvbt_range_query(mvbt_tree* t, const uint32_t* lower, const uint32_t* upper,
   cudaStream_t s = as_stream(stream);
   uint2* out     = reinterpret_cast<uint2*>(result);
   const int bs   = t->block_size;
-  if (use_sorted(t, n)) {
+  if (concurrent ? use_sorted(t, n) : sorted_ranges(t, n)) {
     sorted_ops so;
     int st = sort_ops(t, lower, n, kReadSortLowBit, s, &so);
     if (st) return st;
     const device_tree v = t->view();
-    if (t->tile_width == 8) {
-      if (concurrent) k_range_sorted<8, true><<<grid_for(t, k_range_sorted<8, true>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
-      else k_range_sorted<8, false><<<grid_for(t, k_range_sorted<8, false>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
-    } else {
-      if (concurrent) k_range_sorted<16, true><<<grid_for(t, k_range_sorted<16, true>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
-      else k_range_sorted<16, false><<<grid_for(t, k_range_sorted<16, false>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
-    }
+    if (!concurrent) k_range_warp<true><<<grid_for_warps(t, k_range_warp<true>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
+    else if (t->tile_width == 8) k_range_sorted<8><<<grid_for(t, k_range_sorted<8>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
+    else k_range_sorted<16><<<grid_for(t, k_range_sorted<16>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
     st = check_launch();
     const int rs = so.release(s);
     return st ? st : rs;
+  }
+  if (!concurrent && n >= kWarpFindMin) {
+    k_range_warp<false><<<grid_for_warps(t, k_range_warp<false>, n), bs, 0, s>>>(t->view(), lower, nullptr, upper, out, counts, avg_len, n, ts);
+    return check_launch();
   }
   if (t->tile_width == 8) {
     if (concurrent) k_range<8, true><<<grid_for(t, k_range<8, true>, n), bs, 0, s>>>(t->view(), lower, upper, out, counts, avg_len, n, ts);
@@ -1359,13 +1448,15 @@ int mvbt_concurrent_insert_range(mvbt_tree* t, const uint32_t* keys, const uint3
     if (st) return st;
   }
   t->grown += n_ins;
-  uint2* out = reinterpret_cast<uint2*>(result);
+  uint2* out           = reinterpret_cast<uint2*>(result);
+  const uint32_t lanes = unit_lanes(t, total);
+  const uint64_t keys32 = (((uint64_t)n_ins + lanes - 1) / lanes + ((uint64_t)n_rq + lanes - 1) / lanes) * 32;
   if (t->tile_width == 8) {
-    k_insert_range<8><<<grid_for(t, k_insert_range<8>, total), t->block_size, 0, s>>>(
-        t->view(), keys, values, n_ins, lower, upper, n_rq, out, avg_len, counts, t->d_words);
+    k_insert_range<8><<<grid_for_warps(t, k_insert_range<8>, keys32), t->block_size, 0, s>>>(
+        t->view(), keys, values, n_ins, lower, upper, n_rq, out, avg_len, counts, lanes, t->d_words);
   } else {
-    k_insert_range<16><<<grid_for(t, k_insert_range<16>, total), t->block_size, 0, s>>>(
-        t->view(), keys, values, n_ins, lower, upper, n_rq, out, avg_len, counts, t->d_words);
+    k_insert_range<16><<<grid_for_warps(t, k_insert_range<16>, keys32), t->block_size, 0, s>>>(
+        t->view(), keys, values, n_ins, lower, upper, n_rq, out, avg_len, counts, lanes, t->d_words);
   }
   return check_launch();
 }
@@ -1382,12 +1473,14 @@ int mvbt_concurrent_find_erase(mvbt_tree* t, const uint32_t* fkeys, uint32_t* fr
     int st = check_launch();
     if (st) return st;
   }
+  const uint32_t lanes  = unit_lanes(t, total);
+  const uint64_t keys32 = (((uint64_t)n_erase + lanes - 1) / lanes + ((uint64_t)n_find + lanes - 1) / lanes) * 32;
   if (t->tile_width == 8) {
-    k_find_erase<8><<<grid_for(t, k_find_erase<8>, total), t->block_size, 0, s>>>(
-        t->view(), fkeys, fres, n_find, ekeys, n_erase, t->d_words);
+    k_find_erase<8><<<grid_for_warps(t, k_find_erase<8>, keys32), t->block_size, 0, s>>>(
+        t->view(), fkeys, fres, n_find, ekeys, n_erase, lanes, t->d_words);
   } else {
-    k_find_erase<16><<<grid_for(t, k_find_erase<16>, total), t->block_size, 0, s>>>(
-        t->view(), fkeys, fres, n_find, ekeys, n_erase, t->d_words);
+    k_find_erase<16><<<grid_for_warps(t, k_find_erase<16>, keys32), t->block_size, 0, s>>>(
+        t->view(), fkeys, fres, n_find, ekeys, n_erase, lanes, t->d_words);
   }
   return check_launch();
 }

@@ -28,6 +28,7 @@ def lib():
             "emu_erase": (None, [vp, u32p, u64, i, i]),
             "emu_find": (None, [vp, u32p, u32p, u64, u32, i, i, i]),
             "emu_find_warp": (None, [vp, u32p, u32p, u32p, u64, u32, i, u32, i, u32]),
+            "emu_range_warp": (None, [vp, u32p, u32p, u32p, u32p, u32p, u32, u64, u32, i, i, i]),
             "emu_write_warp": (None, [vp, u32p, u32p, u32p, u64, i, i, i]),
             "emu_range": (None, [vp, u32p, u32p, vp, vp, u32, u64, u32, i, i, i]),
             "emu_insert_range": (None, [vp, u32p, u32p, u64, u32p, u32p, u64, vp, vp, u32, i, i]),
@@ -110,6 +111,15 @@ class EmuTree:
         self.L.emu_find_warp(self.h, np.ascontiguousarray(k[order]), order, out, k.size, ts, warps, lanes, int(sorted_run),
                              (1 << (32 - bits)) - 1)
         return out
+
+    def range_warp(self, lo, hi, avg_len, ts=0xFFFFFFFF, warps=2, live=False, sorted_run=False):
+        """Range queries by warps: quiescent (in the caller's order or in a sorted run) or live."""
+        lo, hi = _u32(lo), _u32(hi)
+        order = np.argsort(lo, kind="stable").astype(np.uint32) if sorted_run else np.arange(lo.size, dtype=np.uint32)
+        pairs, counts = np.full((lo.size, avg_len, 2), 0xFFFFFFFF, np.uint32), np.zeros(lo.size, np.uint32)
+        self.L.emu_range_warp(self.h, np.ascontiguousarray(lo[order]), hi, order, pairs.reshape(-1), counts, avg_len, lo.size,
+                              ts, warps, int(live), int(sorted_run))
+        return pairs, counts
 
     def write_warp(self, kind, keys, vals, warps=2, sorted_run=False):
         """Warp writes: kind 1 insert, 2 erase per op; sorted_run: in key order (stable) with path memory, the

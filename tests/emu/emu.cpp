@@ -323,6 +323,44 @@ void emu_find_warp(void* h, const uint32_t* keys, const uint32_t* pos, uint32_t*
   });
 }
 
+// Range queries by warps (range_warp), 32 per warp at a time; live != 0: the form that runs beside writers
+// (snapshots only), from the leaf that its descent at the newest state finds; sorted as above.
+void emu_range_warp(void* h, const uint32_t* lo, const uint32_t* hi, const uint32_t* pos, uint32_t* pairs,
+                    uint32_t* counts, uint32_t avg_len, uint64_t n, uint32_t ts, int warps, int live, int sorted) {
+  auto* t = static_cast<emu_tree*>(h);
+  auto v  = t->view();
+  if (!v.versioned) ts = mvbt::kLatest;
+  const uint64_t groups = (n + 31) / 32, per = (groups + warps - 1) / warps;
+  std::vector<mvbt::warp_stage> stage(warps);
+  std::vector<mvbt::warp_path> path(warps);
+  run_warps(warps, 8, [&](const emu_tile& warp, const emu_tile&) {
+    const uint64_t w = mvbt::emu::sm;
+    auto& st         = stage[w];
+    uint64_t g       = sorted ? w * per : w;
+    const uint64_t end = sorted ? std::min(g + per, groups) : groups;
+    if (sorted) path[w].clear(warp);
+    for (; g < end; g += sorted ? 1 : warps) {
+      const uint64_t i = g * 32 + warp.thread_rank();
+      const bool has   = i < n;
+      const uint64_t p = !has ? 0 : (sorted ? pos[i] : i);
+      const uint32_t a = has ? lo[i] : 0u, b = has ? hi[p] : 0u;
+      uint2* o         = reinterpret_cast<uint2*>(pairs) + p * (uint64_t)avg_len;
+      uint32_t start = mvbt::kAnchor, c;
+      if (live) {
+        const uint32_t leaf = mvbt::leaf_warp(v, a, has && a != mvbt::kEmptyKey, start, nullptr, st, warp);
+        c = mvbt::range_warp<true>(v, a, b, has, ts, o, avg_len, leaf == mvbt::kNone ? mvbt::kAnchor : leaf, nullptr, st, warp);
+      } else {
+        if (sorted) {
+          const uint32_t m = warp.ballot(has);
+          start = path[w].start(warp.shfl(a, 0), warp.shfl(a, 31 - __clz(m)), warp);
+        }
+        c = mvbt::range_warp<false>(v, a, b, has, ts, o, avg_len, start, sorted ? &path[w] : nullptr, st, warp);
+      }
+      if (has) counts[p] = c;
+    }
+  });
+}
+
 // Warp writes (write_warp), 32 ops per warp at a time over `warps` warps: kind 1 insert, 2 erase.
 // sorted != 0: the ops are in key order, each warp takes a contiguous run with its path memory, and of
 // a repeated key the last op alone is run.

@@ -40,6 +40,75 @@ def test_emulated_warp_lookups_match_oracle(versioned, lanes, sorted_run, bits):
     assert t.errors == 0
 
 
+def _queries(seed, q, n):
+    """Bounds around present and absent keys: empty, inverted, one key wide, over many leaves, to the end."""
+    lo = np.resize(q, n).astype(np.uint64)
+    width = np.resize(np.array([0, 1, 2, 1 << 20, 1 << 24, 1 << 27, 1 << 29], np.uint64), n)
+    hi = np.minimum(lo + width, 0xFFFFFFFF)
+    hi[::17] = lo[::17] // 2
+    return lo.astype(np.uint32), hi.astype(np.uint32)
+
+
+def _same_ranges(got, want, cap):
+    (gp, gc), (wp, wc) = got, want
+    assert np.array_equal(gc, wc)
+    mask = np.arange(cap)[None, :] < np.minimum(wc, cap)[:, None]
+    assert np.array_equal(gp[mask], wp[mask])
+    assert np.all(gp[~mask] == 0xFFFFFFFF)  # nothing past the count
+
+
+@pytest.mark.parametrize("versioned,live,sorted_run", [(False, False, False), (False, False, True), (True, False, True),
+                                                       (True, False, False), (True, True, False)])
+def test_emulated_warp_ranges_match_oracle(versioned, live, sorted_run):
+    from emu import EmuTree
+    import oracle
+    ops, q = _history(73, 700)
+    lo, hi = _queries(5, q, 150)
+    t, m = EmuTree(versioned, capacity=1 << 14, tiles=4, W=8), oracle.MVMap(versioned)
+    snaps = [] if live else [0xFFFFFFFF]
+    for kind, k, v in ops:
+        for x in (t, m):
+            x.insert(k, v) if kind == "insert" else x.erase(k)
+        if versioned:
+            snaps.append(t.snapshot())
+            assert snaps[-1] == m.take_snapshot()
+    for ts in snaps:
+        for n, cap in ((1, 4), (33, 20), (lo.size, 64)):
+            want = m.range_query(lo[:n], hi[:n], cap, ts) if versioned else m.range_query(lo[:n], hi[:n], cap)
+            _same_ranges(t.range_warp(lo[:n], hi[:n], cap, ts=ts, warps=3, live=live, sorted_run=sorted_run), want, cap)
+    assert t.errors == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("versioned,frontend", [(False, 0), (True, 1), (True, 2)])
+def test_gpu_ranges_of_warps_match_oracle(versioned, frontend):
+    import torch
+    import mvgpubtree_b200 as mv
+    import oracle
+    ops, q = _history(74, 20_000)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.uint32).view(np.int32)).cuda()
+    cls = mv.gpu_versioned_btree if versioned else mv.gpu_blink_tree
+    t, m = cls(pool_bytes=1 << 28, frontend=frontend), oracle.MVMap(versioned)
+    snaps = [mv.LATEST]
+    for kind, k, v in ops:
+        t.insert(dev(k), dev(v)) if kind == "insert" else t.erase(dev(k))
+        m.insert(k, v) if kind == "insert" else m.erase(k)
+        if versioned:
+            snaps.append(t.take_snapshot())
+            assert snaps[-1] == m.take_snapshot()
+    lo, hi = _queries(6, q, 8193)
+    for ts in snaps[:1] + snaps[2:3]:
+        for cap in (1, 13, 40):
+            want = m.range_query(lo, hi, cap, ts) if versioned else m.range_query(lo, hi, cap)
+            for n in (8191, 8192, 8193):
+                pairs = torch.full((n * cap * 2,), -1, dtype=torch.int32, device="cuda")
+                counts = torch.zeros(n, dtype=torch.int32, device="cuda")
+                t.range_query(dev(lo[:n]), dev(hi[:n]), pairs, counts, cap, timestamp=ts)
+                got = pairs.cpu().numpy().view(np.uint32).reshape(n, cap, 2), counts.cpu().numpy().view(np.uint32)
+                _same_ranges(got, (want[0][:n], want[1][:n]), cap)
+    assert t.check_errors() == 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("versioned,block", [(False, 256), (True, 256), (True, 32), (True, 96)])
 def test_gpu_lookup_sizes_around_the_rules_match_oracle(versioned, block):
