@@ -625,7 +625,7 @@ def run_ours(args, dist: Dist):
                      "kernel": "k_batched", "kernel_ms": round(avg_kms, 3),
                      "algorithmic_bytes_per_launch": int(avg_bytes), "peak_source": peak_kind},
         "clocks": clk,
-        "gpu_launches": 5 * K,
+        "gpu_launches": 4 * K,
         "verified": {"batched_vs_plain": batched_vs_plain},
     }
     if reclaim_inside is not None:

@@ -32,10 +32,9 @@ struct mvbt_batch_plan {
   uint32_t max_batches;
   // device scratch
   uint64_t* d_batch_off;  // [max_batches + 1]
-  uint32_t* d_params;     // [0] num_batches, [1] snapshot of batch 0
+  uint32_t* d_params;     // after the offsets: [0] num_batches, [1] snapshot of batch 0, [2] external watermark
   uint32_t* d_perm;       // [max_ops]
-  uint32_t* d_counts;     // n_writes | n_finds | writes_done | fill (3 classes) (each [max_batches]),
-                          // then done_batches
+  uint32_t* d_counts;     // run_scratch::counts
   uint64_t* d_pre;        // write-ordinal prefix [max_batches + 1] | read-ordinal prefix [...]
   unsigned long long* d_cursor;  // write cursor, read cursor
   // pinned staging
@@ -71,9 +70,12 @@ struct mvbt_batch_plan {
 namespace {
 
 // uint32 words of the reclamation scratch before its 64-bit part (reads_done[mb], full_done, pad)
-inline uint64_t rc_head_words(uint64_t mb) { return (mb + 2) & ~1ull; }
+__host__ __device__ inline uint64_t rc_head_words(uint64_t mb) { return (mb + 2) & ~1ull; }
 
-constexpr int kPrepassBlocks = 512;
+// Bytes of the batch offsets and the params after them, copied to the device in one piece.
+inline uint64_t stage_bytes(uint64_t mb) { return (mb + 1) * sizeof(uint64_t) + 4 * sizeof(uint32_t); }
+
+constexpr int kPrepassBlocks = 592;  // four 256-thread blocks per SM
 constexpr int kPrepassThreads = 256;
 
 int fail(int code, const std::string& msg) {
@@ -102,11 +104,76 @@ __device__ __forceinline__ uint32_t op_class(uint32_t type) {
   return mvbt::is_write_op(type) ? 0u : (type == mvbt::kOpFind ? 1u : 2u);
 }
 
-// Pass 1: writes and finds per batch (warp-aggregated atomics).
-__global__ void k_count_writes(const uint32_t* __restrict__ type, const uint64_t* __restrict__ off,
-                               const uint32_t* __restrict__ params, uint32_t* n_writes,
-                               uint32_t* n_finds) {
-  const uint32_t nb    = params[0];
+// Scratch of one persistent run, in a plan or in the no-allocation array.
+struct run_scratch {
+  uint64_t* off;               // [mb + 1] batch offsets
+  uint32_t* params;            // [0] num_batches, [1] snapshot of batch 0, [2] external watermark
+  uint32_t* counts;            // n_writes | n_finds | writes_done | fill (3 classes) (each [mb]), then
+                               // done_batches, blocks of the count pass and of the run that have finished
+  uint64_t* pre;               // wpre [mb + 1] | rpre [mb + 1]
+  unsigned long long* cursor;  // write cursor, read cursor
+  uint32_t* perm;
+  uint32_t mb;
+  // reclamation inside the run (null: off): reads_done [mb] | full_done, padded | tail_at [mb] | rc_limit
+  // | series [4 mb]
+  uint32_t* rc;
+  __host__ __device__ uint32_t* n_writes() const { return counts; }
+  __host__ __device__ uint32_t* n_finds() const { return counts + mb; }
+  __host__ __device__ uint32_t* writes_done() const { return counts + 2 * mb; }
+  __host__ __device__ uint32_t* fill() const { return counts + 3 * mb; }
+  __host__ __device__ uint32_t* done() const { return counts + 6 * mb; }
+  __host__ __device__ uint32_t* counted() const { return counts + 6 * mb + 1; }
+  __host__ __device__ uint32_t* left() const { return counts + 6 * mb + 2; }
+  __host__ __device__ uint64_t* wpre() const { return pre; }
+  __host__ __device__ uint64_t* rpre() const { return pre + (mb + 1); }
+  __host__ __device__ unsigned long long* tail_at() const {
+    return reinterpret_cast<unsigned long long*>(rc + rc_head_words(mb));
+  }
+};
+
+// Zeroes the scratch of a run (tail_at: all ones); one launch in place of a memset per array.
+__global__ void __launch_bounds__(256) k_batch_reset(run_scratch r) {
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (uint32_t i = first; i < 6 * r.mb + 4; i += stride) r.counts[i] = 0;
+  if (first < 2) r.cursor[first] = 0;
+  if (!r.rc) return;
+  for (uint32_t i = first; i < rc_head_words(r.mb); i += stride) r.rc[i] = 0;
+  unsigned long long* tail = r.tail_at();
+  for (uint32_t i = first; i < 5 * r.mb + 1; i += stride) tail[i] = i < r.mb ? ~0ull : 0ull;
+}
+
+// Exclusive scan of (w, r) over the block's 256 threads; the totals in every thread.
+__device__ __forceinline__ void block_scan_pair(uint64_t& w, uint64_t& r, uint64_t& tw, uint64_t& tr) {
+  __shared__ uint64_t s[2][8];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint64_t iw = w, ir = r;
+#pragma unroll
+  for (uint32_t d = 1; d < 32; d <<= 1) {
+    const uint64_t a = __shfl_up_sync(0xFFFFFFFFu, iw, d), b = __shfl_up_sync(0xFFFFFFFFu, ir, d);
+    if (lane >= d) iw += a, ir += b;
+  }
+  if (lane == 31) s[0][warp] = iw, s[1][warp] = ir;
+  __syncthreads();
+  uint64_t ow = 0, orr = 0;
+  tw = tr = 0;
+  for (uint32_t k = 0; k < 8; ++k) {
+    if (k == warp) ow = tw, orr = tr;
+    tw += s[0][k], tr += s[1][k];
+  }
+  w = ow + iw - w;
+  r = orr + ir - r;
+}
+
+// Pass 1: writes and finds per batch (warp-aggregated atomics). The last block to finish turns the
+// counts into the first write / read ordinal of every batch and opens the run: its first snapshot,
+// and with reclamation on the log position below which copies are free at once (the copies made
+// before this launch, epochs <= its first snapshot S0, are read by no snapshot of it; they are kept
+// only if the caller still reads a snapshot below S0, watermark params[2] < S0).
+__global__ void __launch_bounds__(kPrepassThreads) k_count_ops(const uint32_t* __restrict__ type, run_scratch r,
+                                                               mvbt::control_block* ctl) {
+  __shared__ bool last;
+  const uint64_t* off  = r.off;
+  const uint32_t nb    = r.params[0];
   const uint64_t total = off[nb];
   const uint32_t lane  = threadIdx.x & 31;
   const uint64_t warps = (uint64_t)gridDim.x * blockDim.x / 32;
@@ -119,8 +186,46 @@ __global__ void k_count_writes(const uint32_t* __restrict__ type, const uint64_t
     if (counted) {
       const uint32_t b   = batch_of(off, nb, i);
       const uint32_t grp = __match_any_sync(act, (b << 1) | c);
-      if (lane == (uint32_t)(__ffs(grp) - 1)) atomicAdd(c == 0 ? &n_writes[b] : &n_finds[b], (uint32_t)__popc(grp));
+      if (lane == (uint32_t)(__ffs(grp) - 1))
+        atomicAdd(c == 0 ? &r.n_writes()[b] : &r.n_finds()[b], (uint32_t)__popc(grp));
     }
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(r.counted(), 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const uint32_t per = (nb + blockDim.x - 1) / blockDim.x;
+  const uint32_t b0  = threadIdx.x * per;
+  const uint32_t b1  = b0 + per < nb ? b0 + per : nb;
+  uint64_t w = 0, rd = 0, tw, tr;
+  for (uint32_t b = b0; b < b1; ++b) {
+    const uint32_t n = __ldcg(&r.n_writes()[b]);
+    w += n;
+    rd += (off[b + 1] - off[b]) - n;
+  }
+  block_scan_pair(w, rd, tw, tr);
+  for (uint32_t b = b0; b < b1; ++b) {
+    const uint32_t n = __ldcg(&r.n_writes()[b]);
+    r.wpre()[b]      = w;
+    r.rpre()[b]      = rd;
+    w += n;
+    rd += (off[b + 1] - off[b]) - n;
+  }
+  if (r.rc) {
+    // unread chunks half a lap behind go back to the ring; those that fall behind while the launch
+    // runs follow in its reclamation steps
+    auto warp = cg::tiled_partition<32>(cg::this_thread_block());
+    mvbt::flush_chunks(ctl, threadIdx.x >> 5, ctl->ring_cap / 2, warp);
+  }
+  if (threadIdx.x == 0) {
+    r.wpre()[nb] = tw;
+    r.rpre()[nb] = tr;
+    __threadfence();
+    const uint32_t S0 = mvbt::ld_relaxed_u32(&ctl->epoch), ext = r.params[2];
+    r.params[1]       = S0;
+    if (r.rc) r.tail_at()[r.mb] = (ext == mvbt::kReclaimAll || S0 <= ext) ? ctl->retire_tail : ctl->retire_head;
   }
 }
 
@@ -152,75 +257,6 @@ __global__ void k_place(const uint32_t* __restrict__ type, const uint64_t* __res
   }
 }
 
-// First write / read ordinal of every batch (one block; exclusive scans over the batches).
-__global__ void __launch_bounds__(1024) k_prefix(const uint64_t* __restrict__ off,
-                                                 const uint32_t* __restrict__ params,
-                                                 const uint32_t* __restrict__ n_writes, uint64_t* wpre,
-                                                 uint64_t* rpre) {
-  __shared__ uint64_t sw[1024], sr[1024];
-  const uint32_t nb   = params[0];
-  const uint32_t per  = (nb + blockDim.x - 1) / blockDim.x;
-  const uint32_t b0   = threadIdx.x * per;
-  const uint32_t b1   = b0 + per < nb ? b0 + per : nb;
-  uint64_t w = 0, r = 0;
-  for (uint32_t b = b0; b < b1; ++b) {
-    w += n_writes[b];
-    r += (off[b + 1] - off[b]) - n_writes[b];
-  }
-  sw[threadIdx.x] = w;
-  sr[threadIdx.x] = r;
-  __syncthreads();
-  for (uint32_t d = 1; d < blockDim.x; d <<= 1) {
-    uint64_t aw = threadIdx.x >= d ? sw[threadIdx.x - d] : 0;
-    uint64_t ar = threadIdx.x >= d ? sr[threadIdx.x - d] : 0;
-    __syncthreads();
-    sw[threadIdx.x] += aw;
-    sr[threadIdx.x] += ar;
-    __syncthreads();
-  }
-  uint64_t pw = threadIdx.x ? sw[threadIdx.x - 1] : 0, pr = threadIdx.x ? sr[threadIdx.x - 1] : 0;
-  for (uint32_t b = b0; b < b1; ++b) {
-    wpre[b] = pw;
-    rpre[b] = pr;
-    pw += n_writes[b];
-    pr += (off[b + 1] - off[b]) - n_writes[b];
-  }
-  if (threadIdx.x == blockDim.x - 1) {
-    wpre[nb] = sw[blockDim.x - 1];
-    rpre[nb] = sr[blockDim.x - 1];
-  }
-}
-
-__global__ void k_batch_begin(mvbt::control_block* ctl, uint32_t* params) {
-  if (threadIdx.x == 0) {
-    __threadfence();
-    params[1] = mvbt::ld_relaxed_u32(&ctl->epoch);
-  }
-}
-
-// Reclamation on: the copies made before this launch (epochs <= its first snapshot S0) are read
-// by no snapshot of the launch, so they are reclaimable from the start unless the caller still
-// reads a snapshot below S0 (watermark params[2] < S0).
-__global__ void __launch_bounds__(256) k_batch_begin_reclaim(mvbt::control_block* ctl, const uint32_t* params,
-                                                             unsigned long long* rc_limit) {
-  // unread chunks half a lap behind go back to the ring; those that fall behind while the launch runs
-  // follow in its reclamation steps
-  auto warp = cg::tiled_partition<32>(cg::this_thread_block());
-  mvbt::flush_chunks(ctl, threadIdx.x >> 5, ctl->ring_cap / 2, warp);
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const uint32_t S0 = params[1], ext = params[2];
-    *rc_limit = (ext == mvbt::kReclaimAll || S0 <= ext) ? ctl->retire_tail : ctl->retire_head;
-  }
-}
-
-__global__ void k_batch_end(mvbt::control_block* ctl, const uint32_t* params) {
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicExch(&ctl->epoch, params[1] + params[0]);
-  }
-}
-
 struct launch_ctx {
   device_tree view;
   int W, block, sms;
@@ -245,7 +281,8 @@ unsigned occupancy_grid(const launch_ctx& c, K kernel) {
 constexpr int kWarpsPerBlock = 8;  // of 256 threads, the largest block
 
 template <int W>
-__global__ void __launch_bounds__(256, kBatchBlocks) k_batched(device_tree T, batch_view B, batch_sched sc) {
+__global__ void __launch_bounds__(256, kBatchBlocks) k_batched(device_tree T, batch_view B, batch_sched sc,
+                                                               uint32_t* left) {
   __shared__ mvbt::write_stage stage[kWarpsPerBlock];
   auto warp = cg::tiled_partition<32>(cg::this_thread_block());
   auto tile = cg::tiled_partition<W>(warp);
@@ -253,11 +290,49 @@ __global__ void __launch_bounds__(256, kBatchBlocks) k_batched(device_tree T, ba
   if (threadIdx.x == 0) gate.done = 0, gate.looked = 0;
   __syncthreads();
   mvbt::batched_worker<W>(T, B, sc, gridDim.x * (blockDim.x >> 5), gate, stage[threadIdx.x >> 5], warp, tile);
+  // the last block to finish closes the run: the epoch after its batches
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(left, 1u) == gridDim.x - 1) atomicExch(&T.ctl->epoch, sc.params[1] + sc.params[0]);
+  }
 }
 
 template <int W>
-void launch_batched(const launch_ctx& c, const batch_view& B, const batch_sched& sc, cudaStream_t s) {
-  k_batched<W><<<occupancy_grid(c, k_batched<W>), c.block, 0, s>>>(c.view, B, sc);
+void launch_batched(const launch_ctx& c, const batch_view& B, const batch_sched& sc, uint32_t* left, cudaStream_t s) {
+  k_batched<W><<<occupancy_grid(c, k_batched<W>), c.block, 0, s>>>(c.view, B, sc, left);
+}
+
+// The run's kernels once its offsets and params are in the scratch: reset, count (and open), place, run
+// (and close). begin / end: events around the run (nullable).
+void launch_run(const launch_ctx& c, const batch_view& B, const run_scratch& r, cudaStream_t s,
+                cudaEvent_t begin = nullptr, cudaEvent_t end = nullptr) {
+  k_batch_reset<<<1 + r.mb / 1024, 256, 0, s>>>(r);
+  k_count_ops<<<kPrepassBlocks, kPrepassThreads, 0, s>>>(B.type, r, c.ctl);
+  k_place<<<kPrepassBlocks, kPrepassThreads, 0, s>>>(B.type, r.off, r.params, r.n_writes(), r.n_finds(), r.fill(),
+                                                     r.mb, r.perm);
+  batch_sched sc;
+  sc.batch_off    = r.off;
+  sc.perm         = r.perm;
+  sc.n_writes     = r.n_writes();
+  sc.wpre         = r.wpre();
+  sc.rpre         = r.rpre();
+  sc.writes_done  = r.writes_done();
+  sc.done_batches = r.done();
+  sc.wcursor      = r.cursor;
+  sc.rcursor      = r.cursor + 1;
+  sc.params       = r.params;
+  if (r.rc) {
+    sc.reads_done = r.rc;
+    sc.full_done  = r.rc + r.mb;
+    sc.tail_at    = r.tail_at();
+    sc.rc_limit   = r.tail_at() + r.mb;
+    sc.series     = r.tail_at() + r.mb + 1;
+  }
+  if (begin) cudaEventRecord(begin, s);
+  if (c.W == 8) launch_batched<8>(c, B, sc, r.left(), s);
+  else launch_batched<16>(c, B, sc, r.left(), s);
+  if (end) cudaEventRecord(end, s);
 }
 
 // One batch [begin, end) in one launch: reads at the snapshot in snap_word, writes one epoch later.
@@ -287,64 +362,24 @@ __global__ void k_snapshot_word(mvbt::control_block* ctl, uint32_t* out) {
   }
 }
 
+run_scratch plan_scratch(const mvbt_batch_plan* p) {
+  run_scratch r;
+  r.off    = p->d_batch_off;
+  r.params = p->d_params;
+  r.counts = p->d_counts;
+  r.pre    = p->d_pre;
+  r.cursor = p->d_cursor;
+  r.perm   = p->d_perm;
+  r.mb     = p->max_batches;
+  r.rc     = p->reclaim_on ? static_cast<uint32_t*>(p->d_rc) : nullptr;
+  return r;
+}
+
 int enqueue_persistent(mvbt_batch_plan* p, const launch_ctx& c, const batch_view& B, cudaStream_t s) {
-  const uint32_t mb = p->max_batches;
-  MVBT_TRY(cudaMemcpyAsync(p->d_batch_off, p->h_batch_off, (mb + 1) * sizeof(uint64_t),
-                           cudaMemcpyHostToDevice, s));
-  MVBT_TRY(cudaMemcpyAsync(p->d_params, p->h_params, 3 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  MVBT_TRY(cudaMemsetAsync(p->d_counts, 0, (6ull * mb + 4) * sizeof(uint32_t), s));
-  uint32_t* rc_reads            = nullptr;
-  unsigned long long* rc_tail   = nullptr;
-  unsigned long long* rc_series = nullptr;
-  if (p->reclaim_on) {
-    rc_reads  = static_cast<uint32_t*>(p->d_rc);
-    rc_tail   = reinterpret_cast<unsigned long long*>(rc_reads + rc_head_words(mb));
-    rc_series = rc_tail + mb + 1;
-    MVBT_TRY(cudaMemsetAsync(rc_reads, 0, rc_head_words(mb) * sizeof(uint32_t), s));
-    MVBT_TRY(cudaMemsetAsync(rc_tail, 0xFF, mb * sizeof(unsigned long long), s));
-    MVBT_TRY(cudaMemsetAsync(rc_series, 0, 4ull * mb * sizeof(unsigned long long), s));
-  }
-  MVBT_TRY(cudaMemsetAsync(p->d_cursor, 0, 2 * sizeof(unsigned long long), s));
-  uint32_t* nw    = p->d_counts;
-  uint32_t* nf    = p->d_counts + mb;
-  uint32_t* wdone = p->d_counts + 2 * mb;
-  uint32_t* fill  = p->d_counts + 3 * mb;
-  uint32_t* done  = p->d_counts + 6 * mb;
-  uint64_t* wpre  = p->d_pre;
-  uint64_t* rpre  = p->d_pre + (mb + 1);
-  k_count_writes<<<kPrepassBlocks, kPrepassThreads, 0, s>>>(B.type, p->d_batch_off, p->d_params, nw, nf);
-  k_place<<<kPrepassBlocks, kPrepassThreads, 0, s>>>(B.type, p->d_batch_off, p->d_params, nw, nf, fill,
-                                                     mb, p->d_perm);
-  k_prefix<<<1, 1024, 0, s>>>(p->d_batch_off, p->d_params, nw, wpre, rpre);
-  k_batch_begin<<<1, 32, 0, s>>>(c.ctl, p->d_params);
-  if (p->reclaim_on) k_batch_begin_reclaim<<<1, 256, 0, s>>>(c.ctl, p->d_params, rc_tail + mb);
-  batch_sched sc;
-  sc.batch_off    = p->d_batch_off;
-  sc.perm         = p->d_perm;
-  sc.n_writes     = nw;
-  sc.wpre         = wpre;
-  sc.rpre         = rpre;
-  sc.writes_done  = wdone;
-  sc.done_batches = done;
-  sc.wcursor      = p->d_cursor;
-  sc.rcursor      = p->d_cursor + 1;
-  sc.params       = p->d_params;
-  if (p->reclaim_on) {
-    sc.reads_done = rc_reads;
-    sc.full_done  = rc_reads + mb;
-    sc.tail_at    = rc_tail;
-    sc.rc_limit   = rc_tail + mb;
-    sc.series     = rc_series;
-  }
+  MVBT_TRY(cudaMemcpyAsync(p->d_batch_off, p->h_batch_off, stage_bytes(p->max_batches), cudaMemcpyHostToDevice, s));
   const int slot = (int)(p->timed_runs % mvbt_batch_plan::kTimed);
-  if (p->timing) cudaEventRecord(p->ev_begin[slot], s);
-  if (c.W == 8) launch_batched<8>(c, B, sc, s);
-  else launch_batched<16>(c, B, sc, s);
-  if (p->timing) {
-    cudaEventRecord(p->ev_end[slot], s);
-    ++p->timed_runs;
-  }
-  k_batch_end<<<1, 32, 0, s>>>(c.ctl, p->d_params);
+  launch_run(c, B, plan_scratch(p), s, p->timing ? p->ev_begin[slot] : nullptr, p->timing ? p->ev_end[slot] : nullptr);
+  if (p->timing) ++p->timed_runs;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MVBT_ERR_CUDA, std::string("batched launch: ") + cudaGetErrorString(e));
   return MVBT_OK;
@@ -382,19 +417,19 @@ int mvbt_batch_plan_create(mvbt_tree* tree, uint64_t max_ops, uint32_t max_batch
   p->tree        = tree;
   p->max_ops     = max_ops;
   p->max_batches = max_batches;
-  bool ok = cudaMalloc(&p->d_batch_off, (max_batches + 1) * sizeof(uint64_t)) == cudaSuccess &&
-            cudaMalloc(&p->d_params, 64) == cudaSuccess &&
+  bool ok = cudaMalloc(&p->d_batch_off, stage_bytes(max_batches)) == cudaSuccess &&
             cudaMalloc(&p->d_perm, max_ops * sizeof(uint32_t)) == cudaSuccess &&
             cudaMalloc(&p->d_counts, (6ull * max_batches + 4) * sizeof(uint32_t)) == cudaSuccess &&
             cudaMalloc(&p->d_pre, 2ull * (max_batches + 1) * sizeof(uint64_t)) == cudaSuccess &&
             cudaMalloc(&p->d_cursor, 2 * sizeof(unsigned long long)) == cudaSuccess &&
-            cudaMallocHost(&p->h_batch_off, (max_batches + 1) * sizeof(uint64_t)) == cudaSuccess &&
-            cudaMallocHost(&p->h_params, 64) == cudaSuccess;
+            cudaMallocHost(&p->h_batch_off, stage_bytes(max_batches)) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     mvbt_batch_plan_destroy(p);
     return fail(MVBT_ERR_OUT_OF_MEMORY, "batch plan allocation failed");
   }
+  p->d_params = reinterpret_cast<uint32_t*>(p->d_batch_off + max_batches + 1);
+  p->h_params = reinterpret_cast<uint32_t*>(p->h_batch_off + max_batches + 1);
   *out = p;
   return MVBT_OK;
 }
@@ -404,13 +439,11 @@ int mvbt_batch_plan_destroy(mvbt_batch_plan* p) {
   cudaDeviceSynchronize();
   if (p->have_graph) cudaGraphExecDestroy(p->graph);
   cudaFree(p->d_batch_off);
-  cudaFree(p->d_params);
   cudaFree(p->d_perm);
   cudaFree(p->d_counts);
   cudaFree(p->d_pre);
   cudaFree(p->d_cursor);
   cudaFreeHost(p->h_batch_off);
-  cudaFreeHost(p->h_params);
   if (p->d_scratch) cudaFree(p->d_scratch);
   if (p->d_rc) cudaFree(p->d_rc);
   if (p->staging_ev) cudaEventDestroy(p->staging_ev);
@@ -765,35 +798,17 @@ extern "C" int mvbt_batch_run_noalloc(mvbt_tree* tree, uint32_t num_batches, con
   B.result    = result;
   B.range_out = reinterpret_cast<uint2*>(range_out);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // the array keeps the previous call's contents: counters and cursors start from zero again
-  MVBT_TRY(cudaMemsetAsync(counts, 0, (6ull * mb + 4) * sizeof(uint32_t), s));
-  MVBT_TRY(cudaMemsetAsync(cursor, 0, 2 * sizeof(unsigned long long), s));
+  run_scratch r;
+  r.off    = off;
+  r.params = params;
+  r.counts = counts;
+  r.pre    = pre;
+  r.cursor = cursor;
+  r.perm   = perm;
+  r.mb     = mb;
+  r.rc     = nullptr;
   k_noalloc_setup<<<1, 256, 0, s>>>(batch_off, num_batches, num_ops, off, params, c.ctl);
-  uint32_t* nw    = counts;
-  uint32_t* nf    = counts + mb;
-  uint32_t* wdone = counts + 2 * mb;
-  uint32_t* fill  = counts + 3 * mb;
-  uint32_t* done  = counts + 6 * mb;
-  uint64_t* wpre  = pre;
-  uint64_t* rpre  = pre + (mb + 1);
-  k_count_writes<<<kPrepassBlocks, kPrepassThreads, 0, s>>>(type, off, params, nw, nf);
-  k_place<<<kPrepassBlocks, kPrepassThreads, 0, s>>>(type, off, params, nw, nf, fill, mb, perm);
-  k_prefix<<<1, 1024, 0, s>>>(off, params, nw, wpre, rpre);
-  k_batch_begin<<<1, 32, 0, s>>>(c.ctl, params);
-  batch_sched sc;
-  sc.batch_off    = off;
-  sc.perm         = perm;
-  sc.n_writes     = nw;
-  sc.wpre         = wpre;
-  sc.rpre         = rpre;
-  sc.writes_done  = wdone;
-  sc.done_batches = done;
-  sc.wcursor      = cursor;
-  sc.rcursor      = cursor + 1;
-  sc.params       = params;
-  if (c.W == 8) launch_batched<8>(c, B, sc, s);
-  else launch_batched<16>(c, B, sc, s);
-  k_batch_end<<<1, 32, 0, s>>>(c.ctl, params);
+  launch_run(c, B, r, s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MVBT_ERR_CUDA, std::string("batched launch (noalloc): ") + cudaGetErrorString(e));
   return MVBT_OK;
