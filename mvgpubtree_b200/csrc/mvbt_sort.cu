@@ -1,6 +1,6 @@
 // Stable LSD radix sort of 32-bit keys with 32-bit payloads, hand-written for sm_100a: the sort
-// stage of the sorted batch front-end (mvbt_sort.h). The payload of each key is its position in
-// the caller's array, generated by the first pass.
+// stage of the sorted batch front-end (mvbt_sort.h). The payload of each key is the caller's word for
+// it, or its position in the caller's array, generated by the first pass.
 //
 // A pass over one 8-bit digit is three kernels:
 //   k_sort_hist     per tile of keys, the count of each digit (shared-memory counters), digit-major:
@@ -225,61 +225,85 @@ __global__ void __launch_bounds__(kScanThreads) k_sort_rows(uint32_t* __restrict
   if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __restrict__ a, uint64_t n,
-                                                              uint32_t* __restrict__ sums) {
-  __shared__ uint32_t s[32];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanChunk;
-  uint32_t x = 0;
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = base + (uint64_t)j * kScanThreads + threadIdx.x;
-    if (i < n) x += a[i];
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(0xffffffffu, x, d);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = x;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    uint32_t y = s[threadIdx.x];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) y += __shfl_down_sync(0xffffffffu, y, d);
-    if (threadIdx.x == 0) sums[blockIdx.x] = y;
-  }
+// Whether sorted position i of n holds a pair that a load keeps: the last occurrence of its key.
+__device__ __forceinline__ bool kept(const uint32_t* keys, uint32_t i, uint32_t n, uint32_t key) {
+  return i < n && key != 0xFFFFFFFFu && !(i + 1 < n && keys[i + 1] == key);
 }
 
-// One block: exclusive scan of the block sums in place (any count, in chunks with a carry).
-__global__ void __launch_bounds__(kScanThreads) k_scan_top(uint32_t* __restrict__ sums, uint32_t n) {
+// Kept pairs per tile of kKeepTile positions: counts[1 + tile].
+constexpr uint32_t kKeepItems = 8, kKeepTile = kThreads * kKeepItems;
+__global__ void __launch_bounds__(kThreads) k_keep_count(const uint32_t* __restrict__ keys, uint32_t n,
+                                                         uint32_t* __restrict__ counts) {
+  __shared__ uint32_t s_sum;
+  if (threadIdx.x == 0) s_sum = 0;
+  __syncthreads();
+  const uint32_t first = blockIdx.x * kKeepTile + threadIdx.x;
+  uint32_t c = 0;
+#pragma unroll
+  for (uint32_t r = 0; r < kKeepItems; ++r) {
+    const uint32_t i = first + r * kThreads;
+    if (i >= first && i < n && kept(keys, i, n, keys[i])) ++c;
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, c);
+  __syncthreads();
+  if (threadIdx.x == 0) counts[1 + blockIdx.x] = s_sum;
+}
+
+// One block: counts[1 + tile] becomes the tile's first output position, counts[0] the total.
+__global__ void __launch_bounds__(kScanThreads) k_keep_scan(uint32_t* __restrict__ counts, uint32_t tiles) {
   __shared__ uint32_t s_warp[33];
   uint32_t carry = 0;
-  for (uint32_t base = 0; base < n; base += kScanChunk) {
+  for (uint32_t base = 0; base < tiles; base += kScanChunk) {
     uint32_t v[kScanItems];
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j) {
       const uint32_t i = base + threadIdx.x * kScanItems + j;
-      v[j]             = i < n ? sums[i] : 0u;
+      v[j]             = i < tiles ? counts[1 + i] : 0u;
     }
     const uint32_t total = block_exclusive_scan(v, s_warp);
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j) {
       const uint32_t i = base + threadIdx.x * kScanItems + j;
-      if (i < n) sums[i] = v[j] + carry;
+      if (i < tiles) counts[1 + i] = v[j] + carry;
     }
     carry += total;
   }
+  if (threadIdx.x == 0) counts[0] = carry;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_down(uint32_t* __restrict__ a, uint64_t n,
-                                                            const uint32_t* __restrict__ sums) {
-  __shared__ uint32_t s_warp[33];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanChunk + (uint64_t)threadIdx.x * kScanItems;
-  uint32_t v[kScanItems];
+// The tile's kept pairs, compacted: a ballot per row of 256 positions.
+__global__ void __launch_bounds__(kThreads) k_keep_move(const uint32_t* __restrict__ keys,
+                                                        const uint32_t* __restrict__ values, uint32_t n,
+                                                        uint32_t* __restrict__ k_out, uint32_t* __restrict__ v_out,
+                                                        const uint32_t* __restrict__ counts) {
+  __shared__ uint32_t s_cnt[kKeepItems * kWarps], s_at[kKeepItems * kWarps];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t first = blockIdx.x * kKeepTile + threadIdx.x;
+  uint32_t k[kKeepItems], m[kKeepItems];
 #pragma unroll
-  for (int j = 0; j < kScanItems; ++j) v[j] = base + j < n ? a[base + j] : 0u;
-  block_exclusive_scan(v, s_warp);
-  const uint32_t off = sums[blockIdx.x];
+  for (uint32_t r = 0; r < kKeepItems; ++r) {
+    const uint32_t i = first + r * kThreads;
+    const bool ok    = i >= first && i < n;
+    k[r]             = ok ? keys[i] : 0u;
+    m[r]             = __ballot_sync(0xffffffffu, ok && kept(keys, i, n, k[r]));
+    if (lane == 0) s_cnt[r * kWarps + warp] = __popc(m[r]);
+  }
+  __syncthreads();
+  if (threadIdx.x < kKeepItems * kWarps) {  // exclusive scan of the rows' warps, in order
+    uint32_t sum = 0;
+    for (uint32_t j = 0; j < threadIdx.x; ++j) sum += s_cnt[j];
+    s_at[threadIdx.x] = sum;
+  }
+  __syncthreads();
+  const uint32_t base = counts[1 + blockIdx.x];
 #pragma unroll
-  for (int j = 0; j < kScanItems; ++j)
-    if (base + j < n) a[base + j] = v[j] + off;
+  for (uint32_t r = 0; r < kKeepItems; ++r) {
+    if (!((m[r] >> lane) & 1u)) continue;
+    const uint32_t at = base + s_at[r * kWarps + warp] + (uint32_t)__popc(m[r] & ((1u << lane) - 1u));
+    k_out[at]         = k[r];
+    v_out[at]         = values[first + r * kThreads];
+  }
 }
 
 int launch_error() {
@@ -292,19 +316,19 @@ namespace mvbt_sort {
 
 uint64_t scratch_words(uint32_t n) { return (uint64_t)kRadix * tiles_for(n) + kRadix; }
 
-uint64_t scan_scratch_words(uint64_t n) { return (n + kScanChunk - 1) / kScanChunk + 64; }
+uint64_t keep_words(uint32_t n) { return 1 + ((uint64_t)n + kKeepTile - 1) / kKeepTile; }
 
-int exclusive_scan(uint32_t* a, uint64_t n, uint32_t* sums, cudaStream_t s) {
-  if (n == 0) return 0;
-  const uint32_t chunks = (uint32_t)((n + kScanChunk - 1) / kScanChunk);
-  k_scan_reduce<<<chunks, kScanThreads, 0, s>>>(a, n, sums);
-  k_scan_top<<<1, kScanThreads, 0, s>>>(sums, chunks);
-  k_scan_down<<<chunks, kScanThreads, 0, s>>>(a, n, sums);
+int keep_last(const uint32_t* keys, const uint32_t* values, uint32_t n, uint32_t* k_out, uint32_t* v_out,
+              uint32_t* counts, cudaStream_t s) {
+  const uint32_t tiles = (uint32_t)(((uint64_t)n + kKeepTile - 1) / kKeepTile);
+  k_keep_count<<<tiles, kThreads, 0, s>>>(keys, n, counts);
+  k_keep_scan<<<1, kScanThreads, 0, s>>>(counts, tiles);
+  k_keep_move<<<tiles, kThreads, 0, s>>>(keys, values, n, k_out, v_out, counts);
   return launch_error() ? 2 : 0;
 }
 
-int sort_pairs(const uint32_t* keys, uint32_t n, int low_bit, uint32_t* k_out, uint32_t* v_out, uint32_t* k_tmp,
-               uint32_t* v_tmp, uint32_t* scratch, cudaStream_t s) {
+int sort_pairs(const uint32_t* keys, const uint32_t* payload, uint32_t n, int low_bit, uint32_t* k_out,
+               uint32_t* v_out, uint32_t* k_tmp, uint32_t* v_tmp, uint32_t* scratch, cudaStream_t s) {
   if (n == 0) return 0;
   if (low_bit < 0 || low_bit > 24 || (low_bit & 7)) return 1;
   const uint32_t tiles = tiles_for(n);
@@ -312,7 +336,7 @@ int sort_pairs(const uint32_t* keys, uint32_t n, int low_bit, uint32_t* k_out, u
   uint32_t* counts     = scratch;
   uint32_t* totals     = scratch + (uint64_t)kRadix * tiles;
   const uint32_t* kin  = keys;
-  const uint32_t* vin  = nullptr;
+  const uint32_t* vin  = payload;
   const bool large     = items_for(n) == kItemsLarge;
   for (int p = 0; p < passes; ++p) {
     // the last pass lands in k_out / v_out; earlier ones alternate so that it does

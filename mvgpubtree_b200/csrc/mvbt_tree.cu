@@ -445,10 +445,9 @@ __device__ __forceinline__ bool superseded(const uint32_t* skeys, uint64_t i, ui
 }
 
 // Inserts (kErase: erases), 32 per warp at a time (mvbt::write_warp). kSorted: the keys are a sorted
-// call's with values at their input positions, and each warp takes one contiguous run of them.
+// call's, with values in the same order, and each warp takes one contiguous run of them.
 template <bool kSorted, bool kErase>
 __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint32_t* __restrict__ keys,
-                                                       const uint32_t* __restrict__ spos,
                                                        const uint32_t* __restrict__ values, uint32_t n) {
   __shared__ mvbt::write_stage stage[kWarpsPerBlock];
   __shared__ mvbt::warp_path paths[kSorted ? kWarpsPerBlock : 1];
@@ -470,7 +469,7 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
     const uint32_t k = has ? keys[i] : 0u;
     const bool live  = has && !(kSorted && superseded(keys, i, n));
     uint32_t v       = 0;
-    if (!kErase && live) v = values[kSorted ? spos[i] : i];
+    if (!kErase && live) v = values[i];
     uint32_t start = mvbt::kAnchor;
     if (kSorted) {
       const uint32_t m = __ballot_sync(0xffffffffu, has);
@@ -487,7 +486,6 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
 // nothing visible).
 template <int W>
 __global__ void __launch_bounds__(256) k_insert_spread(device_tree T, const uint32_t* __restrict__ skeys,
-                                                       const uint32_t* __restrict__ spos,
                                                        const uint32_t* __restrict__ values, uint32_t n,
                                                        uint32_t m) {
   auto tile        = cg::tiled_partition<W>(cg::this_thread_block());
@@ -496,7 +494,7 @@ __global__ void __launch_bounds__(256) k_insert_spread(device_tree T, const uint
     if (j >= m) continue;
     const uint64_t i = j * n / m;
     if (superseded(skeys, i, n)) continue;
-    T.cooperative_insert<W>(skeys[i], values[spos[i]], tile, E);
+    T.cooperative_insert<W>(skeys[i], values[i], tile, E);
   }
 }
 
@@ -576,7 +574,7 @@ int insert_launches(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, 
     if (blocks >= full && chunk >= kWarpWriteMin) {  // the rest in one launch, 32 keys a warp
       const uint64_t in_flight = std::max<uint64_t>(1, (t->grown / 10) / t->block_size);  // about a key per leaf
       const unsigned grid      = (unsigned)std::min<uint64_t>(grid_for_warps(t, k_write_warp<false, false>, chunk), in_flight);
-      k_write_warp<false, false><<<grid, t->block_size, 0, s>>>(t->view(), keys + done, nullptr, values + done, (uint32_t)chunk);
+      k_write_warp<false, false><<<grid, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);
     } else {
       blocks = std::min(blocks, full);
       k_insert<W><<<(unsigned)blocks, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);
@@ -631,11 +629,12 @@ int sort_pool(int dev, cudaMemPool_t* out) {
   return MVBT_OK;
 }
 
-// The keys of a call in ascending order with their input positions, in pool memory released by
-// release() (stream-ordered, after the kernels that read it).
+// The keys of a call in ascending order with their values (inserts) or input positions, in pool memory
+// released by release() (stream-ordered, after the kernels that read it). Inserts sort their values
+// along: fetched by position afterwards they were a scattered 4-byte read per key.
 struct sorted_ops {
   uint32_t* keys = nullptr;
-  uint32_t* pos  = nullptr;
+  uint32_t* pos  = nullptr;  // or the values
   uint32_t* extra = nullptr;  // extra_words of scratch after the sort's own (64-word aligned)
   void* mem      = nullptr;
   int release(cudaStream_t s) {
@@ -646,7 +645,7 @@ struct sorted_ops {
 };
 
 int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaStream_t s, sorted_ops* out,
-             uint64_t extra_words = 0) {
+             const uint32_t* values = nullptr, uint64_t extra_words = 0) {
   cudaMemPool_t pool;
   int st = sort_pool(t->device, &pool);
   if (st) return st;
@@ -662,7 +661,7 @@ int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaSt
   out->keys   = w;
   out->pos    = w + n;
   out->extra  = extra_words ? w + sort_words : nullptr;
-  if (mvbt_sort::sort_pairs(keys, n, low_bit, w, w + n, w + 2ull * n, w + 3ull * n, w + 4ull * n, s)) {
+  if (mvbt_sort::sort_pairs(keys, values, n, low_bit, w, w + n, w + 2ull * n, w + 3ull * n, w + 4ull * n, s)) {
     out->release(s);
     return fail(MVBT_ERR_CUDA, std::string("sort launch: ") + cudaGetErrorString(cudaGetLastError()));
   }
@@ -670,7 +669,7 @@ int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaSt
 }
 
 template <int W>
-int insert_sorted_launches(mvbt_tree* t, const sorted_ops& so, const uint32_t* values, uint32_t n, cudaStream_t s) {
+int insert_sorted_launches(mvbt_tree* t, const sorted_ops& so, uint32_t n, cudaStream_t s) {
   const uint64_t full  = grid_for(t, k_insert_spread<W>, n);
   const uint64_t tiles = (uint64_t)t->block_size / W;
   uint64_t spread      = 0;
@@ -678,14 +677,14 @@ int insert_sorted_launches(mvbt_tree* t, const sorted_ops& so, const uint32_t* v
     uint64_t blocks = std::max<uint64_t>(1, (t->grown / 10) / tiles);
     blocks          = std::min(blocks, full);
     uint64_t m      = std::min<uint64_t>(n, std::max<uint64_t>(t->grown, blocks * tiles * 16));
-    k_insert_spread<W><<<(unsigned)blocks, t->block_size, 0, s>>>(t->view(), so.keys, so.pos, values, n, (uint32_t)m);
+    k_insert_spread<W><<<(unsigned)blocks, t->block_size, 0, s>>>(t->view(), so.keys, so.pos, n, (uint32_t)m);
     int st = check_launch();
     if (st) return st;
     t->grown += m;
     spread = m;
   }
   if (spread < n) {
-    k_write_warp<true, false><<<grid_for_warps(t, k_write_warp<true, false>, n), t->block_size, 0, s>>>(t->view(), so.keys, so.pos, values, n);
+    k_write_warp<true, false><<<grid_for_warps(t, k_write_warp<true, false>, n), t->block_size, 0, s>>>(t->view(), so.keys, so.pos, n);
     int st = check_launch();
     if (st) return st;
     t->grown += n - spread;
@@ -980,35 +979,14 @@ __global__ void k_bulk_anchor(uint32_t* pool, control_block* c, const bulk_plan*
 }
 
 // ---- insert into a pristine tree: a bulk load of the sorted call ----
-// keep[i] = 1 for the last occurrence of each key (the one an in-order upsert leaves), 0 for an
-// earlier occurrence and for the reserved key 0xFFFFFFFF (which insert ignores).
-__global__ void k_keep_flags(const uint32_t* __restrict__ skeys, uint64_t n, uint32_t* __restrict__ keep) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    keep[i] = (skeys[i] != mvbt::kEmptyKey && !(i + 1 < n && skeys[i + 1] == skeys[i])) ? 1u : 0u;
-}
-// After the exclusive scan of keep (at[i] = output position): the kept pairs, compacted.
-__global__ void k_keep_compact(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ spos,
-                               const uint32_t* __restrict__ values, const uint32_t* __restrict__ at, uint64_t n,
-                               uint32_t* __restrict__ ck, uint32_t* __restrict__ cv) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t k = skeys[i];
-    if (k != mvbt::kEmptyKey && !(i + 1 < n && skeys[i + 1] == k)) {
-      ck[at[i]] = k;
-      cv[at[i]] = values[spos[i]];
-    }
-  }
-}
-// One thread: the plan for the compacted pairs (their count is at[n - 1] + keep(n - 1)).
-__global__ void k_bulk_plan_kept(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ at, uint64_t n,
-                                 const uint32_t* ck, const uint32_t* cv, uint32_t fill, uint64_t capacity,
-                                 bulk_plan* plan) {
-  const uint32_t last = skeys[n - 1];
-  const uint64_t kept = (uint64_t)at[n - 1] + (last != mvbt::kEmptyKey ? 1u : 0u);
+// One thread: the plan for the kept pairs (mvbt_sort::keep_last).
+__global__ void k_bulk_plan_kept(const uint32_t* __restrict__ kept, const uint32_t* ck, const uint32_t* cv,
+                                 uint32_t fill, uint64_t capacity, bulk_plan* plan) {
   bulk_plan P;
   P.keys   = ck;
   P.values = cv;
-  P.off    = (kept && ck[0] == 0u) ? 0u : 1u;  // key 0 in the call replaces the tombstone's value
-  P.m      = kept + P.off;
+  P.off    = (*kept && ck[0] == 0u) ? 0u : 1u;  // key 0 in the call replaces the tombstone's value
+  P.m      = (uint64_t)*kept + P.off;
   P.L.fill = fill;
   plan_levels(P, capacity);
   *plan = P;
@@ -1259,27 +1237,23 @@ namespace {
 constexpr uint32_t kLoadFill = 10;
 constexpr uint32_t kLoadMin  = 1u << 12;  // smaller inserts into a pristine tree go key by key
 
-// Scratch of a bulk load after the sort's own: keep[n] | scan sums | the plan. Every region starts
-// on a 64-word (256-byte) boundary: the plan holds 64-bit fields, and n may be odd.
+// Scratch of a bulk load after the sort's own: the kept pairs' counts | the plan. Every region starts
+// on a 64-word (256-byte) boundary: the plan holds 64-bit fields.
 inline uint64_t round64(uint64_t words) { return (words + 63) & ~63ull; }
 uint64_t bulk_load_extra_words(uint32_t n) {
-  return round64(n) + round64(mvbt_sort::scan_scratch_words(n)) + round64((sizeof(bulk_plan) + 3) / 4);
+  return round64(mvbt_sort::keep_words(n)) + round64((sizeof(bulk_plan) + 3) / 4);
 }
 
 // Insert of a sorted call into a pristine tree: the last occurrence of every key, compacted, built
 // bottom up (k_bulk_build) in place of the tombstone leaf. Stream-ordered, no host round trip: the
 // entry count and the level plan are computed on the device.
-int bulk_load_sorted(mvbt_tree* t, const sorted_ops& so, const uint32_t* values, uint32_t n, cudaStream_t s) {
-  uint32_t* ck   = so.keys + 2ull * n;  // the sort's ping-pong buffers are free again
-  uint32_t* cv   = so.keys + 3ull * n;
-  uint32_t* keep = so.extra;
-  uint32_t* sums = so.extra + round64(n);
-  auto* plan     = reinterpret_cast<bulk_plan*>(sums + round64(mvbt_sort::scan_scratch_words(n)));
-  const unsigned grid = (unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, (uint64_t)t->num_sms * 16);
-  k_keep_flags<<<grid, 256, 0, s>>>(so.keys, n, keep);
-  if (mvbt_sort::exclusive_scan(keep, n, sums, s)) return check_launch();
-  k_keep_compact<<<grid, 256, 0, s>>>(so.keys, so.pos, values, keep, n, ck, cv);
-  k_bulk_plan_kept<<<1, 1, 0, s>>>(so.keys, keep, n, ck, cv, kLoadFill, t->capacity, plan);
+int bulk_load_sorted(mvbt_tree* t, const sorted_ops& so, uint32_t n, cudaStream_t s) {
+  uint32_t* ck     = so.keys + 2ull * n;  // the sort's ping-pong buffers are free again
+  uint32_t* cv     = so.keys + 3ull * n;
+  uint32_t* counts = so.extra;
+  auto* plan       = reinterpret_cast<bulk_plan*>(counts + round64(mvbt_sort::keep_words(n)));
+  if (mvbt_sort::keep_last(so.keys, so.pos, n, ck, cv, counts, s)) return check_launch();
+  k_bulk_plan_kept<<<1, 1, 0, s>>>(counts, ck, cv, kLoadFill, t->capacity, plan);
   const uint64_t threads = bulk_nodes_bound((uint64_t)n + 1, kLoadFill) * 32;
   k_bulk_build<<<(unsigned)std::min<uint64_t>((threads + 255) / 256, (uint64_t)t->num_sms * 64), 256, 0, s>>>(t->pool, plan);
   k_bulk_anchor<<<1, 32, 0, s>>>(t->pool, t->ctl, plan);
@@ -1298,13 +1272,13 @@ int mvbt_insert(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, uint
   t->pristine     = false;
   if (load || use_sorted(t, n)) {
     sorted_ops so;
-    int st = sort_ops(t, keys, n, 0, s, &so, load ? bulk_load_extra_words(n) : 0);
+    int st = sort_ops(t, keys, n, 0, s, &so, values, load ? bulk_load_extra_words(n) : 0);
     if (st) return st;
     if (load)
-      st = bulk_load_sorted(t, so, values, n, s);
+      st = bulk_load_sorted(t, so, n, s);
     else
-      st = t->tile_width == 8 ? insert_sorted_launches<8>(t, so, values, n, s)
-                              : insert_sorted_launches<16>(t, so, values, n, s);
+      st = t->tile_width == 8 ? insert_sorted_launches<8>(t, so, n, s)
+                              : insert_sorted_launches<16>(t, so, n, s);
     const int rs = so.release(s);
     return st ? st : rs;
   }
@@ -1354,13 +1328,13 @@ int mvbt_erase(mvbt_tree* t, const uint32_t* keys, uint32_t n, void* stream, int
     sorted_ops so;
     int st = sort_ops(t, keys, n, 0, s, &so);
     if (st) return st;
-    k_write_warp<true, true><<<grid_for_warps(t, k_write_warp<true, true>, n), t->block_size, 0, s>>>(t->view(), so.keys, nullptr, nullptr, n);
+    k_write_warp<true, true><<<grid_for_warps(t, k_write_warp<true, true>, n), t->block_size, 0, s>>>(t->view(), so.keys, nullptr, n);
     st = check_launch();
     const int rs = so.release(s);
     return st ? st : rs;
   }
   if (n >= kWarpWriteMin) {
-    k_write_warp<false, true><<<grid_for_warps(t, k_write_warp<false, true>, n), t->block_size, 0, s>>>(t->view(), keys, nullptr, nullptr, n);
+    k_write_warp<false, true><<<grid_for_warps(t, k_write_warp<false, true>, n), t->block_size, 0, s>>>(t->view(), keys, nullptr, n);
   } else if (t->tile_width == 8) {
     k_erase<8><<<grid_for(t, k_erase<8>, n), t->block_size, 0, s>>>(t->view(), keys, n);
   } else {
