@@ -879,12 +879,10 @@ struct finger {
   uint32_t idx  = kNone;
   uint32_t low  = 0;
   uint32_t high = 0;
-  // Lowest remembered node covering key, or the anchor. level (nullable): that node's level, or
-  // kNone for the anchor.
+  // Lowest remembered node covering key, or the anchor.
   template <class Tile>
-  MVBT_DEV uint32_t start_for(uint32_t key, const Tile& t, uint32_t* level = nullptr) const {
+  MVBT_DEV uint32_t start_for(uint32_t key, const Tile& t) const {
     const uint32_t m = t.ballot(idx != kNone && low <= key && key < high);
-    if (level) *level = m ? (uint32_t)(__ffs(m) - 1) : kNone;
     return m ? t.shfl(idx, __ffs(m) - 1) : kAnchor;
   }
   template <class Tile>
@@ -894,11 +892,6 @@ struct finger {
       low  = lo;
       high = hi;
     }
-  }
-  // The interior node remembered at `level` (kNone if none): the parent hint of insert_at.
-  template <class Tile>
-  MVBT_DEV uint32_t at(uint32_t level, const Tile& t) const {
-    return level < (uint32_t)W ? t.shfl(idx, (int)level) : kNone;
   }
 };
 
@@ -1310,14 +1303,13 @@ struct device_tree {
   }
 
   // The point lookup of a tree no writer changes meanwhile (concurrent = false): the same route
-  // and result as cooperative_find(key, t, ts, false, start, f), but every lane loads the header
+  // and result as cooperative_find(key, t, ts), but every lane loads the header
   // words itself (ld_header_words) beside its share of the node instead of receiving them by
   // shuffle, and the versions a snapshot read passes over are read as headers alone.
   template <int W, class Tile>
-  MVBT_DEV uint32_t find_quiescent(uint32_t key, const Tile& t, uint32_t ts = kLatest, uint32_t start = kAnchor,
-                                   finger<W>* f = nullptr) const {
+  MVBT_DEV uint32_t find_quiescent(uint32_t key, const Tile& t, uint32_t ts = kLatest) const {
     const bool snap = versioned && ts != kLatest;
-    uint32_t idx    = start;
+    uint32_t idx    = kAnchor;
     node_regs<W> n;
     for (uint32_t step = 0; step < kMaxSteps; ++step) {
       if (!valid(idx, t)) return kNotFound;
@@ -1340,10 +1332,8 @@ struct device_tree {
         continue;
       }
       if (h.is_leaf()) {
-        if (f) f->record(0, idx, h.low, h.high, t);
         return leaf_value<W>(n, key, t);
       }
-      if (f) f->record(h.level(), idx, h.low, h.high, t);
       idx = child_for<W>(n, key, t);
       if (idx == kNone) idx = kAnchor;
     }
@@ -1470,15 +1460,15 @@ struct device_tree {
   }
 
   // The range query of a tree no writer changes meanwhile (concurrent = false): the same route
-  // and result as cooperative_range_query(lo, hi, t, ts, out, cap, false, start, f), with every
+  // and result as cooperative_range_query(lo, hi, t, ts, out, cap), with every
   // lane loading the header words itself (as find_quiescent) on the descent and along the leaf
   // chain, and the versions a snapshot read passes over read as headers alone.
   template <int W, class Tile>
   MVBT_DEV uint32_t range_quiescent(uint32_t lo, uint32_t hi, const Tile& t, uint32_t ts, uint2* out,
-                                    uint32_t cap, uint32_t start = kAnchor, finger<W>* f = nullptr) const {
+                                    uint32_t cap) const {
     if (hi <= lo) return 0;
     const bool snap = versioned && ts != kLatest;
-    uint32_t idx    = start;
+    uint32_t idx    = kAnchor;
     node_regs<W> n;
     header h;
     for (uint32_t step = 0;; ++step) {  // descend to the leaf that holds lo
@@ -1506,10 +1496,8 @@ struct device_tree {
         continue;
       }
       if (h.is_leaf()) {
-        if (f) f->record(0, idx, h.low, h.high, t);
         break;
       }
-      if (f) f->record(h.level(), idx, h.low, h.high, t);
       idx = child_for<W>(n, lo, t);
       if (idx == kNone) idx = kAnchor;
     }
@@ -1540,120 +1528,6 @@ struct device_tree {
   // ------------------------------------------------------------------------------------------
   // Writers
   // ------------------------------------------------------------------------------------------
-  // Descent of a writer in a sorted run: like descend_for_write, but it starts at the lowest node
-  // of f covering key and records every interior node it passes in f, which then serves as the
-  // path of parent hints (insert_at with path0 = f's per-lane nodes). The leaf is recorded by the
-  // caller once it has read it under its lock.
-  template <int W, class Tile>
-  MVBT_DEV uint32_t descend_with_finger(uint32_t key, finger<W>& f, const Tile& t) const {
-    uint32_t start_level;
-    uint32_t idx = f.start_for(key, t, &start_level);
-    if (start_level == 0) return idx;  // the leaf of the previous op covers key
-    node_regs<W> n;
-    for (uint32_t step = 0; step < kMaxSteps; ++step) {
-      if (!valid(idx, t)) return kNone;
-      load<W>(idx, n, true, t);
-      header h = get_header<W>(n, t);
-      if (key < h.low) {  // a torn read upstream routed too far right: start over from the anchor
-        idx = kAnchor;
-        continue;
-      }
-      if (key >= h.high && h.sibling() != kNone) {
-        idx = h.sibling();
-        continue;
-      }
-      f.record(h.level(), idx, h.low, h.high, t);
-      if (h.is_leaf()) return idx;  // reached through a sibling link or a misrouted read
-      const uint32_t child = child_for<W>(n, key, t);
-      if (child == kNone) {
-        idx = kAnchor;
-        continue;
-      }
-      if (h.level() == 1) return child;  // a leaf: read under the lock, not before it
-      idx = child;
-    }
-    if (t.thread_rank() == 0) set_error(kErrStepLimit, 8);
-    return kNone;
-  }
-
-  // Insert / erase of one key of a sorted run (the sorted batch front-end): the descent starts
-  // from the run's path memory f instead of the anchor.
-  template <int W, class Tile>
-  MVBT_DEV bool insert_in_run(uint32_t key, uint32_t value, const Tile& t, uint32_t E, finger<W>& f) const {
-    if (key == kEmptyKey) return false;
-    const uint32_t leaf = descend_with_finger<W>(key, f, t);
-    if (leaf == kNone) return false;
-    return insert_at<W>(key, value, t, E, leaf, f.idx, kNone, (uint32_t)W - 1, &f);
-  }
-
-  // Inserts the keys of a sorted run that land in one leaf under a single lock (the sorted batch
-  // front-end): skeys[i] ascending, its value at values[spos[i]]. The leaf of skeys[i] is locked
-  // and prepared for epoch E once; then that key and each following key of the run below the
-  // leaf's high fence is merged into the node in registers while the leaf has room, and the leaf
-  // is stored and released once. A key that finds the leaf full splits it (split_insert), its
-  // separators go up as in insert_at, and the group ends there. Keys repeated in the run count at
-  // their last occurrence only (i + 1 < n_all with the same key: skipped); the caller starts a
-  // group at such a last occurrence. Advances i past every key the group consumed (at least one).
-  template <int W, class Tile>
-  MVBT_DEV void insert_run_group(const uint32_t* skeys, const uint32_t* spos, const uint32_t* values,
-                                 uint64_t& i, uint64_t end, uint64_t n_all, const Tile& t, uint32_t E,
-                                 finger<W>& f) const {
-    uint32_t key = skeys[i];
-    if (key == kEmptyKey) {  // not a key; the run is sorted, so every later one is the same
-      i = end;
-      return;
-    }
-    node_regs<W> n;
-    header h;
-    uint32_t leaf = descend_with_finger<W>(key, f, t);
-    if (leaf != kNone) leaf = lock_covering<W>(leaf, 0, key, n, h, t, true);
-    if (leaf == kNone) {
-      ++i;
-      return;
-    }
-    f.record(0, leaf, h.low, h.high, t);
-    if (!prepare_write<W>(leaf, n, h, E, t)) {
-      unlock(leaf, t);
-      ++i;
-      return;
-    }
-    int nvalid = count_valid<W>(n, t);
-    for (;;) {
-      const uint32_t value = values[spos[i]];
-      ++i;
-      const int pos = find_pos<W>(n, key, t);
-      if (pos >= 0) {
-#pragma unroll
-        for (int j = 0; j < 16 / W; ++j)
-          if (pair_index<W>(t, j) == pos) n.v[j] = value;
-      } else if (nvalid < kDataPairs) {
-        node_regs<W> out;
-        build_from_merged<W>(n, count_less<W>(n, key, t), key, value, 0, nvalid + 1, out, t);
-        n = out;
-        ++nvalid;
-      } else {  // full: split with this key (stores the node, releases it) and end the group
-        uint32_t sep_key = 0, sep_child = kNone;
-        if (split_insert<W>(leaf, n, h, key, value, E, sep_key, sep_child, t))
-          push_up<W>(sep_key, sep_child, E, f.idx, kNone, (uint32_t)W - 1, t);
-        return;
-      }
-      while (i < end && i + 1 < n_all && skeys[i + 1] == skeys[i]) ++i;
-      if (i >= end) break;
-      key = skeys[i];
-      if (key >= h.high || key == kEmptyKey) break;
-    }
-    store<W>(leaf, n, t);
-    release(leaf, h, t);
-  }
-
-  template <int W, class Tile>
-  MVBT_DEV bool erase_in_run(uint32_t key, const Tile& t, uint32_t E, finger<W>& f) const {
-    if (key == kEmptyKey) return false;
-    const uint32_t leaf = descend_with_finger<W>(key, f, t);
-    if (leaf == kNone) return false;
-    return erase_at<W>(key, t, E, leaf, &f);
-  }
-
   // Descends to the leaf for key (newest versions, strong loads), recording in `path` the
   // interior node visited at each level: lane l holds level l in path0 and level l + W in path1.
   // Returns the leaf its level-1 parent names without reading it: the writer reads it under its
@@ -1880,17 +1754,15 @@ struct device_tree {
   // The insert after its descent: `leaf` and the path (path0 / path1 / top, as descend_for_write
   // records them) may have been found before other writers changed the tree; lock_covering moves
   // right as far as needed and a stale path entry only lengthens the approach to a parent.
-  // f (nullable): path memory of a sorted run, which records the leaf as read under the lock.
   template <int W, class Tile>
   MVBT_DEV bool insert_at(uint32_t key, uint32_t value, const Tile& t, uint32_t E, uint32_t leaf,
-                          uint32_t path0, uint32_t path1, uint32_t top, finger<W>* f = nullptr) const {
+                          uint32_t path0, uint32_t path1, uint32_t top) const {
     if (key == kEmptyKey) return false;
     {
       node_regs<W> n;
       header h;
       leaf = lock_covering<W>(leaf, 0, key, n, h, t, true);
       if (leaf == kNone) return false;
-      if (f) f->record(0, leaf, h.low, h.high, t);
       // update in place if present
       int pos = find_pos<W>(n, key, t);
       if (pos >= 0) {
@@ -1980,16 +1852,14 @@ struct device_tree {
     return erase_at<W>(key, t, E, leaf);
   }
 
-  // The erase after its descent (the leaf may be stale: lock_covering moves right). f (nullable):
-  // as in insert_at.
+  // The erase after its descent (the leaf may be stale: lock_covering moves right).
   template <int W, class Tile>
-  MVBT_DEV bool erase_at(uint32_t key, const Tile& t, uint32_t E, uint32_t leaf, finger<W>* f = nullptr) const {
+  MVBT_DEV bool erase_at(uint32_t key, const Tile& t, uint32_t E, uint32_t leaf) const {
     if (key == kEmptyKey) return false;
     node_regs<W> n;
     header h;
     leaf = lock_covering<W>(leaf, 0, key, n, h, t, true);
     if (leaf == kNone) return false;
-    if (f) f->record(0, leaf, h.low, h.high, t);
     int pos = find_pos<W>(n, key, t);
     if (pos < 0) {
       unlock(leaf, t);

@@ -1339,14 +1339,17 @@ int mvbt_find(mvbt_tree* t, const uint32_t* keys, uint32_t* values, uint32_t n, 
   if (concurrent ? use_sorted(t, n) : sorted_lookups(t, n)) {
     sorted_ops so;
     int st = sort_ops(t, keys, n, kReadSortLowBit, s, &so);
-    if (st) return st;
-    const device_tree v = t->view();
-    if (!concurrent) k_find_warp<true><<<grid_for_warps(t, k_find_warp<true>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
-    else if (t->tile_width == 8) k_find_sorted<8><<<grid_for(t, k_find_sorted<8>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
-    else k_find_sorted<16><<<grid_for(t, k_find_sorted<16>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
-    st = check_launch();
-    const int rs = so.release(s);
-    return st ? st : rs;
+    // without memory for the sort a call that need not be sorted runs in the caller's order
+    if (st != MVBT_ERR_OUT_OF_MEMORY || t->frontend == MVBT_FRONTEND_SORTED) {
+      if (st) return st;
+      const device_tree v = t->view();
+      if (!concurrent) k_find_warp<true><<<grid_for_warps(t, k_find_warp<true>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
+      else if (t->tile_width == 8) k_find_sorted<8><<<grid_for(t, k_find_sorted<8>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
+      else k_find_sorted<16><<<grid_for(t, k_find_sorted<16>, n), bs, 0, s>>>(v, so.keys, so.pos, values, n, ts);
+      st = check_launch();
+      const int rs = so.release(s);
+      return st ? st : rs;
+    }
   }
   if (!concurrent && n >= kWarpFindMin) {
     k_find_warp<false><<<grid_for_warps(t, k_find_warp<false>, n), bs, 0, s>>>(t->view(), keys, nullptr, values, n, ts);
@@ -1399,14 +1402,17 @@ int mvbt_range_query(mvbt_tree* t, const uint32_t* lower, const uint32_t* upper,
   if (concurrent ? use_sorted(t, n) : sorted_ranges(t, n)) {
     sorted_ops so;
     int st = sort_ops(t, lower, n, kReadSortLowBit, s, &so);
-    if (st) return st;
-    const device_tree v = t->view();
-    if (!concurrent) k_range_warp<true><<<grid_for_warps(t, k_range_warp<true>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
-    else if (t->tile_width == 8) k_range_sorted<8><<<grid_for(t, k_range_sorted<8>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
-    else k_range_sorted<16><<<grid_for(t, k_range_sorted<16>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
-    st = check_launch();
-    const int rs = so.release(s);
-    return st ? st : rs;
+    // without memory for the sort a call that need not be sorted runs in the caller's order
+    if (st != MVBT_ERR_OUT_OF_MEMORY || t->frontend == MVBT_FRONTEND_SORTED) {
+      if (st) return st;
+      const device_tree v = t->view();
+      if (!concurrent) k_range_warp<true><<<grid_for_warps(t, k_range_warp<true>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
+      else if (t->tile_width == 8) k_range_sorted<8><<<grid_for(t, k_range_sorted<8>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
+      else k_range_sorted<16><<<grid_for(t, k_range_sorted<16>, n), bs, 0, s>>>(v, so.keys, so.pos, upper, out, counts, avg_len, n, ts);
+      st = check_launch();
+      const int rs = so.release(s);
+      return st ? st : rs;
+    }
   }
   if (!concurrent && n >= kWarpFindMin) {
     k_range_warp<false><<<grid_for_warps(t, k_range_warp<false>, n), bs, 0, s>>>(t->view(), lower, nullptr, upper, out, counts, avg_len, n, ts);

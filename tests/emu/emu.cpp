@@ -431,10 +431,10 @@ void emu_insert_range(void* h, const uint32_t* keys, const uint32_t* vals, uint6
 }
 
 // Sorted runs (the sorted batch front-end): keys[0, n) ascending, pos[i] = the input position of
-// keys[i]; each of `tiles` tiles takes one contiguous share of the run and keeps its path memory
-// (mvbt::finger, one per lane, as registers are on the GPU). kind: 0 find, 1 range, 2 insert (a
-// repeated key: its last occurrence wins; the keys of one leaf under one lock), 3 erase, 4 find and
-// 5 range of a tree no writer changes meanwhile.
+// keys[i]. kind: 0 find, 1 range beside writers, each of `tiles` tiles taking one contiguous share of the
+// run with its path memory (mvbt::finger, one per lane, as registers are on the GPU); 2 insert (a
+// repeated key: its last occurrence wins), 3 erase, 4 find and 5 range of a tree no writer changes
+// meanwhile, by as many warps as the tiles make.
 void emu_sorted_run(void* h, int kind, const uint32_t* keys, const uint32_t* pos, const uint32_t* arg,
                     uint32_t* out, uint32_t* pairs, uint32_t avg_len, uint64_t n, uint32_t ts, int tiles, int W) {
   auto* t = static_cast<emu_tree*>(h);
@@ -442,6 +442,18 @@ void emu_sorted_run(void* h, int kind, const uint32_t* keys, const uint32_t* pos
   if (!v.versioned) ts = mvbt::kLatest;
   if (n == 0) return;
   if (tiles < 1) tiles = 1;
+  if (kind >= 2) {
+    const int warps = std::max(1, tiles * W / 32);
+    if (kind == 4) return emu_find_warp(h, keys, pos, out, n, ts, warps, 32, 1, 0);
+    if (kind == 5) {
+      std::vector<uint32_t> none(pairs ? 0 : 2 * n * (uint64_t)avg_len), counts(out ? 0 : n);
+      return emu_range_warp(h, keys, arg, pos, pairs ? pairs : none.data(), out ? out : counts.data(), avg_len, n, ts, warps, 0, 1);
+    }
+    std::vector<uint32_t> kinds(n, kind == 2 ? 1u : 2u), vals(n, 0u);
+    if (kind == 2)
+      for (uint64_t i = 0; i < n; ++i) vals[i] = arg[pos[i]];
+    return emu_write_warp(h, kinds.data(), keys, vals.data(), n, warps, W, 1);
+  }
   const uint64_t per = (n + tiles - 1) / tiles;
   EMU_DISPATCH(W, {
     std::vector<std::unique_ptr<tile_shared>> sh;
@@ -453,37 +465,17 @@ void emu_sorted_run(void* h, int kind, const uint32_t* keys, const uint32_t* pos
           mvbt::emu::sm = (uint32_t)x;
           emu_tile tile{l, kW, sh[x].get()};
           mvbt::finger<kW> f;
-          const uint32_t E = v.versioned ? v.current_epoch() : 0u;
           const uint64_t b = (uint64_t)x * per, e = std::min<uint64_t>(n, b + per);
           for (uint64_t i = b; i < e; ++i) {
             const uint32_t k = keys[i];
-            if (kind == 2) {
-              while (i < e) {
-                if (i + 1 < n && keys[i + 1] == keys[i]) {
-                  ++i;
-                  continue;
-                }
-                v.insert_run_group<kW>(keys, pos, arg, i, e, n, tile, E, f);
-              }
-              break;
-            }
-            if (kind == 4) {
-              const uint32_t r = v.find_quiescent<kW>(k, tile, ts, f.start_for(k, tile), &f);
-              if (tile.thread_rank() == 0) out[pos[i]] = r;
-            } else if (kind == 5) {
-              uint2* o = pairs ? reinterpret_cast<uint2*>(pairs) + pos[i] * (uint64_t)avg_len : nullptr;
-              const uint32_t c = v.range_quiescent<kW>(k, arg[pos[i]], tile, ts, o, avg_len, f.start_for(k, tile), &f);
-              if (out && tile.thread_rank() == 0) out[pos[i]] = c;
-            } else if (kind == 0) {
+            if (kind == 0) {
               const uint32_t r = v.cooperative_find<kW>(k, tile, ts, true, f.start_for(k, tile), &f);
               if (tile.thread_rank() == 0) out[pos[i]] = r;
-            } else if (kind == 1) {
+            } else {
               uint2* o = pairs ? reinterpret_cast<uint2*>(pairs) + pos[i] * (uint64_t)avg_len : nullptr;
               const uint32_t c = v.cooperative_range_query<kW>(k, arg[pos[i]], tile, ts, o, avg_len, true,
                                                                f.start_for(k, tile), &f);
               if (out && tile.thread_rank() == 0) out[pos[i]] = c;
-            } else {
-              v.erase_in_run<kW>(k, tile, E, f);
             }
           }
         });
