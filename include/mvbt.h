@@ -88,11 +88,13 @@ typedef struct mvbt_config {
  * occurrence in the array wins; the top 24 bits for reads, which only need locality) and gives
  * each tile a contiguous run of them; each op then starts its descent at the deepest node of the
  * previous op's path that covers its key, and results go back to the caller's positions. UNSORTED
- * runs the ops in the caller's order, each from the root. AUTO takes SORTED when the call is large
- * and dense against the tree (at least 2^16 ops and one op per 128 keys), where neighbouring ops
- * share nodes. Results are the same either way (for a repeated key in one insert call, UNSORTED
- * leaves which value wins unspecified, as the reference does). The sort's scratch (16 bytes per op)
- * comes from a stream-ordered memory pool of the library. No counterpart in the reference. */
+ * runs the ops in the caller's order, each from the root. AUTO takes SORTED for reads of a tree that no
+ * writer changes meanwhile (concurrent = 0) from 2^20 ops on, and for other calls that are large and
+ * dense against the tree (at least 2^16 ops and one op per 128 keys), where neighbouring ops share
+ * nodes. Results are the same either way (for a repeated key in one insert call, UNSORTED leaves which
+ * value wins unspecified, as the reference does). The sort's scratch (16 bytes per op) comes from a
+ * stream-ordered memory pool of the library; reads that AUTO would sort run unsorted without it. No
+ * counterpart in the reference. */
 #define MVBT_FRONTEND_AUTO 0u
 #define MVBT_FRONTEND_UNSORTED 1u
 #define MVBT_FRONTEND_SORTED 2u

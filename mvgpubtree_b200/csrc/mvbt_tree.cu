@@ -169,7 +169,8 @@ __device__ __forceinline__ auto slow_tile() { return cg::tiled_partition<kSlowTi
 // the deepest node of the last keys' path that covers the next ones, and the results go back to the
 // caller's positions (spos). A tile per key spends about 40 instructions of every lane on each of
 // its nodes (issue-bound); here they serve 32 keys. 36 KB of shared memory and 40 registers: six
-// blocks per SM.
+// blocks per SM. Tile kernel / this: 200003 finds in 40M keys 74 / 32 us, 2^20 in 2^20 keys 193 / 90 us
+// unsorted and 130 / 91 sorted; what is left is shared-memory and L1 traffic of the staged nodes.
 constexpr int kReadSortLowBit   = 8;  // reads: order by the top 24 bits (locality is all they need)
 constexpr uint32_t kUnsortedBits = (1u << kReadSortLowBit) - 1u;
 template <bool kSorted>
@@ -217,7 +218,8 @@ __global__ void __launch_bounds__(256) k_find_warp(device_tree T, const uint32_t
 }
 
 // Range queries in a tree no writer changes meanwhile, 32 per warp at a time (mvbt::range_warp);
-// kSorted as in k_find_warp, by lower bound.
+// kSorted as in k_find_warp, by lower bound. Tile kernel / this: 2M queries of 32 pairs in 10M keys 789 /
+// 528 us sorted, 250007 in 40M keys 97 / 89 us unsorted (dependent leaf loads bound both there).
 template <bool kSorted>
 __global__ void __launch_bounds__(256) k_range_warp(device_tree T, const uint32_t* __restrict__ lower,
                                                     const uint32_t* __restrict__ spos,
@@ -446,7 +448,10 @@ __device__ __forceinline__ bool superseded(const uint32_t* skeys, uint64_t i, ui
 }
 
 // Inserts (kErase: erases), 32 per warp at a time (mvbt::write_warp). kSorted: the keys are a sorted
-// call's, with values in the same order, and each warp takes one contiguous run of them.
+// call's, with values in the same order, and each warp takes one contiguous run of them. Bound by the
+// round trips on a leaf (lock, read, copy, two fences), which 32 leaves share. A tile per leaf / this:
+// update of 2^22 keys in 2^25 with both states read back 5.1 / 2.7 ms; inserts, erases and lookups of
+// 300007 keys in a plain tree of 2^20 455 / 201 us.
 template <bool kSorted, bool kErase>
 __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint32_t* __restrict__ keys,
                                                        const uint32_t* __restrict__ values, uint32_t n) {
@@ -546,14 +551,15 @@ int status_from_bits(uint32_t bits) {
   return MVBT_OK;
 }
 
-// Whether range queries likewise are sorted by lower bound first.
+// Whether range queries likewise are sorted by lower bound first (the lookups' line).
 bool sorted_ranges(const mvbt_tree* t, uint32_t n) {
   if (t->frontend == MVBT_FRONTEND_AUTO) return n >= (1u << 20);
   return t->frontend == MVBT_FRONTEND_SORTED && n > 1;
 }
 
 // Fewer lookups than this leave most warps of k_find_warp empty; a tile per key has the shorter
-// chain then.
+// chain then. Tile / warp per call in a tree of 2^20 keys: 4000 lookups 10.7 / 10.7 us (the launch),
+// 16000 11.2 / 10.6, 65536 16.5 / 10.9, 262144 55 / 29.
 constexpr uint32_t kWarpFindMin  = 1u << 13;
 constexpr uint32_t kWarpWriteMin = 1u << 13;  // writes likewise
 
