@@ -613,26 +613,29 @@ bool sorted_lookups(const mvbt_tree* t, uint32_t n) {
 }
 
 
-// A stream-ordered memory pool per device for the sort's scratch and for trees: no device-wide
+// Stream-ordered memory pools per device, one for the sort's scratch and one for trees: no device-wide
 // synchronisation, and freed blocks stay cached in the pool for the next call (up to kPoolKeepBytes).
+// Two, because a pool that holds more than it may keep gives back every freed block at the next
+// synchronisation: with 5.8 GB of trees in the scratch's pool each sorted call mapped its scratch anew
+// (2^25 finds 13 ms instead of 2).
 constexpr int kMaxDevices           = 64;
 constexpr uint64_t kPoolKeepBytes   = 4ull << 30;
-cudaMemPool_t g_sort_pool[kMaxDevices] = {};
-std::mutex g_sort_pool_mu;
+cudaMemPool_t g_pools[2][kMaxDevices] = {};  // scratch, trees
+std::mutex g_pools_mu;
 
-int sort_pool(int dev, cudaMemPool_t* out) {
+int library_pool(int dev, bool trees, cudaMemPool_t* out) {
   if (dev < 0 || dev >= kMaxDevices) return fail(MVBT_ERR_BAD_ARG, "device ordinal out of range");
-  std::lock_guard<std::mutex> lk(g_sort_pool_mu);
-  if (!g_sort_pool[dev]) {
+  std::lock_guard<std::mutex> lk(g_pools_mu);
+  if (!g_pools[trees][dev]) {
     cudaMemPoolProps props = {};
     props.allocType        = cudaMemAllocationTypePinned;
     props.location.type    = cudaMemLocationTypeDevice;
     props.location.id      = dev;
-    MVBT_CUDA_TRY(cudaMemPoolCreate(&g_sort_pool[dev], &props));
+    MVBT_CUDA_TRY(cudaMemPoolCreate(&g_pools[trees][dev], &props));
     uint64_t keep = kPoolKeepBytes;
-    MVBT_CUDA_TRY(cudaMemPoolSetAttribute(g_sort_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+    MVBT_CUDA_TRY(cudaMemPoolSetAttribute(g_pools[trees][dev], cudaMemPoolAttrReleaseThreshold, &keep));
   }
-  *out = g_sort_pool[dev];
+  *out = g_pools[trees][dev];
   return MVBT_OK;
 }
 
@@ -642,14 +645,17 @@ int sort_pool(int dev, cudaMemPool_t* out) {
 constexpr uint64_t kPooledTree = 2ull << 30;
 int tree_alloc(int dev, uint64_t bytes, void** out, bool* pooled) {
   cudaMemPool_t pool;
-  int st = sort_pool(dev, &pool);
+  int st = library_pool(dev, true, &pool);
   if (st) return st;
   *pooled = bytes <= kPooledTree && cudaMallocFromPoolAsync(out, bytes, pool, nullptr) == cudaSuccess;
   if (*pooled) return MVBT_OK;
   cudaGetLastError();
   if (cudaMalloc(out, bytes) == cudaSuccess) return MVBT_OK;
   cudaGetLastError();
-  if (cudaMemPoolTrimTo(pool, 0) == cudaSuccess && cudaMalloc(out, bytes) == cudaSuccess) return MVBT_OK;
+  cudaMemPool_t scratch;
+  if (library_pool(dev, false, &scratch) == MVBT_OK) cudaMemPoolTrimTo(scratch, 0);
+  cudaMemPoolTrimTo(pool, 0);
+  if (cudaMalloc(out, bytes) == cudaSuccess) return MVBT_OK;
   cudaGetLastError();
   return fail(MVBT_ERR_OUT_OF_MEMORY, "cudaMalloc of the node pool failed");
 }
@@ -695,7 +701,7 @@ struct sorted_ops {
 int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaStream_t s, sorted_ops* out,
              const uint32_t* values = nullptr, uint64_t extra_words = 0) {
   cudaMemPool_t pool;
-  int st = sort_pool(t->device, &pool);
+  int st = library_pool(t->device, false, &pool);
   if (st) return st;
   const uint64_t sort_words = 4ull * n + ((mvbt_sort::scratch_words(n) + 63) & ~63ull);
   const uint64_t words      = sort_words + extra_words;
@@ -1074,7 +1080,7 @@ int mvbt_bulk_build(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, 
   if (P.status == 1) return fail(MVBT_ERR_BAD_ARG, "bulk build: tree too tall");
   if (P.status == 2) return fail(MVBT_ERR_POOL_EXHAUSTED, "bulk build: the pool is too small");
   cudaMemPool_t pool;
-  int st = sort_pool(t->device, &pool);
+  int st = library_pool(t->device, false, &pool);
   if (st) return st;
   bulk_plan* dplan = nullptr;
   MVBT_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dplan), sizeof(bulk_plan), pool, s));
