@@ -289,9 +289,11 @@ __global__ void __launch_bounds__(256, kBatchBlocks) k_batched(device_tree T, ba
   auto warp = cg::tiled_partition<32>(cg::this_thread_block());
   auto tile = cg::tiled_partition<W>(warp);
   __shared__ mvbt::batch_gate gate;
+  __shared__ mvbt::held_reads held[kWarpsPerBlock];
   if (threadIdx.x == 0) gate.done = 0, gate.looked = 0;
   __syncthreads();
-  mvbt::batched_worker<W>(T, B, sc, gridDim.x * (blockDim.x >> 5), gate, stage[threadIdx.x >> 5], warp, tile);
+  mvbt::batched_worker<W>(T, B, sc, gridDim.x * (blockDim.x >> 5), gate, held[threadIdx.x >> 5], stage[threadIdx.x >> 5],
+                          warp, tile);
   // the last block to finish closes the run: the epoch after its batches
   __syncthreads();
   if (threadIdx.x == 0) {

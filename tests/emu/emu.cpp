@@ -72,6 +72,8 @@ struct tile_shared {
   std::barrier<> bar;
   uint64_t slot[32];
   fibers* fib = nullptr;  // the lanes are contexts of one thread
+  std::barrier<>* meet = nullptr;  // the other warps, to be met at this tile's meet_at-th shuffle
+  int meet_at = 0, shuffles = 0;
   int width, arrived = 0;
   unsigned generation = 0;
   explicit tile_shared(int w) : bar(w), width(w) {}
@@ -100,6 +102,7 @@ struct emu_tile {
   template <class T>
   T shfl(T v, int src) const {
     sh->slot[rank] = (uint64_t)v;
+    if (rank == 0 && sh->meet && ++sh->shuffles == sh->meet_at) sh->meet->arrive_and_wait();
     sync();
     T r = (T)sh->slot[((src % W) + W) % W];
     sync();
@@ -152,13 +155,16 @@ void run(uint64_t n, int tiles, int W, const std::function<void(uint64_t, const 
   for (auto& x : th) x.join();
 }
 
-// Runs fn(warp, tile) on `warps` emulated warps of 32 threads, each split into tiles of W lanes.
-void run_warps(int warps, int W, const std::function<void(const emu_tile&, const emu_tile&)>& fn) {
+// Runs fn(warp, tile) on `warps` emulated warps of 32 threads, each split into tiles of W lanes. meet_at > 0:
+// no warp goes past its meet_at-th shuffle before all have come to theirs.
+void run_warps(int warps, int W, const std::function<void(const emu_tile&, const emu_tile&)>& fn, int meet_at = 0) {
   if (warps < 1) warps = 1;
   const int tpw = 32 / W;
   std::vector<std::unique_ptr<tile_shared>> wsh, tsh;
+  std::barrier<> meet(warps);
   for (int w = 0; w < warps; ++w) {
     wsh.emplace_back(new tile_shared(32));
+    if (meet_at) wsh.back()->meet = &meet, wsh.back()->meet_at = meet_at;
     for (int j = 0; j < tpw; ++j) tsh.emplace_back(new tile_shared(W));
   }
   std::vector<std::thread> th;
@@ -506,10 +512,12 @@ void emu_find_erase(void* h, const uint32_t* fkeys, uint32_t* out, uint64_t n_fi
 // waits for the writes of batch b - 1); mode 1: one snapshot + one run per batch.
 // reclaim = 1: reclamation inside the persistent run (mvbt_batch_plan_set_reclaim) with external
 // watermark ext; series (nullable) receives 4 values per batch as mvbt_batch_plan_memory_series.
+// together = 1: no warp of a persistent run claims before all have looked at the queues (three shuffles), as
+// the warps of a block that start together nearly do.
 void emu_batch_run(void* h, uint32_t nb, const uint64_t* off, const uint32_t* type, const uint32_t* key,
                    const uint32_t* arg, const uint64_t* out_off, const uint32_t* cap, uint32_t* result,
                    uint32_t* range_out, int mode, int tiles, int W, int reclaim, uint32_t ext,
-                   uint64_t* series) {
+                   uint64_t* series, int together) {
   auto* t = static_cast<emu_tree*>(h);
   auto v  = t->view();
   mvbt::batch_view B{type, key, arg, out_off, cap, result, reinterpret_cast<uint2*>(range_out)};
@@ -557,9 +565,10 @@ void emu_batch_run(void* h, uint32_t nb, const uint64_t* off, const uint32_t* ty
   const int warps = std::max(1, tiles * W / 32);
   std::vector<mvbt::write_stage> stage(warps);
   mvbt::batch_gate gate{0, 0};  // the warps as one block
+  std::vector<mvbt::held_reads> held(warps);
   EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {
-    mvbt::batched_worker<kW>(v, B, sc, (uint32_t)warps, gate, stage[mvbt::emu::sm], warp, tile);
-  }));
+    mvbt::batched_worker<kW>(v, B, sc, (uint32_t)warps, gate, held[mvbt::emu::sm], stage[mvbt::emu::sm], warp, tile);
+  }, together ? 3 : 0));
   t->ctl.epoch = params[1] + nb;
   if (series && sc.series) std::memcpy(series, ser.data(), ser.size() * sizeof(uint64_t));
 }

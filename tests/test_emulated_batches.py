@@ -1,0 +1,38 @@
+"""CPU tier: the persistent batch worker (mvbt::batched_worker) on lists and launch shapes where its claims, waits
+and reclamation can go wrong, run by the emulator against the oracle."""
+import numpy as np
+import pytest
+
+
+def _list(ops):
+    """workload.Batches of ops: per batch a list of (type, key, value or upper bound, range capacity)."""
+    import workload as wl
+    flat = [o for b in ops for o in b]
+    off = np.cumsum([0] + [len(b) for b in ops]).astype(np.uint64)
+    col = lambda j, t: np.ascontiguousarray(np.array([o[j] for o in flat] or [0]).astype(t))
+    cap = col(3, np.uint32)
+    ends = np.cumsum(cap.astype(np.uint64))
+    return wl.Batches(off, col(0, np.uint32), col(1, np.uint32), col(2, np.uint32), ends - cap, cap, int(ends[-1]))
+
+
+def _insert(k, v): return (1, k, v, 0)
+def _find(k): return (0, k, 0, 0)
+
+
+def _same_as_oracle(t, m, b, **how):
+    got, pairs = t.run_batches(b, **how)
+    want, want_pairs = m.run_batches(b)
+    assert t.errors == 0, t.stats()
+    n = b.num_ops
+    assert np.array_equal(got[:n], want[:n]) and np.array_equal(pairs[: want_pairs.size], want_pairs)
+
+
+@pytest.mark.parametrize("warps,lead", [(1, 2), (2, 2), (3, 3), (4, 2), (8, 2)])
+def test_reads_claimed_far_ahead_leave_warps_for_the_writes(warps, lead):
+    """The first `lead` batches hold no write, so every warp takes reads first: one claim of them reaches over many
+    batches, and each warp's claims need writes that no warp has taken yet."""
+    from emu import EmuTree
+    import oracle
+    t, m = EmuTree(True, capacity=1 << 13, tiles=4 * warps, W=8), oracle.MVMap(True)
+    ops = [[_find(10 * b)] if b < lead else [_insert(10 * b + 10, b + 1), _find(10 * b)] for b in range(200)]
+    _same_as_oracle(t, m, _list(ops), together=True)

@@ -66,6 +66,39 @@ def test_batch_lists_at_the_edges_match_oracle(mode, case, nb, one_warp):
     assert t.take_snapshot() == m.take_snapshot()
 
 
+@pytest.mark.parametrize("mode", [0, "noalloc"])
+@pytest.mark.parametrize("block", [64, 96, 128, 256])
+def test_late_writes_in_one_block_match_oracle(mode, block):
+    """2, 3, 4 and 8 warps in all and a list whose first batches only read: the first claims of the warps are
+    reads that reach over many batches, and wait for writes that are not claimed yet."""
+    import torch
+    import mvgpubtree_b200 as mv
+    import oracle
+    import workload as wl
+    n0, nb = 3000, 200
+    init = wl.distinct_keys(9, 0, n0)
+    t = mv.gpu_versioned_btree(pool_bytes=1 << 28, block_size=block, max_blocks=1)
+    m = oracle.MVMap(True)
+    t.insert(_dev(init), _dev(wl.values_for(init, 0)))
+    m.insert(init, wl.values_for(init, 0))
+    gen = wl.MixGenerator(9, n0, stride=wl.stride_for(n0), fixed_batch=4)
+    b = gen.generate(nb)
+    batch = np.repeat(np.arange(nb), np.diff(b.batch_off.astype(np.int64)))
+    c = _keep(b, ~((b.type == 1) | (b.type == 2)) | (batch >= 3))
+    n = int(c.batch_off[-1])
+    result = torch.zeros(n, dtype=torch.int32, device="cuda")
+    pairs = torch.full((max(1, int(b.range_pairs)) * 2,), -1, dtype=torch.int32, device="cuda")
+    ops = [_dev(x) for x in (c.type, c.key, c.arg, c.out_off, c.range_cap)]
+    if mode == "noalloc":
+        t.batch_run_noalloc(_dev(c.batch_off), n, *ops, result, pairs)
+    else:
+        t.batch_plan(n, nb).run(c.batch_off, *ops, result, pairs, mode=mode)
+    assert t.check_errors() == 0
+    want, want_pairs = m.run_batches(c)
+    assert np.array_equal(_host(result), want)
+    assert np.array_equal(_host(pairs), want_pairs)
+
+
 @pytest.mark.parametrize("n", [4096, 4097, 10239, 10240, 10241])
 def test_loads_at_tile_edges_keep_the_last_of_each_key(n):
     import torch
