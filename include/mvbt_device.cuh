@@ -110,6 +110,7 @@ inline T atomicMax(T* p, U v) {
 namespace mvbt {
 namespace emu {
 inline thread_local uint32_t sm = 0;  // emulated SM id of the calling lane
+inline std::atomic<uint32_t> slow{1};      // global_ns runs this much slower than the host's clock
 }
 }  // namespace mvbt
 #else
@@ -313,7 +314,7 @@ MVBT_DEV uint32_t tile_ordinal(const Tile&) { return emu::sm; }
 MVBT_DEV unsigned long long global_ns() {
   return (unsigned long long)std::chrono::duration_cast<std::chrono::nanoseconds>(
              std::chrono::steady_clock::now().time_since_epoch())
-      .count();
+      .count() / emu::slow.load(std::memory_order_relaxed);
 }
 MVBT_DEV uint32_t ld_relaxed_u32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
 MVBT_DEV uint32_t ld_block_u32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
@@ -2431,7 +2432,7 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
   const uint32_t erases     = warp.ballot(erase);
   uint32_t tries = 0, backoff = 32;
   unsigned long long t0     = 0;
-  for (uint32_t step = 0; step < kMaxSteps; ++step) {
+  for (uint32_t step = 0; step < kMaxSteps;) {
     if (pend && leaf >= T.capacity) {
       T.set_error(kErrCorrupt, 1);
       pend = false;
@@ -2446,16 +2447,21 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
     bool locked         = false;
     if (lead) locked = !(atomicOr(mod, kLockBit) & kLockBit);
     const uint32_t okm = warp.ballot(locked);
-    if (okm == 0) {
+    if (okm == 0) {  // all held elsewhere: as device_tree::lock, bounded by the clock and the attempts alone
       if (tries == 0) t0 = global_ns();
       if (++tries >= T.ctl->spin_limit || wait_expired(t0, T.ctl->wait_ns, warp)) {
         if (lead) T.set_error(kErrSpinLimit, 2);
         return;
       }
-      __nanosleep(backoff);
-      backoff = backoff < 1024 ? backoff * 2 : 1024;
+      // wait until one looks free before the next atomics
+      for (uint32_t w = 0; w < 64; ++w) {
+        __nanosleep(backoff);
+        if (warp.ballot(lead && !(ld_relaxed_u32(mod) & kLockBit))) break;
+        backoff = backoff < 1024 ? backoff * 2 : 1024;
+      }
       continue;
     }
+    ++step;
     tries   = 0;
     backoff = 32;
     __threadfence();

@@ -24,6 +24,8 @@ def lib():
             "emu_errors": (u32, [vp]),
             "emu_bump": (u32, [vp]),
             "emu_snapshot": (u32, [vp]),
+            "emu_hold_first_leaf": (None, [vp, i]),
+            "emu_slow_clock": (None, [u32]),
             "emu_insert": (None, [vp, u32p, u32p, u64, i, i]),
             "emu_erase": (None, [vp, u32p, u64, i, i]),
             "emu_find": (None, [vp, u32p, u32p, u64, u32, i, i, i]),
@@ -87,6 +89,10 @@ class EmuTree:
 
     def snapshot(self) -> int:
         return int(self.L.emu_snapshot(self.h))
+
+    def hold_first_leaf(self, on: bool):
+        """Locks or releases the first leaf from outside the operations."""
+        self.L.emu_hold_first_leaf(self.h, int(on))
 
     def insert(self, k, v):
         k, v = _u32(k), _u32(v)

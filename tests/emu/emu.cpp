@@ -254,6 +254,17 @@ void emu_stats(void* h, uint64_t* out) {
   out[25] = c.stat_log_dropped;
 }
 
+// Locks (on != 0) or releases the first leaf from outside, as a writer that holds it for long would.
+void emu_hold_first_leaf(void* h, int on) {
+  uint32_t* mod = &static_cast<emu_tree*>(h)->pool[32 * mvbt::kFirstLeaf + mvbt::kModWord];
+  if (on) __atomic_fetch_or(mod, mvbt::kLockBit, __ATOMIC_SEQ_CST);
+  else __atomic_fetch_and(mod, ~mvbt::kLockBit, __ATOMIC_SEQ_CST);
+}
+
+// Lets the emulated clock run `by` times slower: a wait then looks about as often as on the GPU before its
+// limit has passed.
+void emu_slow_clock(uint32_t by) { mvbt::emu::slow.store(by ? by : 1u); }
+
 uint32_t emu_snapshot(void* h) {
   auto* t = static_cast<emu_tree*>(h);
   return __atomic_fetch_add(&t->ctl.epoch, 1u, __ATOMIC_SEQ_CST);

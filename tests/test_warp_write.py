@@ -44,3 +44,29 @@ def test_emulated_warp_writes_match_oracle(w, versioned, reclaim, chunk, sorted_
     rep = t.validate()
     assert rep["violations"] == 0 and rep["locked_nodes"] == 0
     assert t.stats()["splits"] > 20
+
+
+def test_warp_writes_wait_for_a_lock_by_the_clock():
+    """A leaf that stays locked for long, but not past the wait limit, delays the warp's writes and loses none,
+    however often they look at it meanwhile; one that stays locked past the limit (4 s in the emulator) is given
+    up as a wait, not as a broken structure."""
+    import threading
+    from emu import EmuTree
+    keys = np.arange(1, 9, dtype=np.uint32)
+    t = EmuTree(False, capacity=1 << 10, chunk=64)
+    t.hold_first_leaf(True)
+    t.L.emu_slow_clock(64)
+    timer = threading.Timer(8, t.hold_first_leaf, (False,))
+    timer.start()
+    try:
+        t.write_warp(np.ones(8), keys, keys, warps=1)
+    finally:
+        t.L.emu_slow_clock(1)
+        timer.join()
+    assert t.errors == 0, t.stats()
+    assert np.array_equal(t.find(keys), keys)
+    t.hold_first_leaf(True)
+    t.write_warp(np.ones(8), keys, keys + 1, warps=1)
+    assert t.errors == 2, t.stats()
+    t.hold_first_leaf(False)
+    assert np.array_equal(t.find(keys), keys)
