@@ -196,7 +196,8 @@ struct control_block {
   unsigned long long stat_restarts;   // locked approaches abandoned for an unlocked re-approach
   uint32_t err_site[32];              // errors per raising site (diagnostics; 16 = the
                                       // offsets check of mvbt_batch_run_noalloc, 17 = a
-                                      // bulk load that did not fit the pool)
+                                      // bulk load that did not fit the pool, 18 / 19 = a free-ring
+                                      // slot that stayed empty / unread)
   unsigned long long sm_pool[kMaxSmSlots];  // per-SM chunk cursor: (base << 32) | used
   // Reclamation of version copies (off when reclaim_cap == 0). The retire log holds the index of
   // every copy not yet reclaimed, in the order the copies were made (which is epoch order); the
@@ -790,11 +791,12 @@ MVBT_DEV bool take_free_chunk(control_block* c, uint32_t C, uint32_t& base) {
 // and the rest of per-SM chunks taken from the ring) never fill the ring, so a pusher meets a
 // slot of the previous lap only while its reader is about to clear it -- or while it is the unread
 // rest of the chunk of an SM that has stopped allocating, which flush_chunk returns in time.
-// kCount: the nodes were freed just now (stat_reclaimed).
+// kCount: the nodes were freed just now (stat_reclaimed). Returns whether the push went past one of the
+// positions, 16 to a lap, where the chunks are looked over (return_idle_chunks).
 template <bool kCount = true, class Warp>
-MVBT_DEV void ring_push(control_block* c, bool freed, uint32_t node, const Warp& warp) {
+MVBT_DEV bool ring_push(control_block* c, bool freed, uint32_t node, const Warp& warp) {
   const uint32_t m = warp.ballot(freed);
-  if (!m) return;
+  if (!m) return false;
   const uint32_t lane = warp.thread_rank();
   const int lead      = __ffs(m) - 1;
   unsigned long long base = 0;
@@ -804,7 +806,14 @@ MVBT_DEV void ring_push(control_block* c, bool freed, uint32_t node, const Warp&
     uint32_t* slot = reinterpret_cast<uint32_t*>(c->free_ring) +
                      ((base + __popc(m & ((1u << lane) - 1u))) & (c->ring_cap - 1u));
     const unsigned long long t0 = global_ns();
-    while (ld_relaxed_u32(slot) != kRingEmpty && global_ns() - t0 <= c->wait_ns) __nanosleep(64);
+    while (ld_relaxed_u32(slot) != kRingEmpty) {
+      if (global_ns() - t0 > c->wait_ns) {
+        atomicOr(&c->error, kErrSpinLimit);
+        atomicAdd(&c->err_site[19], 1u);
+        break;
+      }
+      __nanosleep(64);
+    }
     st_relaxed_u32(slot, node);
   }
   __threadfence();
@@ -813,13 +822,16 @@ MVBT_DEV void ring_push(control_block* c, bool freed, uint32_t node, const Warp&
     atomicAdd(&c->free_avail, (unsigned long long)__popc(m));
     if (kCount) atomicAdd(&c->stat_reclaimed, (unsigned long long)__popc(m));
   }
+  const uint32_t pos = (uint32_t)base & (c->ring_cap - 1u), part = c->ring_cap / 16;
+  return pos / part != (pos + (uint32_t)__popc(m)) / part;
 }
 // Returns the unread rest of SM slot `sm`'s chunk to the free ring if the chunk is a run of ring
 // positions that lies `behind` or more positions behind the ring's tail (warp-collective). Without it
 // an SM that took a chunk and then stopped allocating would keep its positions unread until the ring's
 // tail comes round, and the pushers that meet them would wait out their limit.
+// Returns what ring_push did.
 template <class Warp>
-MVBT_DEV void flush_chunk(control_block* c, uint32_t sm, uint32_t behind, const Warp& warp) {
+MVBT_DEV bool flush_chunk(control_block* c, uint32_t sm, uint32_t behind, const Warp& warp) {
   unsigned long long* slot = &c->sm_pool[sm];
   const uint32_t C         = c->chunk;
   unsigned long long cur   = 0;
@@ -834,9 +846,10 @@ MVBT_DEV void flush_chunk(control_block* c, uint32_t sm, uint32_t behind, const 
       take = C - used;
   }
   take = warp.shfl(take, 0);
-  if (take == 0) return;
+  if (take == 0) return false;
   cur = warp.shfl(cur, 0);
   const uint32_t base = (uint32_t)(cur >> 32), used = (uint32_t)cur;
+  bool past           = false;
   for (uint32_t j = 0; j < take; j += 32) {  // read (and clear) before pushing: no pusher waits for this warp
     const uint32_t at = j + warp.thread_rank();
     uint32_t node     = kNone;
@@ -844,18 +857,30 @@ MVBT_DEV void flush_chunk(control_block* c, uint32_t sm, uint32_t behind, const 
       node = chunk_node(c, base, used + at);
       atomicAdd(&c->sm_stats[sm_id() % kMaxSmSlots][2], (unsigned long long)-1ll);  // not handed out after all
     }
-    ring_push<false>(c, node != kNone, node, warp);
+    past |= ring_push<false>(c, node != kNone, node, warp);
   }
+  return past;
 }
 // flush_chunk of all SM slots: warp w looks at slots [32 w, 32 w + 32), a lane at each.
 template <class Warp>
-MVBT_DEV void flush_chunks(control_block* c, uint32_t w, uint32_t behind, const Warp& warp) {
-  if (w >= (uint32_t)kMaxSmSlots / 32) return;
+MVBT_DEV bool flush_chunks(control_block* c, uint32_t w, uint32_t behind, const Warp& warp) {
+  if (w >= (uint32_t)kMaxSmSlots / 32) return false;
+  bool past = false;
   const unsigned long long cur = ld_relaxed_u64(&c->sm_pool[32 * w + warp.thread_rank()]);
   const uint32_t base = (uint32_t)(cur >> 32);
   const uint32_t lag  = ((uint32_t)ld_relaxed_u64(&c->free_tail) - (base & ~kRingChunk)) & (c->ring_cap - 1u);
   for (uint32_t m = warp.ballot((base & kRingChunk) && (uint32_t)cur < c->chunk && lag >= behind); m; m &= m - 1u)
-    flush_chunk(c, 32 * w + (uint32_t)__ffs(m) - 1u, behind, warp);
+    past |= flush_chunk(c, 32 * w + (uint32_t)__ffs(m) - 1u, behind, warp);
+  return past;
+}
+// After a push that went past one of the ring's 16 marks: returns the unread rests of all chunks half a lap
+// behind. Whichever SMs run or stand still, a chunk goes back 7/16 of a lap before the tail comes round to it.
+template <class Warp>
+MVBT_CALL void return_idle_chunks(control_block* c, Warp warp) {
+  for (bool past = true; past;) {  // the rests that it pushes may pass the next mark
+    past = false;
+    for (uint32_t w = 0; w < (uint32_t)kMaxSmSlots / 32; ++w) past |= flush_chunks(c, w, c->ring_cap / 2, warp);
+  }
 }
 // Records a version copy in the retire log. A copy the full log cannot take is never freed
 // (counted in stat_log_dropped).
@@ -1144,12 +1169,14 @@ struct device_tree {
     n = warp.shfl(n, 0);
     if (n == 0) return 0;
     __threadfence();  // the copies' last readers finished before `limit` was published
+    bool past = false;
     for (uint32_t j = 0; j < n; j += 32) {
       const uint32_t at = j + warp.thread_rank();
       uint32_t idx      = kNone;
       const bool freed  = at < n && reclaim_entry(h + at, 0, idx, false) == 1;
-      ring_push(c, freed, idx, warp);
+      past |= ring_push(c, freed, idx, warp);
     }
+    if (past) return_idle_chunks(c, warp);
     return n;
   }
 
@@ -2794,8 +2821,7 @@ MVBT_DEV uint32_t wait_batch_ready(const device_tree& T, const batch_sched& sc, 
 }
 
 // One step of reclamation inside the launch (warp-collective): advances full_done, then frees up to
-// kReclaimClaim copies below rc_limit; now and then (or with none to free) it returns this SM's chunk if the ring's tail
-// is about to come round to it. Returns true if it claimed any log position.
+// kReclaimClaim copies below rc_limit. Returns true if it claimed any log position.
 template <class Warp>
 MVBT_DEV bool reclaim_step(const device_tree& T, const batch_sched& sc, uint32_t nb, const Warp& warp) {
   unsigned long long lim = 0;
@@ -2804,9 +2830,7 @@ MVBT_DEV bool reclaim_step(const device_tree& T, const batch_sched& sc, uint32_t
     lim = ld_relaxed_u64(sc.rc_limit);
   }
   lim = warp.shfl(lim, 0);
-  const uint32_t n = T.reclaim_online(lim, warp);
-  if (n == 0 || (lim & 7u) == 0) flush_chunk(T.ctl, sm_id() % kMaxSmSlots, T.ctl->ring_cap - T.ctl->ring_cap / 8, warp);
-  return n > 0;
+  return T.reclaim_online(lim, warp) > 0;
 }
 // At the end of a warp's work: one more reclamation step, then leave. The
 // copies the last batches made become reclaimable only when their last reads finish, at the very

@@ -574,6 +574,10 @@ void emu_batch_run(void* h, uint32_t nb, const uint64_t* off, const uint32_t* ty
     sc.series     = ser.data();
   }
   const int warps = std::max(1, tiles * W / 32);
+  if (sc.rc_limit)  // as k_count_ops
+    run_warps(mvbt::kMaxSmSlots / 32, 8, [&](const emu_tile& warp, const emu_tile&) {
+      mvbt::flush_chunks(&t->ctl, mvbt::emu::sm, t->ctl.ring_cap / 2, warp);
+    });
   std::vector<mvbt::write_stage> stage(warps);
   mvbt::batch_gate gate{0, 0};  // the warps as one block
   std::vector<mvbt::held_reads> held(warps);

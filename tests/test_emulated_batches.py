@@ -36,3 +36,30 @@ def test_reads_claimed_far_ahead_leave_warps_for_the_writes(warps, lead):
     t, m = EmuTree(True, capacity=1 << 13, tiles=4 * warps, W=8), oracle.MVMap(True)
     ops = [[_find(10 * b)] if b < lead else [_insert(10 * b + 10, b + 1), _find(10 * b)] for b in range(200)]
     _same_as_oracle(t, m, _list(ops), together=True)
+
+
+def _updates(keys, batches, per, reads=0, read_only=0):
+    """`batches` batches of `per` updates of `keys` and `reads` lookups, then `read_only` ones that hold as many
+    lookups as there were updates, and one more each."""
+    rng = np.random.default_rng(5)
+    out = [[_insert(int(k), b + 1) for k in rng.permutation(keys)[:per]] + [_find(int(k)) for k in rng.choice(keys, reads)]
+           for b in range(batches)]
+    return _list(out + [[_find(int(k)) for k in rng.choice(keys, batches * per // max(read_only, 1) + 1)] for _ in range(read_only)])
+
+
+def test_chunks_of_idle_sms_go_back_before_the_ring_comes_round():
+    """SMs that take a chunk from the free ring and then run nothing: a later run on fewer warps pushes more than a
+    lap of the ring past the unread rest of their chunks."""
+    from emu import EmuTree
+    import oracle
+    t, m = EmuTree(True, capacity=1 << 12, tiles=32, W=8, reclaim=True), oracle.MVMap(True)
+    keys = np.arange(10, 12010, 10, dtype=np.uint32)
+    t.insert(keys, keys)
+    m.insert(keys, keys)
+    for _ in range(3):  # 8 warps, an SM each: their chunks come from the ring
+        _same_as_oracle(t, m, _updates(keys, 12, 150, 5), reclaim=True)
+    assert t.stats()["reused"] > 0
+    t.tiles = 4  # one warp
+    before = t.stats()["reclaimed"]
+    _same_as_oracle(t, m, _updates(keys, 110, 150), reclaim=True)
+    assert t.stats()["reclaimed"] - before > 8192  # more than the ring holds
