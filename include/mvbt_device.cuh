@@ -2998,9 +2998,13 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
       }
       if (lane == 0 && resume && !hold) held.lanes = 0;
       // Reclamation keeps pace with copying even when no warp is ever idle: a step after each claim of
-      // reads, which nothing waits for, and after each claim of writes only where those outnumber the
-      // reads (the next batch waits for them).
-      if (did && sc.rc_limit && (reads || TW > TR)) reclaim_step(T, sc, nb, warp);
+      // reads, which nothing waits for, and after a claim of writes only if their batch has more of them
+      // than reads (the next batch waits for them). A step takes 64 copies, two for each op of a full claim, so
+      // either kind keeps up with the copies of its batch.
+      if (did && sc.rc_limit) {
+        const bool more = has && writes && 2ull * sc.n_writes[b] > sc.batch_off[b + 1] - sc.batch_off[b];
+        if (warp.ballot(reads || more)) reclaim_step(T, sc, nb, warp);
+      }
     }
     if (did) {
       spin       = 0;

@@ -63,3 +63,18 @@ def test_chunks_of_idle_sms_go_back_before_the_ring_comes_round():
     before = t.stats()["reclaimed"]
     _same_as_oracle(t, m, _updates(keys, 110, 150), reclaim=True)
     assert t.stats()["reclaimed"] - before > 8192  # more than the ring holds
+
+
+def test_reclamation_keeps_pace_in_batches_that_only_write():
+    """Write-only batches in a list that reads more than it writes elsewhere: their copies are reclaimed while they
+    run, so a pool far smaller than the copies of the whole list suffices."""
+    from emu import EmuTree
+    import oracle
+    t, m = EmuTree(True, capacity=1 << 12, tiles=8, W=8, reclaim=True), oracle.MVMap(True)
+    keys = np.arange(10, 12010, 10, dtype=np.uint32)
+    t.insert(keys, keys)
+    m.insert(keys, keys)
+    b = _updates(keys, 60, 150, read_only=10)
+    assert np.count_nonzero(b.type == 1) < np.count_nonzero(b.type == 0)
+    _same_as_oracle(t, m, b, reclaim=True)
+    assert t.stats()["cow"] > 4096  # more copies than the pool has nodes
