@@ -2901,6 +2901,7 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
   const uint32_t lane = warp.thread_rank();
   const uint32_t nb   = ld_relaxed_u32(sc.params + 0);
   const uint32_t S0   = ld_relaxed_u32(sc.params + 1);
+  if (nb == 0) return;  // an empty list, or one whose offsets were rejected
   const uint64_t TW = sc.wpre[nb], TR = sc.rpre[nb];
   const uint32_t wclaim = claim_size(TW, (uint64_t)nb * kWriteClaims, kTiles);
   const uint32_t rclaim = claim_size(TR, (uint64_t)warps * kReadClaims, kTiles);

@@ -78,3 +78,11 @@ def test_reclamation_keeps_pace_in_batches_that_only_write():
     assert np.count_nonzero(b.type == 1) < np.count_nonzero(b.type == 0)
     _same_as_oracle(t, m, b, reclaim=True)
     assert t.stats()["cow"] > 4096  # more copies than the pool has nodes
+
+
+def test_an_empty_list_of_batches_runs_nothing():
+    from emu import EmuTree
+    import oracle
+    t, m = EmuTree(True, capacity=1 << 10), oracle.MVMap(True)
+    _same_as_oracle(t, m, _list([]))
+    assert t.snapshot() == 0
