@@ -2795,6 +2795,7 @@ MVBT_DEV uint32_t wait_batch_ready(const device_tree& T, const batch_sched& sc, 
         if (now - last >= kPollNs && atomicCAS(&gate.looked, last, now) == last) {
           if (w % kAdvanceEvery == kAdvanceEvery - 1) advance_done(sc, nb, T.ctl);
           d = ld_relaxed_u32(sc.done_batches);
+          __threadfence();  // the writes counted in d come before the word that the other warps see
           atomicMax(&gate.done, d);
         }
       }
