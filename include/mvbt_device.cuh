@@ -2249,6 +2249,7 @@ MVBT_DEV uint32_t range_warp(const device_tree& T, uint32_t lo, uint32_t hi, boo
 struct write_stage : warp_stage {
   uint32_t op[32][2];  // each lane's {key, value}; once tried, whether its leaf was full in place of the key
   uint32_t dst[32];    // where each staged node is stored (kNone: nowhere)
+  uint32_t parent[32]; // the level-1 node that named each lane's leaf (kNone: not seen)
 };
 
 // The stages of a block's warps follow one another in shared memory, and their staged nodes start on 128-byte
@@ -2257,11 +2258,13 @@ struct write_stage : warp_stage {
 static_assert(sizeof(write_stage) % 128 == 0, "staged nodes start on 128-byte boundaries");
 
 // The leaf that each live lane's key belongs to, unread: the child its level-1 node names (kNone:
-// failed). Routing at the newest state while writers run, as descend_for_write.
+// failed), and that node (st.parent), where a split of the leaf puts its separator. Routing at the newest
+// state while writers run, as descend_for_write.
 template <class Warp>
 MVBT_DEV uint32_t leaf_warp(const device_tree& T, uint32_t key, bool live, uint32_t start, warp_path* path,
-                            warp_stage& st, const Warp& warp) {
+                            write_stage& st, const Warp& warp) {
   const uint32_t lane = warp.thread_rank();
+  st.parent[lane]     = kNone;
   uint32_t leaf       = kNone;
   uint32_t idx        = start;
   const uint32_t all  = warp.ballot(live);
@@ -2290,7 +2293,8 @@ MVBT_DEV uint32_t leaf_warp(const device_tree& T, uint32_t key, bool live, uint3
       } else {
         if (last) path->record(level, idx, low, high);
         const uint32_t c = count_up_to(st, slot, key);
-        idx              = c ? st.word(slot, 2 * c - 1) : kAnchor;
+        if (c && level == 1) st.parent[lane] = idx;
+        idx = c ? st.word(slot, 2 * c - 1) : kAnchor;
         if (c && level == 1) {
           leaf = idx;
           live = false;
@@ -2432,11 +2436,12 @@ MVBT_DEV void for_lanes(uint32_t m, const Warp& warp, const F& f) {
   }
 }
 
-// One write by a tile, from the leaf where its warp found it.
+// One write by a tile, from the leaf where its warp found it, under its level-1 node `parent` (kNone: unknown).
 template <int W, class Tile>
-MVBT_CALL void write_tile(device_tree T, uint32_t key, uint32_t value, bool erase, uint32_t E, uint32_t leaf, Tile tile) {
+MVBT_CALL void write_tile(device_tree T, uint32_t key, uint32_t value, bool erase, uint32_t E, uint32_t leaf,
+                          uint32_t parent, Tile tile) {
   if (erase) T.erase_at<W>(key, tile, E, leaf);
-  else T.insert_at<W>(key, value, tile, E, leaf, kNone, kNone, 0u);
+  else T.insert_at<W>(key, value, tile, E, leaf, parent, kNone, 1u);  // path0 holds level 1 in its lane 1
 }
 
 // Runs the live lanes' inserts (key -> value) and erases in write epoch E. The warp locks the leaves
@@ -2447,7 +2452,8 @@ MVBT_CALL void write_tile(device_tree T, uint32_t key, uint32_t value, bool eras
 // leaf stored, release. No lane waits for a lock while the warp holds one: leaves found locked are
 // tried again after the others are released. A leaf without room for a new key is split by the tile
 // path (one key per leaf at a time), and the leaf's other keys go on from there.
-// leaf: each live lane's leaf as leaf_warp found it, possibly stale (kNone: the op is given up). Two
+// leaf: each live lane's leaf as leaf_warp found it (which also left its parent in st.parent), possibly stale
+// (kNone: the op is given up). Two
 // live lanes may hold one key only if either order will do.
 template <int W, class Warp, class Tile>
 MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, bool erase, bool live, uint32_t E,
@@ -2594,7 +2600,7 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
       const bool run     = m != 0;  // the same in every lane of a tile
       const int src      = run ? __ffs(m) - 1 : 0;
       const uint32_t k   = warp.shfl(key, src), v = warp.shfl(value, src), to = warp.shfl(leaf, src);
-      if (run) write_tile<W>(T, k, v, (erases >> src) & 1u, E, to, tile);
+      if (run) write_tile<W>(T, k, v, (erases >> src) & 1u, E, to, st.parent[src], tile);
       for (uint32_t q = 0; q < kTiles; ++q) left &= left - 1u;
       warp.sync();
     }

@@ -348,7 +348,7 @@ void emu_range_warp(void* h, const uint32_t* lo, const uint32_t* hi, const uint3
   auto v  = t->view();
   if (!v.versioned) ts = mvbt::kLatest;
   const uint64_t groups = (n + 31) / 32, per = (groups + warps - 1) / warps;
-  std::vector<mvbt::warp_stage> stage(warps);
+  std::vector<mvbt::write_stage> stage(warps);
   std::vector<mvbt::warp_path> path(warps);
   run_warps(warps, 8, [&](const emu_tile& warp, const emu_tile&) {
     const uint64_t w = mvbt::emu::sm;
