@@ -80,6 +80,7 @@ inline int __popc(uint32_t x) { return __builtin_popcount(x); }
 inline int __ffs(uint32_t x) { return __builtin_ffs((int)x); }
 inline int __clz(uint32_t x) { return x ? __builtin_clz(x) : 32; }
 inline void __threadfence() { std::atomic_thread_fence(std::memory_order_seq_cst); }
+inline void __threadfence_block() { std::atomic_thread_fence(std::memory_order_seq_cst); }
 inline void __nanosleep(unsigned) { std::this_thread::yield(); }
 template <class T, class U>
 inline T atomicOr(T* p, U v) { return __atomic_fetch_or(p, (T)v, __ATOMIC_SEQ_CST); }
@@ -318,6 +319,7 @@ MVBT_DEV unsigned long long global_ns() {
       .count() / emu::slow.load(std::memory_order_relaxed);
 }
 MVBT_DEV uint32_t ld_relaxed_u32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
+MVBT_DEV uint32_t ld_acquire_u32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_ACQUIRE); }
 MVBT_DEV uint32_t ld_block_u32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
 MVBT_DEV void st_relaxed_u32(uint32_t* p, uint32_t v) { __atomic_store_n(p, v, __ATOMIC_RELAXED); }
 MVBT_DEV unsigned long long ld_relaxed_u64(const unsigned long long* p) {
@@ -371,6 +373,12 @@ MVBT_DEV uint32_t ld_relaxed_u32(const uint32_t* p) {
 MVBT_DEV unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long r;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(r) : "l"(p) : "memory");
+  return r;
+}
+// An acquire load: what this thread does next comes after the writes that the read value stands for.
+MVBT_DEV uint32_t ld_acquire_u32(const uint32_t* p) {
+  uint32_t r;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(r) : "l"(p) : "memory");
   return r;
 }
 // A word of shared memory that other warps of the block change.
@@ -2800,8 +2808,8 @@ MVBT_DEV uint32_t wait_batch_ready(const device_tree& T, const batch_sched& sc, 
         const uint32_t now = (uint32_t)global_ns(), last = ld_block_u32(&gate.looked);
         if (now - last >= kPollNs && atomicCAS(&gate.looked, last, now) == last) {
           if (w % kAdvanceEvery == kAdvanceEvery - 1) advance_done(sc, nb, T.ctl);
-          d = ld_relaxed_u32(sc.done_batches);
-          __threadfence();  // the writes counted in d come before the word that the other warps see
+          d = ld_acquire_u32(sc.done_batches);  // the writes counted in d come before it, and
+          __threadfence_block();                // before the word that the other warps see
           atomicMax(&gate.done, d);
         }
       }
