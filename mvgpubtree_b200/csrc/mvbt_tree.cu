@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(256, 4) k_write_warp(device_tree T, const uint
       start = path->start(__shfl_sync(0xffffffffu, k, 0), __shfl_sync(0xffffffffu, k, 31 - __clz(m)), warp);
     }
     const uint32_t leaf = mvbt::leaf_warp(T, k, live && k != mvbt::kEmptyKey, start, path, st, warp);
-    mvbt::write_warp<kSlowTile>(T, k, v, kErase, live, E, leaf, st, warp, slow_tile());
+    mvbt::write_warp<kSlowTile, kSorted && !kErase>(T, k, v, kErase, live, E, leaf, st, warp, slow_tile());
   }
 }
 

@@ -406,7 +406,9 @@ void emu_write_warp(void* h, const uint32_t* kind, const uint32_t* keys, const u
         start = path[w].start(warp.shfl(k, 0), warp.shfl(k, 31 - __clz(m)), warp);
       }
       const uint32_t leaf = mvbt::leaf_warp(v, k, live && k != mvbt::kEmptyKey, start, sorted ? &path[w] : nullptr, st, warp);
-      mvbt::write_warp<kW>(v, k, has ? vals[i] : 0u, has && kind[i] == 2, live, E, leaf, st, warp, tile);
+      const uint32_t val = has ? vals[i] : 0u;
+      if (sorted) mvbt::write_warp<kW, true>(v, k, val, has && kind[i] == 2, live, E, leaf, st, warp, tile);
+      else mvbt::write_warp<kW>(v, k, val, has && kind[i] == 2, live, E, leaf, st, warp, tile);
     }
   }));
 }

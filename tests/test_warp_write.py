@@ -70,3 +70,75 @@ def test_warp_writes_wait_for_a_lock_by_the_clock():
     assert t.errors == 2, t.stats()
     t.hold_first_leaf(False)
     assert np.array_equal(t.find(keys), keys)
+
+
+@pytest.mark.parametrize("w,versioned,every,warps", [(8, False, 1, 1), (8, True, 1, 3), (16, True, 2, 3), (8, True, 6, 1),
+                                                     (8, False, 9, 3), (16, True, 20, 2)])
+def test_sorted_inserts_of_new_keys_split_like_the_oracle(w, versioned, every, warps):
+    """Runs of new keys in key order, so dense that a group of 32 splits one or two leaves, or so sparse that each of
+    its keys may split another (fewer slots than splits), over several rounds: parents fill up and split too."""
+    from emu import EmuTree
+    import oracle
+    t = EmuTree(versioned, capacity=1 << 14, tiles=4, W=w, chunk=64)
+    m = oracle.MVMap(versioned)
+    base = np.arange(1, 701, dtype=np.uint32) * 3000
+    snaps = []
+    for r in range(4):
+        new = base[::every] + r
+        t.write_warp(np.ones(new.size), new, new ^ r, warps=warps, sorted_run=True) if r else t.write_warp(np.ones(base.size), base, base)
+        m.insert(new, new ^ r) if r else m.insert(base, base)
+        if versioned:
+            snaps.append(t.snapshot())
+            assert snaps[-1] == m.take_snapshot()
+        assert t.errors == 0, t.stats()
+    q = np.concatenate([base + r for r in range(5)])
+    for s in snaps or [0xFFFFFFFF]:
+        assert np.array_equal(t.find_warp(q, s), m.find(q, s) if versioned else m.find(q)), s
+        rep = t.validate(s)
+        assert rep["violations"] == 0 and rep["locked_nodes"] == 0
+
+
+def test_splits_without_a_node_give_up_their_key_alone():
+    """The pool runs out among the splits of a sorted run: the status says so, and the tree stays whole."""
+    from emu import EmuTree
+    t = EmuTree(False, capacity=256, chunk=32)
+    base = np.arange(1, 601, dtype=np.uint32) * 3000
+    t.write_warp(np.ones(base.size), base, base)
+    assert t.errors == 0
+    new = np.concatenate([base + d for d in range(1, 6)])
+    t.write_warp(np.ones(new.size), new, new, warps=2, sorted_run=True)
+    assert t.errors == 1, t.stats()
+    assert np.array_equal(t.find_warp(base), base)
+    got = t.find_warp(np.sort(new))
+    assert np.all((got == np.sort(new)) | (got == 0xFFFFFFFF)) and np.count_nonzero(got != 0xFFFFFFFF) > 100
+    rep = t.validate()
+    assert rep["violations"] == 0 and rep["locked_nodes"] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("versioned,tile,every", [(False, 8, 1), (True, 16, 1), (True, 8, 3), (False, 16, 11)])
+def test_gpu_sorted_inserts_of_new_keys_match_oracle(versioned, tile, every):
+    import torch
+    import mvgpubtree_b200 as mv
+    import oracle
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.uint32).view(np.int32)).cuda()
+    cls = mv.gpu_versioned_btree if versioned else mv.gpu_blink_tree
+    t, m = cls(pool_bytes=1 << 28, tile_width=tile, frontend=2), oracle.MVMap(versioned)
+    rng = np.random.default_rng(every)
+    base = rng.permutation(np.arange(1, 120_001, dtype=np.uint32)) * 30_000
+    snaps = []
+    for r in range(5):
+        new = base[::every] + r if r else base
+        t.insert(dev(new), dev(new ^ r))
+        m.insert(new, new ^ r)
+        if versioned:
+            snaps.append(t.take_snapshot())
+            assert snaps[-1] == m.take_snapshot()
+    q = np.concatenate([base + r for r in range(6)])
+    out = torch.zeros(q.size, dtype=torch.int32, device="cuda")
+    for s in snaps[::2] or [mv.LATEST]:
+        t.find(dev(q), out, timestamp=s)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), m.find(q, s) if versioned else m.find(q))
+    assert t.check_errors() == 0
+    rep = t.validate_tree_structure()
+    assert rep["violations"] == 0 and rep["locked_nodes"] == 0
