@@ -129,8 +129,17 @@ void mvbt_config_init(mvbt_config* cfg);
  * (include/gpu_versioned_blink_tree.hpp:88-93). */
 int mvbt_create(int kind, const mvbt_config* cfg, mvbt_tree** out);
 
-/* Frees the pool and all buffers. Replaces the shared_ptr teardown of the reference handles. */
+/* Frees the pool and all buffers. Replaces the shared_ptr teardown of the reference handles. The node block of
+ * a tree of up to 2 GiB goes back to a memory pool of the library, which keeps freed blocks for the next
+ * tree: up to 4 GiB per device, live trees from the pool counted in. A second pool keeps the sort's
+ * scratch likewise. The library's own allocations take what the pools keep before they fail; other
+ * allocators in the process cannot, so a program that needs the memory elsewhere calls
+ * mvbt_release_memory. */
 int mvbt_destroy(mvbt_tree* tree);
+
+/* Gives the device memory that the library keeps after frees back to the driver (device -1: the current
+ * one). Synchronises the device. No counterpart in the reference. */
+int mvbt_release_memory(int device);
 
 /* Sets the batch front-end of the bulk calls (MVBT_FRONTEND_*), as config.frontend does at
  * creation. Host-side only; affects calls issued afterwards. No counterpart in the reference. */

@@ -18,7 +18,7 @@ __all__ = [
     "gpu_versioned_btree", "gpu_versioned_blink_tree", "pair_dtype_words", "BatchPlan",
     "BATCH_PERSISTENT", "BATCH_PER_LAUNCH", "BATCH_GRAPH", "NOALLOC_MAX_OPS", "NOALLOC_MAX_BATCHES",
     "FRONTEND_AUTO", "FRONTEND_UNSORTED", "FRONTEND_SORTED",
-    "RECLAIM_ALL", "SERVE_SNAPSHOT_PER_BATCH", "SERVE_SNAPSHOT_PER_REQUEST", "load",
+    "RECLAIM_ALL", "SERVE_SNAPSHOT_PER_BATCH", "SERVE_SNAPSHOT_PER_REQUEST", "load", "release_memory",
 ]
 
 LATEST = 0xFFFFFFFF
@@ -82,6 +82,7 @@ _P = _vp
 _sig("mvbt_config_init", None, ctypes.POINTER(mvbt_config))
 _sig("mvbt_create", ctypes.c_int, ctypes.c_int, ctypes.POINTER(mvbt_config), ctypes.POINTER(_vp))
 _sig("mvbt_destroy", ctypes.c_int, _vp)
+_sig("mvbt_release_memory", ctypes.c_int, ctypes.c_int)
 _sig("mvbt_set_frontend", ctypes.c_int, _vp, _u32)
 _sig("mvbt_insert", ctypes.c_int, _vp, _P, _P, _u32, _vp, ctypes.c_int)
 _sig("mvbt_find", ctypes.c_int, _vp, _P, _P, _u32, _u32, _vp, ctypes.c_int)
@@ -191,6 +192,13 @@ def _stream(stream) -> int:
     if hasattr(stream, "cuda_stream"):
         return int(stream.cuda_stream)
     raise TypeError("stream must be None, an int handle or a torch.cuda.Stream")
+
+
+def release_memory(device: int | None = None) -> None:
+    """Gives the device memory that the library keeps after frees (dropped trees and the sort's scratch, up to
+    4 GiB each per device) back to the driver. The library's own allocations do so before they fail; call it
+    where another allocator of the process needs the memory."""
+    _check(lib.mvbt_release_memory(-1 if device is None else int(device)), "release_memory")
 
 
 class _TreeBase:

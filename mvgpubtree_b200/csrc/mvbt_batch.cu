@@ -13,6 +13,7 @@
 
 #include "mvbt.h"
 #include "mvbt_device.cuh"
+#include "mvbt_memory.h"
 
 namespace cg = cooperative_groups;
 using mvbt::batch_sched;
@@ -421,11 +422,11 @@ int mvbt_batch_plan_create(mvbt_tree* tree, uint64_t max_ops, uint32_t max_batch
   p->tree        = tree;
   p->max_ops     = max_ops;
   p->max_batches = max_batches;
-  bool ok = cudaMalloc(&p->d_batch_off, stage_bytes(max_batches)) == cudaSuccess &&
-            cudaMalloc(&p->d_perm, max_ops * sizeof(uint32_t)) == cudaSuccess &&
-            cudaMalloc(&p->d_counts, (6ull * max_batches + 4) * sizeof(uint32_t)) == cudaSuccess &&
-            cudaMalloc(&p->d_pre, 2ull * (max_batches + 1) * sizeof(uint64_t)) == cudaSuccess &&
-            cudaMalloc(&p->d_cursor, 2 * sizeof(unsigned long long)) == cudaSuccess &&
+  bool ok = mvbt_mem::alloc(&p->d_batch_off, stage_bytes(max_batches)) == cudaSuccess &&
+            mvbt_mem::alloc(&p->d_perm, max_ops * sizeof(uint32_t)) == cudaSuccess &&
+            mvbt_mem::alloc(&p->d_counts, (6ull * max_batches + 4) * sizeof(uint32_t)) == cudaSuccess &&
+            mvbt_mem::alloc(&p->d_pre, 2ull * (max_batches + 1) * sizeof(uint64_t)) == cudaSuccess &&
+            mvbt_mem::alloc(&p->d_cursor, 2 * sizeof(unsigned long long)) == cudaSuccess &&
             cudaMallocHost(&p->h_batch_off, stage_bytes(max_batches)) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
@@ -474,7 +475,7 @@ void* mvbt_internal_plan_scratch(mvbt_batch_plan* p, uint64_t bytes) {
   if (p->d_scratch) cudaFree(p->d_scratch);
   p->d_scratch     = nullptr;
   p->scratch_bytes = 0;
-  if (cudaMalloc(&p->d_scratch, bytes) != cudaSuccess) {
+  if (mvbt_mem::alloc(&p->d_scratch, bytes) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
@@ -627,7 +628,7 @@ int mvbt_batch_plan_set_reclaim(mvbt_batch_plan* p, int enable, uint32_t min_liv
   if (enable && !p->d_rc) {
     const uint64_t mb    = p->max_batches;
     const uint64_t bytes = rc_head_words(mb) * 4 + (mb + 1) * 8 + 4 * mb * 8;
-    if (cudaMalloc(&p->d_rc, bytes) != cudaSuccess) {
+    if (mvbt_mem::alloc(&p->d_rc, bytes) != cudaSuccess) {
       cudaGetLastError();
       return fail(MVBT_ERR_OUT_OF_MEMORY, "batch plan: reclamation scratch");
     }

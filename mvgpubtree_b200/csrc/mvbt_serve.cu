@@ -28,6 +28,7 @@
 
 #include "mvbt.h"
 #include "mvbt_device.cuh"
+#include "mvbt_memory.h"
 
 using mvbt::device_tree;
 
@@ -208,13 +209,13 @@ int mvbt_serve_trace(mvbt_tree* tree, const mvbt_serve_config* cfg_in, uint32_t 
       st = mvbt_batch_plan_set_reclaim(s.plan, 1, MVBT_RECLAIM_ALL);
       if (st) return st;
     }
-    SERVE_TRY(cudaMalloc(&s.type, mo * 4));
-    SERVE_TRY(cudaMalloc(&s.key, mo * 4));
-    SERVE_TRY(cudaMalloc(&s.arg, mo * 4));
-    SERVE_TRY(cudaMalloc(&s.cap, mo * 4));
-    SERVE_TRY(cudaMalloc(&s.result, mo * 4));
-    SERVE_TRY(cudaMalloc(&s.off, mo * 8));
-    SERVE_TRY(cudaMalloc(&s.range, std::max<uint64_t>(mp, 1) * sizeof(mvbt_pair)));
+    SERVE_TRY(mvbt_mem::alloc(&s.type, mo * 4));
+    SERVE_TRY(mvbt_mem::alloc(&s.key, mo * 4));
+    SERVE_TRY(mvbt_mem::alloc(&s.arg, mo * 4));
+    SERVE_TRY(mvbt_mem::alloc(&s.cap, mo * 4));
+    SERVE_TRY(mvbt_mem::alloc(&s.result, mo * 4));
+    SERVE_TRY(mvbt_mem::alloc(&s.off, mo * 8));
+    SERVE_TRY(mvbt_mem::alloc(&s.range, std::max<uint64_t>(mp, 1) * sizeof(mvbt_pair)));
     SERVE_TRY(cudaEventCreateWithFlags(&s.h2d, cudaEventDisableTiming));
     SERVE_TRY(cudaEventCreateWithFlags(&s.kdone, cudaEventDisableTiming));
     SERVE_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));

@@ -11,11 +11,13 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
 #include "mvbt.h"
 #include "mvbt_device.cuh"
+#include "mvbt_memory.h"
 #include "mvbt_sort.h"
 
 namespace cg = cooperative_groups;
@@ -612,66 +614,39 @@ bool sorted_lookups(const mvbt_tree* t, uint32_t n) {
   return t->frontend == MVBT_FRONTEND_SORTED && n > 1;
 }
 
-
-// Stream-ordered memory pools per device, one for the sort's scratch and one for trees: no device-wide
-// synchronisation, and freed blocks stay cached in the pool for the next call (up to kPoolKeepBytes).
-// Two, because a pool that holds more than it may keep gives back every freed block at the next
-// synchronisation: with 5.8 GB of trees in the scratch's pool each sorted call mapped its scratch anew
-// (2^25 finds 13 ms instead of 2).
-constexpr int kMaxDevices           = 64;
-constexpr uint64_t kPoolKeepBytes   = 4ull << 30;
-cudaMemPool_t g_pools[2][kMaxDevices] = {};  // scratch, trees
-std::mutex g_pools_mu;
-
-int library_pool(int dev, bool trees, cudaMemPool_t* out) {
-  if (dev < 0 || dev >= kMaxDevices) return fail(MVBT_ERR_BAD_ARG, "device ordinal out of range");
-  std::lock_guard<std::mutex> lk(g_pools_mu);
-  if (!g_pools[trees][dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType        = cudaMemAllocationTypePinned;
-    props.location.type    = cudaMemLocationTypeDevice;
-    props.location.id      = dev;
-    MVBT_CUDA_TRY(cudaMemPoolCreate(&g_pools[trees][dev], &props));
-    uint64_t keep = kPoolKeepBytes;
-    MVBT_CUDA_TRY(cudaMemPoolSetAttribute(g_pools[trees][dev], cudaMemPoolAttrReleaseThreshold, &keep));
-  }
-  *out = g_pools[trees][dev];
-  return MVBT_OK;
-}
-
 // A tree's device block. Blocks of up to kPooledTree come from the memory pool, so a program that
 // builds and drops trees does not map and unmap their memory each time (1 GiB: cudaMalloc 0.63 ms and
-// cudaFree 0.93 ms, from the pool 0.01 ms). When the device is full, what the pool keeps is given back first.
+// cudaFree 0.93 ms, from the pool 0.01 ms).
 constexpr uint64_t kPooledTree = 2ull << 30;
 int tree_alloc(int dev, uint64_t bytes, void** out, bool* pooled) {
-  cudaMemPool_t pool;
-  int st = library_pool(dev, true, &pool);
-  if (st) return st;
-  *pooled = bytes <= kPooledTree && cudaMallocFromPoolAsync(out, bytes, pool, nullptr) == cudaSuccess;
+  *pooled = bytes <= kPooledTree && mvbt_mem::pool_alloc(dev, mvbt_mem::kTrees, out, bytes, nullptr) == cudaSuccess;
   if (*pooled) return MVBT_OK;
   cudaGetLastError();
-  if (cudaMalloc(out, bytes) == cudaSuccess) return MVBT_OK;
-  cudaGetLastError();
-  cudaMemPool_t scratch;
-  if (library_pool(dev, false, &scratch) == MVBT_OK) cudaMemPoolTrimTo(scratch, 0);
-  cudaMemPoolTrimTo(pool, 0);
-  if (cudaMalloc(out, bytes) == cudaSuccess) return MVBT_OK;
+  if (mvbt_mem::alloc(out, bytes) == cudaSuccess) return MVBT_OK;
   cudaGetLastError();
   return fail(MVBT_ERR_OUT_OF_MEMORY, "cudaMalloc of the node pool failed");
 }
 
 // The pinned host word of a tree, from pages of 64 that the process keeps (as many as it ever held trees
-// at once): pinning a page for each tree took 1.3-2.5 ms, and unpinning it 0.4 ms.
+// at once): pinning a page for each tree took 1.3-2.5 ms, and unpinning it 0.4 ms. The free list has room
+// for the words of every page from the start, so giving one back does not allocate.
 std::vector<uint32_t*> g_host_words;
+size_t g_host_pages = 0;
 std::mutex g_host_words_mu;
 uint32_t* take_host_word() {
   std::lock_guard<std::mutex> lk(g_host_words_mu);
   if (g_host_words.empty()) {
+    try {
+      g_host_words.reserve(64 * (g_host_pages + 1));
+    } catch (const std::bad_alloc&) {
+      return nullptr;
+    }
     void* page = nullptr;
     if (cudaHostAlloc(&page, 4096, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
+    ++g_host_pages;
     for (int i = 0; i < 64; ++i) g_host_words.push_back(static_cast<uint32_t*>(page) + 16 * i);
   }
   uint32_t* w = g_host_words.back();
@@ -700,13 +675,10 @@ struct sorted_ops {
 
 int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaStream_t s, sorted_ops* out,
              const uint32_t* values = nullptr, uint64_t extra_words = 0) {
-  cudaMemPool_t pool;
-  int st = library_pool(t->device, false, &pool);
-  if (st) return st;
   const uint64_t sort_words = 4ull * n + ((mvbt_sort::scratch_words(n) + 63) & ~63ull);
   const uint64_t words      = sort_words + extra_words;
   void* mem            = nullptr;
-  if (cudaMallocFromPoolAsync(&mem, words * 4, pool, s) != cudaSuccess) {
+  if (mvbt_mem::pool_alloc(t->device, mvbt_mem::kScratch, &mem, words * 4, s) != cudaSuccess) {
     cudaGetLastError();
     return fail(MVBT_ERR_OUT_OF_MEMORY, "sort scratch: cudaMallocFromPoolAsync failed");
   }
@@ -844,8 +816,8 @@ int mvbt_create(int kind, const mvbt_config* cfg_in, mvbt_tree** out) {
     auto pow2 = [](uint64_t x) { uint64_t p = 1; while (p < x) p <<= 1; return p; };
     log_cap  = (uint32_t)pow2(capacity);
     ring_cap = (uint32_t)pow2(capacity + (uint64_t)mvbt::kMaxSmSlots * t->chunk);
-    if (cudaMalloc(&t->retire_log, (uint64_t)log_cap * 4) != cudaSuccess ||
-        cudaMalloc(&t->free_ring, (uint64_t)ring_cap * 4) != cudaSuccess) {
+    if (mvbt_mem::alloc(&t->retire_log, (uint64_t)log_cap * 4) != cudaSuccess ||
+        mvbt_mem::alloc(&t->free_ring, (uint64_t)ring_cap * 4) != cudaSuccess) {
       cudaGetLastError();
       mvbt_destroy(t);
       return fail(MVBT_ERR_OUT_OF_MEMORY, "cudaMalloc of the reclamation rings failed");
@@ -882,6 +854,18 @@ int mvbt_destroy(mvbt_tree* t) {
   if (t->free_ring) cudaFree(t->free_ring);
   if (t->h_word) give_host_word(t->h_word);
   delete t;
+  return MVBT_OK;
+}
+
+int mvbt_release_memory(int device) {
+  int before = 0;
+  MVBT_CUDA_TRY(cudaGetDevice(&before));
+  const int dev = device < 0 ? before : device;
+  MVBT_CUDA_TRY(cudaSetDevice(dev));
+  cudaError_t e = cudaDeviceSynchronize();  // blocks freed by calls that still run count as kept
+  if (e == cudaSuccess) e = mvbt_mem::release(dev);
+  cudaSetDevice(before);
+  if (e != cudaSuccess) return fail(MVBT_ERR_CUDA, std::string("release of kept memory: ") + cudaGetErrorString(e));
   return MVBT_OK;
 }
 
@@ -1079,17 +1063,14 @@ int mvbt_bulk_build(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, 
   plan_levels(P, t->capacity);
   if (P.status == 1) return fail(MVBT_ERR_BAD_ARG, "bulk build: tree too tall");
   if (P.status == 2) return fail(MVBT_ERR_POOL_EXHAUSTED, "bulk build: the pool is too small");
-  cudaMemPool_t pool;
-  int st = library_pool(t->device, false, &pool);
-  if (st) return st;
   bulk_plan* dplan = nullptr;
-  MVBT_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dplan), sizeof(bulk_plan), pool, s));
+  MVBT_CUDA_TRY(mvbt_mem::pool_alloc(t->device, mvbt_mem::kScratch, reinterpret_cast<void**>(&dplan), sizeof(bulk_plan), s));
   MVBT_CUDA_TRY(cudaMemcpyAsync(dplan, &P, sizeof(bulk_plan), cudaMemcpyHostToDevice, s));  // staged: P may go
   const uint64_t threads = P.total * 32;
   const unsigned grid    = (unsigned)std::min<uint64_t>((threads + 255) / 256, (uint64_t)t->num_sms * 64);
   k_bulk_build<<<grid, 256, 0, s>>>(t->pool, dplan);
   k_bulk_anchor<<<1, 32, 0, s>>>(t->pool, t->ctl, dplan);
-  st = check_launch();
+  int st = check_launch();
   MVBT_CUDA_TRY(cudaFreeAsync(dplan, s));
   t->pristine = false;
   if (st) return st;
