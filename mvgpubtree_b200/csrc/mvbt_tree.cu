@@ -675,7 +675,7 @@ struct sorted_ops {
 
 int sort_ops(mvbt_tree* t, const uint32_t* keys, uint32_t n, int low_bit, cudaStream_t s, sorted_ops* out,
              const uint32_t* values = nullptr, uint64_t extra_words = 0) {
-  const uint64_t sort_words = 4ull * n + ((mvbt_sort::scratch_words(n) + 63) & ~63ull);
+  const uint64_t sort_words = (4ull * n + mvbt_sort::scratch_words(n) + 63) & ~63ull;
   const uint64_t words      = sort_words + extra_words;
   void* mem            = nullptr;
   if (mvbt_mem::pool_alloc(t->device, mvbt_mem::kScratch, &mem, words * 4, s) != cudaSuccess) {

@@ -142,3 +142,24 @@ def test_gpu_sorted_inserts_of_new_keys_match_oracle(versioned, tile, every):
     assert t.check_errors() == 0
     rep = t.validate_tree_structure()
     assert rep["violations"] == 0 and rep["locked_nodes"] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("versioned", [False, True])
+@pytest.mark.parametrize("frontend", [0, 1])
+def test_gpu_writes_queueing_on_one_leaf_all_run(versioned, frontend):
+    """A million erases in a tree of one leaf, and 100 000 inserts of one key: thousands of warps wait for one lock."""
+    import torch
+    import mvgpubtree_b200 as mv
+    cls = mv.gpu_versioned_btree if versioned else mv.gpu_blink_tree
+    t = cls(pool_bytes=1 << 26, frontend=frontend)
+    t.erase(torch.arange(1, 1_000_001, dtype=torch.int32, device="cuda"))
+    assert t.check_errors() == 0
+    base = torch.arange(1, 300_000, dtype=torch.int32, device="cuda")
+    t.insert(base * 5000, base)
+    one = torch.full((100_000,), 777, dtype=torch.int32, device="cuda")
+    t.insert(one, one)
+    assert t.check_errors() == 0
+    out = torch.zeros(1, dtype=torch.int32, device="cuda")
+    t.find(one[:1], out)
+    assert int(out) == 777
