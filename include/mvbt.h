@@ -93,8 +93,10 @@ typedef struct mvbt_config {
  * dense against the tree (at least 2^16 ops and one op per 128 keys), where neighbouring ops share
  * nodes. Results are the same either way (for a repeated key in one insert call, UNSORTED leaves which
  * value wins unspecified, as the reference does). The sort's scratch (16 bytes per op) comes from a
- * stream-ordered memory pool of the library; reads that AUTO would sort run unsorted without it. No
- * counterpart in the reference. */
+ * stream-ordered memory pool of the library; reads that AUTO would sort run unsorted without it. A sorted call
+ * that is captured into a graph holds the scratch's allocation and free as nodes; reads with concurrent = 0
+ * that are not dense in the tree are not sorted while captured, and stay one kernel. No counterpart in
+ * the reference. */
 #define MVBT_FRONTEND_AUTO 0u
 #define MVBT_FRONTEND_UNSORTED 1u
 #define MVBT_FRONTEND_SORTED 2u

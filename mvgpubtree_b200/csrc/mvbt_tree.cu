@@ -553,12 +553,6 @@ int status_from_bits(uint32_t bits) {
   return MVBT_OK;
 }
 
-// Whether range queries likewise are sorted by lower bound first (the lookups' line).
-bool sorted_ranges(const mvbt_tree* t, uint32_t n) {
-  if (t->frontend == MVBT_FRONTEND_AUTO) return n >= (1u << 20);
-  return t->frontend == MVBT_FRONTEND_SORTED && n > 1;
-}
-
 // Fewer lookups than this leave most warps of k_find_warp empty; a tile per key has the shorter
 // chain then. Tile / warp per call in a tree of 2^20 keys: 4000 lookups 10.7 / 10.7 us (the launch),
 // 16000 11.2 / 10.6, 65536 16.5 / 10.9, 262144 55 / 29.
@@ -605,15 +599,22 @@ bool use_sorted(const mvbt_tree* t, uint32_t n) {
   return n >= (1u << 16) && (uint64_t)n * 128 >= t->grown;
 }
 
-// Whether lookups in a tree no writer changes meanwhile are sorted first. A warp's lookups in the
+// Whether lookups in a tree no writer changes meanwhile are sorted first (range queries by lower bound likewise). A warp's lookups in the
 // caller's order cost about as much as sorting and then looking up at 2^20 keys (us, unsorted /
 // sorted: 93 / 91 in a tree of 2^20 keys, 125 / 120 in one of 40M, 73 / 80 in one of 2^16); at 2^22
 // they cost twice as much (354 / 195, 474 / 262, 271 / 169), at 2^18 half (29 / 62, 38 / 71, 23 / 58).
-bool sorted_lookups(const mvbt_tree* t, uint32_t n) {
-  if (t->frontend == MVBT_FRONTEND_AUTO) return n >= (1u << 20);
+// A call that is sparse in the tree and is being captured into a graph stays one kernel: the sort's scratch
+// would make allocation nodes, and a graph with those has one executable at a time and is no child graph.
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return false;
+}
+bool sorted_lookups(const mvbt_tree* t, uint32_t n, cudaStream_t s) {
+  if (t->frontend == MVBT_FRONTEND_AUTO) return n >= (1u << 20) && (use_sorted(t, n) || !capturing(s));
   return t->frontend == MVBT_FRONTEND_SORTED && n > 1;
 }
-
 // A tree's device block. Blocks of up to kPooledTree come from the memory pool, so a program that
 // builds and drops trees does not map and unmap their memory each time (1 GiB: cudaMalloc 0.63 ms and
 // cudaFree 0.93 ms, from the pool 0.01 ms).
@@ -1329,7 +1330,7 @@ int mvbt_find(mvbt_tree* t, const uint32_t* keys, uint32_t* values, uint32_t n, 
   if (t->kind == MVBT_KIND_BLINK) ts = mvbt::kLatest;
   cudaStream_t s = as_stream(stream);
   const int bs   = t->block_size;
-  if (concurrent ? use_sorted(t, n) : sorted_lookups(t, n)) {
+  if (concurrent ? use_sorted(t, n) : sorted_lookups(t, n, s)) {
     sorted_ops so;
     int st = sort_ops(t, keys, n, kReadSortLowBit, s, &so);
     // without memory for the sort a call that need not be sorted runs in the caller's order
@@ -1392,7 +1393,7 @@ int mvbt_range_query(mvbt_tree* t, const uint32_t* lower, const uint32_t* upper,
   cudaStream_t s = as_stream(stream);
   uint2* out     = reinterpret_cast<uint2*>(result);
   const int bs   = t->block_size;
-  if (concurrent ? use_sorted(t, n) : sorted_ranges(t, n)) {
+  if (concurrent ? use_sorted(t, n) : sorted_lookups(t, n, s)) {
     sorted_ops so;
     int st = sort_ops(t, lower, n, kReadSortLowBit, s, &so);
     // without memory for the sort a call that need not be sorted runs in the caller's order

@@ -1,6 +1,5 @@
 """GPU tier: what the library keeps of dropped trees and of the sort's scratch is given back on request, and before
-any of its own allocations fails."""
-import numpy as np
+any of its own allocations fails; captured reads hold no scratch that they did not need before."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +65,44 @@ def test_own_allocations_take_what_dropped_trees_left(what):
         torch.cuda.empty_cache()
         t.close()
         mv.release_memory()
+
+
+@pytest.mark.parametrize("ranges", [False, True])
+def test_captured_reads_that_are_sparse_in_the_tree_are_one_kernel(ranges):
+    """A captured read of 2^20 keys that the front-end would sort otherwise: one kernel node, no allocation, and
+    the replay answers for what the buffers hold then."""
+    import torch
+    from cuda.bindings import runtime as rt
+    import mvgpubtree_b200 as mv
+    n, keys = 1 << 20, torch.arange(1, (1 << 22) + 1, dtype=torch.int32, device="cuda") * 400
+    t = mv.gpu_blink_tree(pool_bytes=1 << 28)
+    for r in range(34):  # keys put into the tree so far: more than 128 for each of the call
+        t.insert(keys, keys + r)
+    q = torch.zeros(n, dtype=torch.int32, device="cuda")
+    hi, out, pairs = torch.zeros_like(q), torch.zeros_like(q), torch.zeros(4 * n, dtype=torch.int32, device="cuda")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+
+    def ok(r):
+        assert int(r[0]) == 0, r
+        return r[1:] if len(r) > 2 else (r[1] if len(r) > 1 else None)
+
+    ok(rt.cudaStreamBeginCapture(s.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal))
+    if ranges:
+        t.range_query(q, hi, pairs, out, 2, stream=s)
+    else:
+        t.find(q, out, stream=s)
+    graph = ok(rt.cudaStreamEndCapture(s.cuda_stream))
+    assert ok(rt.cudaGraphGetNodes(graph, 0))[1] == 1
+    execs = [ok(rt.cudaGraphInstantiate(graph, 0)) for _ in range(2)]  # both at a time
+    q.copy_(keys[torch.randperm(keys.numel(), device="cuda")[:n]])
+    hi.copy_(q + 1)
+    torch.cuda.synchronize()
+    for e in execs:
+        out.fill_(7)
+        pairs.zero_()
+        ok(rt.cudaGraphLaunch(e, s.cuda_stream))
+        torch.cuda.synchronize()
+        assert torch.equal(pairs[1::4] if ranges else out, q + 33) and (not ranges or torch.equal(out, torch.ones_like(q)))
+    assert t.check_errors() == 0
