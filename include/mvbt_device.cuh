@@ -2718,6 +2718,96 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
 }
 
 // ----------------------------------------------------------------------------------------------
+// The two concurrent calls
+// ----------------------------------------------------------------------------------------------
+// They hand out units of up to 32 ops, one unit per warp at a time: unit u of the
+// `writes + reads` units is a write unit or a read unit (Bresenham split), so both kinds run side
+// by side in every wave. Returns whether it is a write unit, and its number among its kind.
+MVBT_DEV bool split_unit(uint64_t u, uint64_t writes, uint64_t reads, uint64_t& number) {
+  const uint64_t total = writes + reads;
+  const uint64_t a = (u * writes) / total, b = ((u + 1) * writes) / total;
+  number           = b > a ? a : u - a;
+  return b > a;
+}
+
+// Inserts beside range queries, by the warps first, first + stride, ..: writes run by the warp (write_warp);
+// range queries at snapshot S by the warp (range_warp), those of a plain tree's newest state (S = kLatest) a
+// tile per query from their leaves. slow: the tile of kSlow lanes that writes fall back to.
+template <int W, int kSlow, class Warp, class Tile, class Slow>
+MVBT_DEV void insert_range_units(const device_tree& T, const uint32_t* keys, const uint32_t* values, uint32_t n_ins,
+                                 const uint32_t* lower, const uint32_t* upper, uint32_t n_rq, uint2* result,
+                                 uint32_t avg_len, uint32_t* counts, uint32_t lanes, uint32_t S, uint64_t first,
+                                 uint64_t stride, write_stage& st, const Warp& warp, const Tile& tile, const Slow& slow) {
+  const uint32_t lane   = warp.thread_rank();
+  const bool ver        = T.versioned != 0;
+  const uint32_t E      = ver ? S + 1 : 0u;
+  const uint64_t writes = ((uint64_t)n_ins + lanes - 1) / lanes, reads = ((uint64_t)n_rq + lanes - 1) / lanes;
+  for (uint64_t u = first; u < writes + reads; u += stride) {
+    uint64_t number;
+    const bool write   = split_unit(u, writes, reads, number);
+    const uint64_t i   = number * lanes + lane;
+    const bool has     = lane < lanes && i < (write ? n_ins : n_rq);
+    const uint32_t key = has ? (write ? keys[i] : lower[i]) : kEmptyKey;
+    const uint32_t leaf = leaf_warp(T, key, has && key != kEmptyKey, kAnchor, nullptr, st, warp);
+    if (write) {
+      write_warp<kSlow>(T, key, has ? values[i] : 0u, false, has, E, leaf, st, warp, slow);
+    } else {
+      const uint32_t at = leaf == kNone ? kAnchor : leaf;
+      if (ver) {
+        uint2* out       = result ? result + i * (uint64_t)avg_len : nullptr;
+        const uint32_t c = range_warp<true>(T, key, has ? upper[i] : 0u, has, S, out, avg_len, at, nullptr, st, warp);
+        if (counts && has) counts[i] = c;
+        continue;
+      }
+      for_lanes<W>(warp.ballot(has), warp, [&](bool run, int src) {
+        const uint32_t lo = warp.shfl(key, src), from = warp.shfl(at, src);
+        if (run) {
+          const uint64_t r = number * lanes + src;
+          uint2* out       = result ? result + r * (uint64_t)avg_len : nullptr;
+          const uint32_t c = T.cooperative_range_query<W>(lo, upper[r], tile, S, out, avg_len, true, from);
+          if (counts && tile.thread_rank() == 0) counts[r] = c;
+        }
+      });
+    }
+  }
+}
+
+// Erases beside finds likewise: finds at snapshot S by the warp (find_warp_live), finds of a plain tree's newest
+// state a tile per key from their leaves.
+template <int W, int kSlow, class Warp, class Tile, class Slow>
+MVBT_DEV void find_erase_units(const device_tree& T, const uint32_t* fkeys, uint32_t* fres, uint32_t n_find,
+                               const uint32_t* ekeys, uint32_t n_erase, uint32_t lanes, uint32_t S, uint64_t first,
+                               uint64_t stride, write_stage& st, const Warp& warp, const Tile& tile, const Slow& slow) {
+  const uint32_t lane   = warp.thread_rank();
+  const bool ver        = T.versioned != 0;
+  const uint32_t E      = ver ? S + 1 : 0u;
+  const uint64_t writes = ((uint64_t)n_erase + lanes - 1) / lanes, reads = ((uint64_t)n_find + lanes - 1) / lanes;
+  for (uint64_t u = first; u < writes + reads; u += stride) {
+    uint64_t number;
+    const bool write   = split_unit(u, writes, reads, number);
+    const uint64_t i   = number * lanes + lane;
+    const bool has     = lane < lanes && i < (write ? n_erase : n_find);
+    const uint32_t key = has ? (write ? ekeys[i] : fkeys[i]) : kEmptyKey;
+    const uint32_t leaf = leaf_warp(T, key, has && key != kEmptyKey, kAnchor, nullptr, st, warp);
+    const uint32_t at   = leaf == kNone ? kAnchor : leaf;
+    if (write) {
+      write_warp<kSlow>(T, key, 0u, true, has, E, leaf, st, warp, slow);
+    } else if (ver) {
+      const uint32_t v = find_warp_live(T, key, has, S, at, st, warp);
+      if (has) fres[i] = v;
+    } else {
+      for_lanes<W>(warp.ballot(has), warp, [&](bool run, int src) {
+        const uint32_t k = warp.shfl(key, src), from = warp.shfl(at, src);
+        if (run) {
+          const uint32_t v = T.cooperative_find<W>(k, tile, S, true, from);
+          if (tile.thread_rank() == 0) fres[number * lanes + src] = v;
+        }
+      });
+    }
+  }
+}
+
+// ----------------------------------------------------------------------------------------------
 // Mixed operation batches
 //
 // A batch is a list of ops {type, key, arg}: find (arg unused), insert (arg = value), erase, and
@@ -2741,29 +2831,6 @@ struct batch_view {
 };
 
 MVBT_DEV bool is_write_op(uint32_t type) { return type == kOpInsert || type == kOpErase; }
-
-// Runs op i of a batch; returns true if it was a write.
-template <int W, class Tile>
-MVBT_DEV bool run_batch_op(const device_tree& T, const batch_view& B, uint64_t i, uint32_t S,
-                           uint32_t E, const Tile& t) {
-  const uint32_t ty = B.type[i], k = B.key[i];
-  uint32_t r        = 0;
-  bool write        = false;
-  if (ty == kOpFind) {
-    r = T.cooperative_find<W>(k, t, S, true);
-  } else if (ty == kOpRange) {
-    uint2* out = B.range_out ? B.range_out + B.out_off[i] : nullptr;
-    r          = T.cooperative_range_query<W>(k, B.arg[i], t, S, out, B.cap[i], true);
-  } else if (ty == kOpInsert) {
-    T.cooperative_insert<W>(k, B.arg[i], t, E);
-    write = true;
-  } else if (ty == kOpErase) {
-    T.cooperative_erase<W>(k, t, E);
-    write = true;
-  }
-  if (t.thread_rank() == 0) B.result[i] = r;
-  return write;
-}
 
 // Schedule of the persistent batched launch. Within each batch the claim order puts writes first
 // (perm maps a claim position to an op index). Writes of batch b may start once every write of
@@ -2991,6 +3058,20 @@ MVBT_DEV void run_ops_warp(const device_tree& T, const batch_view& B, uint64_t i
     }
     for (uint32_t q = 0; q < kTiles; ++q) left &= left - 1u;
     warp.sync();
+  }
+}
+
+// One batch [begin, end) at snapshot S, `lanes` ops to a warp at a time, by the warps first, first + stride, ..
+template <int W, class Warp, class Tile>
+MVBT_DEV void mixed_ops(const device_tree& T, const batch_view& B, uint64_t begin, uint64_t end, uint32_t lanes, uint32_t S,
+                        uint64_t first, uint64_t stride, write_stage& st, const Warp& warp, const Tile& tile) {
+  const uint32_t lane = warp.thread_rank();
+  for (uint64_t g = begin + first * lanes; g < end; g += stride * lanes) {
+    const uint64_t i    = g + lane;
+    const bool has      = lane < lanes && i < end;
+    const uint32_t type = has ? B.type[i] : (uint32_t)kOpFind, key = has ? B.key[i] : kEmptyKey;
+    const uint32_t leaf = leaf_warp(T, key, has && key != kEmptyKey, kAnchor, nullptr, st, warp);
+    run_ops_warp<W>(T, B, i, type, key, has, S, leaf, st, warp, tile);
   }
 }
 

@@ -347,17 +347,9 @@ __global__ void __launch_bounds__(256, kBatchBlocks) k_mixed(device_tree T, batc
   __shared__ mvbt::write_stage stage[kWarpsPerBlock];
   auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
   auto tile             = cg::tiled_partition<W>(warp);
-  mvbt::write_stage& st = stage[threadIdx.x >> 5];
   const uint32_t S      = mvbt::ld_relaxed_u32(snap_word);
-  const uint32_t lane   = threadIdx.x & 31u;
-  const uint64_t stride = (((uint64_t)gridDim.x * blockDim.x) >> 5) * lanes;
-  for (uint64_t g = begin + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes; g < end; g += stride) {
-    const uint64_t i    = g + lane;
-    const bool has      = lane < lanes && i < end;
-    const uint32_t type = has ? B.type[i] : (uint32_t)mvbt::kOpFind, key = has ? B.key[i] : mvbt::kEmptyKey;
-    const uint32_t leaf = mvbt::leaf_warp(T, key, has && key != mvbt::kEmptyKey, mvbt::kAnchor, nullptr, st, warp);
-    mvbt::run_ops_warp<W>(T, B, i, type, key, has, S, leaf, st, warp, tile);
-  }
+  mvbt::mixed_ops<W>(T, B, begin, end, lanes, S, ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                     ((uint64_t)gridDim.x * blockDim.x) >> 5, stage[threadIdx.x >> 5], warp, tile);
 }
 
 __global__ void k_snapshot_word(mvbt::control_block* ctl, uint32_t* out) {

@@ -297,18 +297,8 @@ __global__ void __launch_bounds__(256) k_range(device_tree T, const uint32_t* __
   }
 }
 
-// The mixed kernels hand out units of up to 32 ops, one unit per warp at a time: unit u of the
-// `writes + reads` units is a write unit or a read unit (Bresenham split), so both kinds run side
-// by side in every wave. Returns whether it is a write unit, and its number among its kind.
-__device__ __forceinline__ bool split_unit(uint64_t u, uint64_t writes, uint64_t reads, uint64_t& number) {
-  const uint64_t total = writes + reads;
-  const uint64_t a = (u * writes) / total, b = ((u + 1) * writes) / total;
-  number           = b > a ? a : u - a;
-  return b > a;
-}
-
-// Writes run by the warp (mvbt::write_warp); range queries at the launch snapshot by the warp
-// (mvbt::range_warp), those of a plain tree's newest state a tile per query from their leaves.
+// Inserts beside range queries, and erases beside finds, in units of `lanes` ops (mvbt::insert_range_units,
+// mvbt::find_erase_units).
 template <int W>
 __global__ void __launch_bounds__(256, 4)
     k_insert_range(device_tree T, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ values,
@@ -316,83 +306,25 @@ __global__ void __launch_bounds__(256, 4)
                    uint32_t n_rq, uint2* result, uint32_t avg_len, uint32_t* counts, uint32_t lanes,
                    const uint32_t* snap_word) {
   __shared__ mvbt::write_stage stage[kWarpsPerBlock];
-  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
-  auto tile             = cg::tiled_partition<W>(warp);
-  mvbt::write_stage& st = stage[threadIdx.x >> 5];
-  const uint32_t lane   = threadIdx.x & 31u;
-  const bool ver        = T.versioned != 0;
-  const uint32_t S      = ver ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
-  const uint32_t E      = ver ? S + 1 : 0u;
-  const uint64_t writes = ((uint64_t)n_ins + lanes - 1) / lanes, reads = ((uint64_t)n_rq + lanes - 1) / lanes;
-  for (uint64_t u = first_tile<32>(); u < writes + reads; u += num_tiles<32>()) {
-    uint64_t number;
-    const bool write   = split_unit(u, writes, reads, number);
-    const uint64_t i   = number * lanes + lane;
-    const bool has     = lane < lanes && i < (write ? n_ins : n_rq);
-    const uint32_t key = has ? (write ? keys[i] : lower[i]) : mvbt::kEmptyKey;
-    const uint32_t leaf = mvbt::leaf_warp(T, key, has && key != mvbt::kEmptyKey, mvbt::kAnchor, nullptr, st, warp);
-    if (write) {
-      mvbt::write_warp<kSlowTile>(T, key, has ? values[i] : 0u, false, has, E, leaf, st, warp, slow_tile());
-    } else {
-      const uint32_t at = leaf == mvbt::kNone ? mvbt::kAnchor : leaf;
-      if (ver) {
-        uint2* out       = result ? result + i * (uint64_t)avg_len : nullptr;
-        const uint32_t c = mvbt::range_warp<true>(T, key, has ? upper[i] : 0u, has, S, out, avg_len, at, nullptr, st, warp);
-        if (counts && has) counts[i] = c;
-        continue;
-      }
-      mvbt::for_lanes<W>(warp.ballot(has), warp, [&](bool run, int src) {
-        const uint32_t lo = warp.shfl(key, src), from = warp.shfl(at, src);
-        if (run) {
-          const uint64_t r = number * lanes + src;
-          uint2* out       = result ? result + r * (uint64_t)avg_len : nullptr;
-          const uint32_t c = T.cooperative_range_query<W>(lo, upper[r], tile, S, out, avg_len, true, from);
-          if (counts && tile.thread_rank() == 0) counts[r] = c;
-        }
-      });
-    }
-  }
+  auto warp        = cg::tiled_partition<32>(cg::this_thread_block());
+  auto tile        = cg::tiled_partition<W>(warp);
+  const uint32_t S = T.versioned ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
+  mvbt::insert_range_units<W, kSlowTile>(T, keys, values, n_ins, lower, upper, n_rq, result, avg_len, counts, lanes, S,
+                                         first_tile<32>(), num_tiles<32>(), stage[threadIdx.x >> 5], warp, tile,
+                                         slow_tile());
 }
 
-// Erases run by the warp; finds at the launch snapshot by the warp (mvbt::find_warp_live), finds of a
-// plain tree's newest state a tile per key from their leaves.
 template <int W>
 __global__ void __launch_bounds__(256, 4)
     k_find_erase(device_tree T, const uint32_t* __restrict__ fkeys, uint32_t* __restrict__ fres,
                  uint32_t n_find, const uint32_t* __restrict__ ekeys, uint32_t n_erase, uint32_t lanes,
                  const uint32_t* snap_word) {
   __shared__ mvbt::write_stage stage[kWarpsPerBlock];
-  auto warp             = cg::tiled_partition<32>(cg::this_thread_block());
-  auto tile             = cg::tiled_partition<W>(warp);
-  mvbt::write_stage& st = stage[threadIdx.x >> 5];
-  const uint32_t lane   = threadIdx.x & 31u;
-  const bool ver        = T.versioned != 0;
-  const uint32_t S      = ver ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
-  const uint32_t E      = ver ? S + 1 : 0u;
-  const uint64_t writes = ((uint64_t)n_erase + lanes - 1) / lanes, reads = ((uint64_t)n_find + lanes - 1) / lanes;
-  for (uint64_t u = first_tile<32>(); u < writes + reads; u += num_tiles<32>()) {
-    uint64_t number;
-    const bool write   = split_unit(u, writes, reads, number);
-    const uint64_t i   = number * lanes + lane;
-    const bool has     = lane < lanes && i < (write ? n_erase : n_find);
-    const uint32_t key = has ? (write ? ekeys[i] : fkeys[i]) : mvbt::kEmptyKey;
-    const uint32_t leaf = mvbt::leaf_warp(T, key, has && key != mvbt::kEmptyKey, mvbt::kAnchor, nullptr, st, warp);
-    const uint32_t at   = leaf == mvbt::kNone ? mvbt::kAnchor : leaf;
-    if (write) {
-      mvbt::write_warp<kSlowTile>(T, key, 0u, true, has, E, leaf, st, warp, slow_tile());
-    } else if (ver) {
-      const uint32_t v = mvbt::find_warp_live(T, key, has, S, at, st, warp);
-      if (has) fres[i] = v;
-    } else {
-      mvbt::for_lanes<W>(warp.ballot(has), warp, [&](bool run, int src) {
-        const uint32_t k = warp.shfl(key, src), from = warp.shfl(at, src);
-        if (run) {
-          const uint32_t v = T.cooperative_find<W>(k, tile, S, true, from);
-          if (tile.thread_rank() == 0) fres[number * lanes + src] = v;
-        }
-      });
-    }
-  }
+  auto warp        = cg::tiled_partition<32>(cg::this_thread_block());
+  auto tile        = cg::tiled_partition<W>(warp);
+  const uint32_t S = T.versioned ? mvbt::ld_relaxed_u32(snap_word) : mvbt::kLatest;
+  mvbt::find_erase_units<W, kSlowTile>(T, fkeys, fres, n_find, ekeys, n_erase, lanes, S, first_tile<32>(),
+                                       num_tiles<32>(), stage[threadIdx.x >> 5], warp, tile, slow_tile());
 }
 
 // ----------------------------------------------------------------------------------------------

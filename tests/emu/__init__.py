@@ -33,8 +33,8 @@ def lib():
             "emu_range_warp": (None, [vp, u32p, u32p, u32p, u32p, u32p, u32, u64, u32, i, i, i]),
             "emu_write_warp": (None, [vp, u32p, u32p, u32p, u64, i, i, i]),
             "emu_range": (None, [vp, u32p, u32p, vp, vp, u32, u64, u32, i, i, i]),
-            "emu_insert_range": (None, [vp, u32p, u32p, u64, u32p, u32p, u64, vp, vp, u32, i, i]),
-            "emu_find_erase": (None, [vp, u32p, u32p, u64, u32p, u64, i, i]),
+            "emu_insert_range": (None, [vp, u32p, u32p, u64, u32p, u32p, u64, vp, vp, u32, i, i, u32]),
+            "emu_find_erase": (None, [vp, u32p, u32p, u64, u32p, u64, i, i, u32]),
             "emu_sorted_run": (None, [vp, i, u32p, u32p, vp, vp, vp, u32, u64, u32, i, i]),
             "emu_validate": (i, [vp, u32, vp]),
             "emu_stats": (None, [vp, np.ctypeslib.ndpointer(dtype=np.uint64, flags="C_CONTIGUOUS")]),
@@ -164,18 +164,18 @@ class EmuTree:
             return pairs[: k.size], out
         return out
 
-    def find_erase(self, fk, ek):
+    def find_erase(self, fk, ek, lanes: int = 32):
         fk, ek = _u32(fk), _u32(ek)
         out = np.empty_like(fk)
-        self.L.emu_find_erase(self.h, fk, out, fk.size, ek, ek.size, self.tiles, self.W)
+        self.L.emu_find_erase(self.h, fk, out, fk.size, ek, ek.size, self.tiles, self.W, lanes)
         return out
 
-    def insert_range(self, k, v, lo, hi, avg_len):
+    def insert_range(self, k, v, lo, hi, avg_len, lanes: int = 32):
         k, v, lo, hi = _u32(k), _u32(v), _u32(lo), _u32(hi)
         pairs = np.full((max(1, lo.size), avg_len, 2), 0xFFFFFFFF, np.uint32)
         counts = np.zeros(max(1, lo.size), np.uint32)
         self.L.emu_insert_range(self.h, k, v, k.size, lo, hi, lo.size, pairs.ctypes.data,
-                                counts.ctypes.data, avg_len, self.tiles, self.W)
+                                counts.ctypes.data, avg_len, self.tiles, self.W, lanes)
         return pairs[: lo.size], counts[: lo.size]
 
     def run_batches(self, b, mode: int = 0, reclaim: bool = False, watermark: int = 0xFFFFFFFF,

@@ -427,25 +427,20 @@ void emu_range(void* h, const uint32_t* lo, const uint32_t* hi, uint32_t* pairs,
   }));
 }
 
-// One run mixing inserts and range queries; queries read snapshot S, inserts land in S + 1.
+// One run mixing inserts and range queries in units of `lanes` ops; queries read snapshot S, inserts land in
+// S + 1.
 void emu_insert_range(void* h, const uint32_t* keys, const uint32_t* vals, uint64_t n_ins,
                       const uint32_t* lo, const uint32_t* hi, uint64_t n_rq, uint32_t* pairs,
-                      uint32_t* counts, uint32_t avg_len, int tiles, int W) {
+                      uint32_t* counts, uint32_t avg_len, int tiles, int W, uint32_t lanes) {
   auto* t          = static_cast<emu_tree*>(h);
   auto v           = t->view();
   const uint32_t S = v.versioned ? emu_snapshot(h) : mvbt::kLatest;
-  const uint32_t E = v.versioned ? S + 1 : 0u;
-  const uint64_t total = n_ins + n_rq;
-  EMU_DISPATCH(W, run(total, tiles, kW, [&](uint64_t i, const emu_tile& tile) {
-    uint64_t a = (i * n_ins) / total, b = ((i + 1) * n_ins) / total;
-    if (b > a) {
-      v.cooperative_insert<kW>(keys[a], vals[a], tile, E);
-    } else {
-      uint64_t r = i - a;
-      uint2* o   = pairs ? reinterpret_cast<uint2*>(pairs) + r * (uint64_t)avg_len : nullptr;
-      uint32_t c = v.cooperative_range_query<kW>(lo[r], hi[r], tile, S, o, avg_len, true);
-      if (counts && tile.thread_rank() == 0) counts[r] = c;
-    }
+  const int warps  = std::max(1, tiles * W / 32);
+  std::vector<mvbt::write_stage> stage(warps);
+  EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {
+    const uint32_t w = mvbt::emu::sm;
+    mvbt::insert_range_units<kW, kW>(v, keys, vals, (uint32_t)n_ins, lo, hi, (uint32_t)n_rq, reinterpret_cast<uint2*>(pairs),
+                                     avg_len, counts, lanes, S, w, (uint64_t)warps, stage[w], warp, tile, tile);
   }));
 }
 
@@ -504,20 +499,18 @@ void emu_sorted_run(void* h, int kind, const uint32_t* keys, const uint32_t* pos
   });
 }
 
-// One run mixing finds of the newest state and erases (the plain tree's concurrent_find_erase).
+// One run mixing finds and erases likewise; finds read snapshot S (a plain tree's newest state).
 void emu_find_erase(void* h, const uint32_t* fkeys, uint32_t* out, uint64_t n_find,
-                    const uint32_t* ekeys, uint64_t n_erase, int tiles, int W) {
-  auto* t              = static_cast<emu_tree*>(h);
-  auto v               = t->view();
-  const uint64_t total = n_find + n_erase;
-  EMU_DISPATCH(W, run(total, tiles, kW, [&](uint64_t i, const emu_tile& tile) {
-    uint64_t a = (i * n_erase) / total, b = ((i + 1) * n_erase) / total;
-    if (b > a) {
-      v.cooperative_erase<kW>(ekeys[a], tile, 0u);
-    } else {
-      uint32_t r = v.cooperative_find<kW>(fkeys[i - a], tile, mvbt::kLatest, true);
-      if (tile.thread_rank() == 0) out[i - a] = r;
-    }
+                    const uint32_t* ekeys, uint64_t n_erase, int tiles, int W, uint32_t lanes) {
+  auto* t          = static_cast<emu_tree*>(h);
+  auto v           = t->view();
+  const uint32_t S = v.versioned ? emu_snapshot(h) : mvbt::kLatest;
+  const int warps  = std::max(1, tiles * W / 32);
+  std::vector<mvbt::write_stage> stage(warps);
+  EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {
+    const uint32_t w = mvbt::emu::sm;
+    mvbt::find_erase_units<kW, kW>(v, fkeys, out, (uint32_t)n_find, ekeys, (uint32_t)n_erase, lanes, S, w, (uint64_t)warps,
+                                   stage[w], warp, tile, tile);
   }));
 }
 
@@ -534,12 +527,15 @@ void emu_batch_run(void* h, uint32_t nb, const uint64_t* off, const uint32_t* ty
   auto* t = static_cast<emu_tree*>(h);
   auto v  = t->view();
   mvbt::batch_view B{type, key, arg, out_off, cap, result, reinterpret_cast<uint2*>(range_out)};
-  if (mode == 1) {
+  const int warps = std::max(1, tiles * W / 32);
+  std::vector<mvbt::write_stage> stage(warps);
+  if (mode == 1) {  // as many ops to a warp as it takes to give each warp some, as the library does
     for (uint32_t b = 0; b < nb; ++b) {
-      uint32_t S = emu_snapshot(h);
-      uint64_t lo = off[b], n = off[b + 1] - off[b];
-      EMU_DISPATCH(W, run(n, tiles, kW, [&](uint64_t i, const emu_tile& tile) {
-        mvbt::run_batch_op<kW>(v, B, lo + i, S, S + 1, tile);
+      const uint32_t S = emu_snapshot(h);
+      const uint32_t lanes = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(4, (off[b + 1] - off[b]) / (uint64_t)warps));
+      EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {
+        const uint32_t w = mvbt::emu::sm;
+        mvbt::mixed_ops<kW>(v, B, off[b], off[b + 1], lanes, S, w, (uint64_t)warps, stage[w], warp, tile);
       }));
     }
     return;
@@ -575,12 +571,10 @@ void emu_batch_run(void* h, uint32_t nb, const uint64_t* off, const uint32_t* ty
     sc.rc_limit   = &rc_limit;
     sc.series     = ser.data();
   }
-  const int warps = std::max(1, tiles * W / 32);
   if (sc.rc_limit)  // as k_count_ops
     run_warps(mvbt::kMaxSmSlots / 32, 8, [&](const emu_tile& warp, const emu_tile&) {
       mvbt::flush_chunks(&t->ctl, mvbt::emu::sm, t->ctl.ring_cap / 2, warp);
     });
-  std::vector<mvbt::write_stage> stage(warps);
   mvbt::batch_gate gate{0, 0};  // the warps as one block
   std::vector<mvbt::held_reads> held(warps);
   EMU_DISPATCH(W, run_warps(warps, kW, [&](const emu_tile& warp, const emu_tile& tile) {

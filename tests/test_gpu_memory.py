@@ -15,8 +15,11 @@ def _drop_trees():
 
 
 def _free():
+    import gc
     import torch
+    gc.collect()
     torch.cuda.synchronize()
+    torch.cuda.empty_cache()  # of the tests before
     return torch.cuda.mem_get_info()[0]
 
 
@@ -32,7 +35,6 @@ def test_release_memory_gives_back_what_dropped_trees_left():
     t.insert(keys, keys)
     t.close()
     del keys
-    torch.cuda.empty_cache()
     assert before - _free() >= 3 * GIB
     mv.release_memory()
     assert before - _free() < GIB // 4

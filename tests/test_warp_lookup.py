@@ -79,6 +79,38 @@ def test_emulated_warp_ranges_match_oracle(versioned, live, sorted_run):
     assert t.errors == 0
 
 
+@pytest.mark.parametrize("versioned,lanes,w", [(False, 5, 8), (False, 32, 16), (True, 4, 16), (True, 7, 8), (True, 32, 8)])
+def test_emulated_units_beside_writers_match_oracle(versioned, lanes, w):
+    """The two concurrent calls by six warps: reads at the call's snapshot beside writers of the same few leaves, which
+    readers find locked, changed since they were staged, or newer than their snapshot."""
+    from emu import EmuTree
+    import oracle
+    import workload as wl
+    t, m = EmuTree(versioned, capacity=1 << 14, tiles=6 * 32 // w, W=w), oracle.MVMap(versioned)
+    keys = np.arange(1, 161, dtype=np.uint32) * 100
+    t.write_warp(np.ones(keys.size), keys, keys)
+    m.insert(keys, keys)
+    for r in range(6):
+        new = wl.shuffle(r, np.concatenate([keys + 1 + r, keys[::2]]))
+        lo = wl.shuffle(r + 50, np.resize(keys, 400))
+        hi = lo + 700
+        pairs, counts = t.insert_range(new, new + r, lo, hi, 64, lanes=lanes)
+        if versioned:
+            want, wc = m.range_query(lo, hi, 64, m.take_snapshot())
+            mask = np.arange(64)[None, :] < np.minimum(wc, 64)[:, None]
+            assert np.array_equal(counts, wc) and np.array_equal(pairs[mask], want[mask])
+        m.insert(new, new + r)
+        gone, q = wl.shuffle(r + 9, new)[::3], wl.shuffle(r + 90, np.concatenate([new, keys]))
+        got = t.find_erase(q, gone, lanes=lanes)
+        was = m.find(q, m.take_snapshot()) if versioned else m.find(q)
+        assert np.all((got == was) | ((not versioned) & np.isin(q, gone) & (got == 0xFFFFFFFF)))
+        m.erase(gone)
+        assert t.errors == 0, t.stats()
+        assert np.array_equal(t.find_warp(q), m.find(q))
+    rep = t.validate()
+    assert rep["violations"] == 0 and rep["locked_nodes"] == 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("versioned,frontend", [(False, 0), (True, 1), (True, 2)])
 def test_gpu_ranges_of_warps_match_oracle(versioned, frontend):
