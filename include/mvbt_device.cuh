@@ -2529,9 +2529,9 @@ MVBT_DEV void write_warp(const device_tree& T, uint32_t key, uint32_t value, boo
     const uint32_t pm = up ? all & seps : all;
     const bool mem    = (pm >> lane) & 1u;
     const bool del    = !up && erase;
-    // one leader per run of lanes with the same node
-    const uint32_t below = pm & ((1u << lane) - 1u);
-    const uint32_t prev  = warp.shfl(leaf, below ? 31 - __clz(below) : 0);
+    // one leader per run of lanes with the same node (kSplit: whatever lanes between them are done)
+    const uint32_t below = pm & (kSplit ? (1u << lane) - 1u : lane ? 1u << (lane - 1u) : 0u);
+    const uint32_t prev  = warp.shfl(leaf, kSplit ? (below ? 31 - __clz(below) : 0) : (lane ? (int)lane - 1 : 0));
     const bool lead      = mem && (below == 0 || prev != leaf);
     const uint32_t lm    = warp.ballot(lead);
     uint32_t* const mod  = T.node_ptr(mem ? leaf : 0u) + kModWord;
@@ -3075,9 +3075,10 @@ MVBT_DEV void mixed_ops(const device_tree& T, const batch_view& B, uint64_t begi
   }
 }
 
-// Ops a warp claims at once: a full warp's worth, less when there would be fewer than `share` claims.
+// Ops a warp claims at once: a full warp's worth, less when there would be fewer than `share` claims (0 for a list
+// without batches, such as rejected offsets leave).
 MVBT_DEV uint32_t claim_size(uint64_t ops, uint64_t share, uint32_t least) {
-  const uint64_t c = ops / share;
+  const uint64_t c = share ? ops / share : 0;
   return c >= 32 ? 32u : (c < least ? least : (uint32_t)c);
 }
 
@@ -3096,7 +3097,6 @@ MVBT_DEV void batched_worker(const device_tree& T, const batch_view& B, const ba
   const uint32_t lane = warp.thread_rank();
   const uint32_t nb   = ld_relaxed_u32(sc.params + 0);
   const uint32_t S0   = ld_relaxed_u32(sc.params + 1);
-  if (nb == 0) return;  // an empty list, or one whose offsets were rejected
   const uint64_t TW = sc.wpre[nb], TR = sc.rpre[nb];
   const uint32_t wclaim = claim_size(TW, (uint64_t)nb * kWriteClaims, kTiles);
   const uint32_t rclaim = claim_size(TR, (uint64_t)warps * kReadClaims, kTiles);
