@@ -86,8 +86,9 @@ typedef struct mvbt_config {
 /* Batch front-end of the bulk calls (insert, find, erase, range_query). SORTED first sorts the
  * call's keys (a stable radix sort on the device: all 32 bits for writes, so a repeated key's last
  * occurrence in the array wins; the top 24 bits for reads, which only need locality) and gives
- * each tile a contiguous run of them; each op then starts its descent at the deepest node of the
- * previous op's path that covers its key, and results go back to the caller's positions. UNSORTED
+ * each warp a contiguous run of them, 32 at a time (reads beside writers: each tile, one at a time); a
+ * group then starts its descent at the deepest node of the previous group's path that covers its keys,
+ * and results go back to the caller's positions. UNSORTED
  * runs the ops in the caller's order, each from the root. AUTO takes SORTED for reads of a tree that no
  * writer changes meanwhile (concurrent = 0) from 2^20 ops on, and for other calls that are large and
  * dense against the tree (at least 2^16 ops and one op per 128 keys), where neighbouring ops share

@@ -7,7 +7,7 @@
 
 namespace mvbt_sort {
 
-// Scratch words (uint32) sort_pairs needs for n keys (digit counts and scan sums).
+// Scratch words (uint32) sort_pairs needs for n keys (digit counts of every tile, and the digits' totals).
 uint64_t scratch_words(uint32_t n);
 
 // Stable sort of keys[0, n) by their bits [low_bit, 32) (low_bit in {0, 8, 16, 24}: 0 = a full

@@ -1,10 +1,11 @@
 // Bulk kernels and the C ABI of the B200 multiversion B-link tree.
 //
-// Each bulk call maps one operation to one W-thread tile (W = 8 or 16) and runs a grid-stride
-// loop over a grid sized to full occupancy, so every SM keeps as many independent root-to-leaf
-// traversals in flight as its registers allow. The reference maps one op to one thread and lets
-// each 16-thread tile drain its 16 ops serially (include/btree_kernels.hpp:535-574); here the
-// hardware scheduler interleaves the tiles instead.
+// Large bulk calls run 32 operations to a warp: each lane holds one, the nodes that the lanes reach are
+// staged in shared memory, and reads and writes of up to 32 leaves share their round trips (k_find_warp,
+// k_range_warp, k_write_warp, the concurrent calls). Small calls, and the reads of single calls beside
+// writers, map one operation to one W-thread tile (W = 8 or 16). Grids are sized to full occupancy. The
+// reference maps one op to one thread and lets each 16-thread tile drain its 16 ops serially
+// (include/btree_kernels.hpp:535-574).
 #include <cuda_runtime.h>
 
 #include <algorithm>
