@@ -496,8 +496,11 @@ constexpr uint32_t kWarpWriteMin = 1u << 13;  // writes likewise
 // would queue on the few leaves there are, and every handoff of a queued lock costs an atomic per
 // waiter: at one leaf and ~25 000 tiles an insert into an empty tree ran at 4 M keys/s. So the
 // batch is cut into launches of about one tile per leaf of the tree each one starts on (~10 keys
-// per leaf), each about doubling the tree, until the full grid has a leaf per tile; the rest runs
-// in one launch. The keys of one call are unordered either way.
+// per leaf), each about doubling the tree, until the full grid has a leaf per tile; then 32 keys go to a
+// warp, again in launches that about double the tree until the full grid has a leaf per lane (from half
+// of that on: below it, few blocks run, and a tile per key is faster; M keys/s, tiles / warps: 2^20 keys into
+// an empty tree 370-440 / 290-330, 2^25 keys 1100-1250 / 1880-1930, and 500-890 when the rest of the call
+// ran on the first warp launch's few blocks). The keys of one call are unordered either way.
 template <int W>
 int insert_launches(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, uint32_t n, cudaStream_t s) {
   const uint64_t full  = grid_for(t, k_insert<W>, n);
@@ -507,10 +510,13 @@ int insert_launches(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, 
     uint64_t blocks = std::max<uint64_t>(1, (t->grown / 10) / tiles);
     uint64_t chunk  = n - done;
     if (blocks < full) chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(t->grown, blocks * tiles * 16));
-    if (blocks >= full && chunk >= kWarpWriteMin) {  // the rest in one launch, 32 keys a warp
-      const uint64_t in_flight = std::max<uint64_t>(1, (t->grown / 10) / t->block_size);  // about a key per leaf
-      const unsigned grid      = (unsigned)std::min<uint64_t>(grid_for_warps(t, k_write_warp<false, false>, chunk), in_flight);
-      k_write_warp<false, false><<<grid, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);
+    const uint64_t most = grid_for_warps(t, k_write_warp<false, false>, chunk);
+    const uint64_t room = (t->grown / 10) / t->block_size;  // blocks whose lanes have a leaf each
+    if (blocks >= full && chunk >= kWarpWriteMin && room < most)
+      chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(t->grown, kWarpWriteMin));
+    if (blocks >= full && chunk >= kWarpWriteMin && 2 * room >= most) {
+      k_write_warp<false, false><<<(unsigned)std::min(most, room), t->block_size, 0, s>>>(t->view(), keys + done, values + done,
+                                                                                         (uint32_t)chunk);
     } else {
       blocks = std::min(blocks, full);
       k_insert<W><<<(unsigned)blocks, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);

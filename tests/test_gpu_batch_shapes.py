@@ -139,3 +139,22 @@ def test_trees_made_and_dropped_reuse_their_memory():
         t.find(keys, out)
         assert torch.equal(out, keys) and t.check_errors() == 0
         t.close()
+
+
+@pytest.mark.parametrize("shape", [{}, {"max_blocks": 1}, {"block_size": 32, "max_blocks": 2}, {"tile_width": 16}])
+def test_unsorted_inserts_into_a_growing_tree_run_in_launches(shape):
+    """Sizes on both sides of the launches' lines, down to a grid of one block: every key is there afterwards."""
+    import torch
+    import mvgpubtree_b200 as mv
+    few = "max_blocks" in shape
+    t = mv.gpu_blink_tree(pool_bytes=1 << 28, frontend=mv.FRONTEND_UNSORTED, **shape)
+    keys = torch.randperm(1 << 21, device="cuda").to(torch.int32) * 1000 + 1
+    done = 0
+    for n in (1, 8191, 8192, 8193, 30_000) if few else (1, 8192, 100_003, 400_000, 1_200_000):
+        t.insert(keys[done:done + n], keys[done:done + n] ^ 5)
+        done += n
+        out = torch.zeros(done, dtype=torch.int32, device="cuda")
+        t.find(keys[:done].contiguous(), out)
+        assert torch.equal(out, keys[:done] ^ 5)
+    assert t.check_errors() == 0
+    assert t.validate_tree_structure()["violations"] == 0
