@@ -2493,7 +2493,7 @@ MVBT_CALL void push_tile(device_tree T, uint32_t key, uint32_t child, uint32_t E
 // before their left halves name them, and the separators are then written like keys, a level up: separators
 // of one parent share its lock. What is left goes to the tile path: splits without a slot, and separators
 // whose parent is full, stale or the anchor. For keys in order, whose leaves have parents in common: 4M new
-// keys into a plain tree of 16M 2.44 -> 1.62 ms, once more 4.32 -> 2.68. Keys all over the tree split
+// keys into a plain tree of 16M 2.44 -> 1.66 ms, once more 4.32 -> 2.81. Keys all over the tree split
 // few leaves of a warp at once, under as many parents, and the other leaves wait for the additional round:
 // 500K inserts beside 500K range queries 0.84 -> 0.86 ms, so these take the tile path.
 // leaf: each live lane's leaf as leaf_warp found it (which also left its parent in st.parent), possibly stale

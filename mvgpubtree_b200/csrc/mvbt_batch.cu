@@ -280,8 +280,8 @@ constexpr int kBatchBlocks   = 4;  // per SM: 64 registers; 37 KB of shared memo
 constexpr int kWarpsPerBlock = 8;  // of 256 threads, the largest block
 
 // Bound by the chain of batches (a batch's writes wait for the previous batch's) and by dependent loads.
-// An op per tile / claims by warps, with reclamation: 256 batches of 11.1M ops on 40M keys 20.0 / 7.0-8.4
-// ms, 8 batches of 5400 ops on 2^20 keys 362-404 / 174 us.
+// An op per tile / claims by warps, with reclamation: 256 batches of 11.1M ops on 40M keys 20.4 / 7.1-8.2
+// ms, 8 batches of 5400 ops on 2^20 keys 362-404 / 175-190 us.
 
 template <int W>
 __global__ void __launch_bounds__(256, kBatchBlocks) k_batched(device_tree T, batch_view B, batch_sched sc,
