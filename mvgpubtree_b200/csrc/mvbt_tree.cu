@@ -510,13 +510,15 @@ int insert_launches(mvbt_tree* t, const uint32_t* keys, const uint32_t* values, 
     uint64_t blocks = std::max<uint64_t>(1, (t->grown / 10) / tiles);
     uint64_t chunk  = n - done;
     if (blocks < full) chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(t->grown, blocks * tiles * 16));
-    const uint64_t most = grid_for_warps(t, k_write_warp<false, false>, chunk);
-    const uint64_t room = (t->grown / 10) / t->block_size;  // blocks whose lanes have a leaf each
-    if (blocks >= full && chunk >= kWarpWriteMin && room < most)
-      chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(t->grown, kWarpWriteMin));
-    if (blocks >= full && chunk >= kWarpWriteMin && 2 * room >= most) {
-      k_write_warp<false, false><<<(unsigned)std::min(most, room), t->block_size, 0, s>>>(t->view(), keys + done, values + done,
-                                                                                         (uint32_t)chunk);
+    uint64_t grid = 0;  // of the warp kernel, 0: tiles
+    if (blocks >= full && chunk >= kWarpWriteMin) {
+      const uint64_t most = grid_for_warps(t, k_write_warp<false, false>, chunk);
+      const uint64_t room = (t->grown / 10) / t->block_size;  // blocks whose lanes have a leaf each
+      if (room < most) chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(t->grown, kWarpWriteMin));
+      if (2 * room >= most) grid = std::min(most, room);
+    }
+    if (grid) {
+      k_write_warp<false, false><<<(unsigned)grid, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);
     } else {
       blocks = std::min(blocks, full);
       k_insert<W><<<(unsigned)blocks, t->block_size, 0, s>>>(t->view(), keys + done, values + done, (uint32_t)chunk);
